@@ -6,7 +6,8 @@
 // iteration cap, and the iterates of Jacobi-PCG (Barrett et al., "Templates",
 // Fig. 2.5) in exact arithmetic.
 //
-// One solve = one cooperative launch of a persistent kernel, one CTA per SM.
+// One solve = one cooperative launch of a persistent kernel, one CTA per SM.  Systems
+// that fit on chip run the kernels of cg_resident.cuh, the others stream their matrix:
 // Each CTA owns a contiguous range of slices (32-row groups of the SELL
 // matrix).  An iteration is two phases, each closed by an exact grid
 // reduction (exact_sum.cuh):
@@ -955,6 +956,14 @@ __global__ void __launch_bounds__(CGT64, 1) k_spmv_ring(SellView A, const V *val
     drain(R);
 }
 
+}  // namespace
+}  // namespace sysu
+
+#include "cg_resident.cuh"
+
+namespace sysu {
+namespace {
+
 // Tile size and ring depth for a matrix whose widest slice has wmax entries
 // per row; ebytes = bytes per matrix value.
 CgPlan plan_cg(int wmax, int ebytes, int consumers) {
@@ -1004,12 +1013,34 @@ static void cg_launch64(const SellDev &A, const double *val, const double *b, do
                         cudaStream_t st) {
     int n = A.n;
     if (n == 0) return;
+    if (const ResPlan rp = plan_resident(A, 8, w.sm_cap); rp.R) {
+        w.ensure(n, 1, num_sms(), st);
+        if (!gate) SYSU_CUDA(cudaMemsetAsync(info, 0, sizeof(SolveInfo), st));
+        CgResArgs ra{};
+        ra.A = view(A, val);
+        ra.b = b;
+        ra.x = x;
+        ra.z = w.s.get();
+        ra.omega = o.omega;
+        ra.jacobi = o.jacobi;
+        ra.x0_zero = x0_zero && !gate;
+        ra.info = info;
+        ra.maxit = o.maxit;
+        ra.eps = o.eps;
+        ra.ts = w.phase_ts;
+        ra.ld = rp.ld;
+        ra.gate = gate;
+        ra.slots = w.clear_slots(st);
+        if (rp.R == 1) launch_resident(k_cg_res<1>, rp, ra, A.wmax, st);
+        else if (rp.R == 2) launch_resident(k_cg_res<2>, rp, ra, A.wmax, st);
+        else if (rp.R == 4) launch_resident(k_cg_res<4>, rp, ra, A.wmax, st);
+        else launch_resident(k_cg_res<6>, rp, ra, A.wmax, st);
+        return;
+    }
     // rows of at most 5 entries (tets): 5 gathers held one tile ahead on 640 threads
     // (2.5 % faster than 6 on the 2M-cell tet p' system); wider rows (hex: 7): one tile
-    // at a time on 1024 threads (3 % faster there than the look-ahead form)
-    // (below 1M rows the wide form also looks ahead: the 256k-row hex p' system of the
-    // CHT channel is latency-bound and measured 7.99 ms per solve that way, 8.37 ms
-    // one tile at a time)
+    // at a time on 1024 threads (3 % faster there than the look-ahead form; below 1M
+    // rows, where latency counts more, the look-ahead form)
     const bool narrow = A.wmax <= 5, wide_big = !narrow && n >= (1 << 20);
     auto kern = narrow ? k_cg_pipe<5, true> : (wide_big ? k_cg_pipe<CG_WR, false> : k_cg_pipe<CG_WR, true>);
     static int maxb5 = 0, maxb6 = 0, maxb6a = 0;
@@ -1077,6 +1108,32 @@ void cg_solve_mixed(const SellDev &A, const double *val, const float *val32, con
                     bool x0_zero, const KrylovOpts &o, KrylovWork &w, SolveInfo *info, cudaStream_t st) {
     int n = A.n;
     if (n == 0) return;
+    if (const ResPlan rp = plan_resident(A, 4, w.sm_cap); rp.R) {
+        w.ensure(n, 1, num_sms(), st);
+        w.ensure32(n, st);
+        if (x0_zero) { k_zero<<<(n + KB - 1) / KB, KB, 0, st>>>(x, n); ++::sysu::g_launches; }
+        SYSU_CUDA(cudaMemsetAsync(info, 0, sizeof(SolveInfo), st));
+        CgResArgs ra{};
+        ra.A = view(A, val);
+        ra.val32 = val32;
+        ra.b = b;
+        ra.x = x;
+        ra.z32 = w.z32.get();
+        ra.omega = o.omega;
+        ra.info = info;
+        ra.maxit = o.maxit;
+        ra.eps = o.eps;
+        ra.inner_tol = o.inner_tol;
+        ra.ts = w.phase_ts;
+        ra.ld = rp.ld;
+        ra.slots = w.clear_slots(st);
+        if (rp.R == 1) launch_resident(k_cg_mixed_res<1>, rp, ra, A.wmax, st);
+        else if (rp.R == 2) launch_resident(k_cg_mixed_res<2>, rp, ra, A.wmax, st);
+        else if (rp.R == 4) launch_resident(k_cg_mixed_res<4>, rp, ra, A.wmax, st);
+        else launch_resident(k_cg_mixed_res<8>, rp, ra, A.wmax, st);
+        if (w.sm_cap <= 0) cg_launch64(A, val, b, x, false, o, w, info, info, st);  // see below
+        return;
+    }
     static int maxb = 0;
     if (!maxb) maxb = cg_max_blocks(k_cg_mixed_pipe, CGT32);
     w.ensure(n, 1, maxb, st);

@@ -22,6 +22,7 @@
 // x += alpha M^-1 p + omega M^-1 s is taken as x += M^-1 (alpha p + omega s).
 // Both are the same iterates in exact arithmetic; the rounding differs from the
 // unfolded form by a unit in the last place per product.
+#include "grid_all.cuh"
 #include "krylov_dev.cuh"
 
 #include <algorithm>
@@ -935,6 +936,13 @@ void KrylovWork::ensure(int n_, int nrhs_, int max_blocks_, cudaStream_t st) {
     partials.alloc((size_t)8 * NVMAX * max_blocks);  // also the 4-word exact-sum partials
     barrier.alloc(1);
     barrier.zero(st);
+    slots.alloc(AX_WORDS);
+}
+
+unsigned long long *KrylovWork::clear_slots(cudaStream_t st) {
+    if (slots.size() < AX_WORDS) throw CaseError{"grid-sum slots are not allocated"};
+    slots.zero(st);
+    return slots.get();
 }
 
 void KrylovWork::ensure32(int n_, cudaStream_t st) {

@@ -80,6 +80,8 @@ struct KrylovWork {
     DevBuf<double> gV, gZ, gW, ilu;                  // GMRES basis, preconditioned basis, ILU(0) factors
     DevBuf<long long> gpart;                         // exact multi-value partial sums
     DevBuf<GridBarrier> barrier;
+    DevBuf<unsigned long long> slots;                // exchange area of the grid sums (grid_all.cuh)
+    unsigned long long *clear_slots(cudaStream_t st);  // the area, cleared on st for one launch
     unsigned long long *phase_ts = nullptr;  // optional: 4 timestamps per CG iteration, first 64
     // > 0: the persistent solves of this work use at most this many SMs' worth of
     // blocks (cases that share the GPU; the batch autotuner sets it)

@@ -1,0 +1,71 @@
+"""The CG kernels that keep the system on chip (csrc/cg_resident.cuh), at the sizes where their
+launch changes: one CTA, the rows a thread holds (1, 2, 4, 6 or 8 for 152 CTAs of 512 threads),
+the last size that fits and the first that goes to the streaming kernel.
+
+b = A x* for a 7-point operator whose diagonal exceeds its row's off-diagonal sum by 10 %, so
+||x - x*|| <= ||A^-1|| ||r|| <= cond(A) eps ||x*|| with cond(A) <= 21 max(d) / min(d) <= 100.
+"""
+import numpy as np
+import pytest
+
+from sysu_cfd_heat_gb300.solver import csr_solve
+
+pytestmark = pytest.mark.gpu
+EPS = 1e-10
+
+
+def seven_point(nx, ny, nz, seed):
+    n = nx * ny * nz
+    rng = np.random.default_rng(seed)
+    idx = np.arange(n).reshape(nz, ny, nx)
+    rows, cols, vals = [np.arange(n)], [np.arange(n)], [np.zeros(n)]
+    diag = np.zeros(n)
+    for ax in range(3):
+        a = np.take(idx, range(idx.shape[ax] - 1), axis=ax).ravel()
+        b = np.take(idx, range(1, idx.shape[ax]), axis=ax).ravel()
+        w = rng.uniform(0.8, 1.2, a.size)
+        rows += [a, b]
+        cols += [b, a]
+        vals += [-w, -w]
+        diag += np.bincount(a, w, n) + np.bincount(b, w, n)
+    vals[0] = 1.1 * np.maximum(diag, 2.0)
+    r, c, v = np.concatenate(rows), np.concatenate(cols), np.concatenate(vals)
+    order = np.lexsort((c, r))
+    r, c, v = r[order], c[order].astype(np.int32), v[order]
+    rp = np.concatenate([[0], np.cumsum(np.bincount(r, minlength=n))]).astype(np.int32)
+    x = rng.standard_normal(n)
+    return rp, c, v, x, np.add.reduceat(v * x[c], rp[:-1])
+
+
+SIZES = [
+    (1, 1, 1), (31, 1, 1), (33, 1, 1), (7, 5, 139),     # one slice, two, a ragged 153rd
+    (64, 38, 32), (64, 38, 33),                         # 77,824 rows: one row a thread, then two
+    (64, 76, 33), (64, 76, 64), (64, 76, 65),           # four; the last with four, the first with six
+    (80, 70, 66), (80, 70, 71), (80, 80, 101),          # beyond FP64's shared memory; beyond FP32's
+]
+
+
+@pytest.mark.parametrize("shape", SIZES)
+@pytest.mark.parametrize("method", ["CG", "CG-mixed"])
+def test_resident_cg(shape, method):
+    rp, c, v, x, b = seven_point(*shape, seed=sum(shape))
+    x0 = np.random.default_rng(1).standard_normal(len(x)) if shape[0] % 2 else None
+    y, it, res, status = csr_solve(rp, c, v, b, x0, method=method, maxit=1000, eps=EPS, omega=1.3)
+    assert status == 0 and res < EPS and it > 0
+    assert np.linalg.norm(y - x) <= 100 * EPS * np.linalg.norm(x)
+    z, it2, res2, _ = csr_solve(rp, c, v, b, x0, method=method, maxit=1000, eps=EPS, omega=1.3)
+    assert it2 == it and res2 == res and np.array_equal(y, z)  # runs are bit-identical
+
+
+def test_resident_cg_cap_breakdown_and_no_preconditioner():
+    rp, c, v, x, b = seven_point(20, 19, 18, seed=3)
+    _, it, res, status = csr_solve(rp, c, v, b, method="CG", maxit=5, eps=1e-14)
+    assert it == 5 and status == 1 and res > 1e-14
+    y, _, res, status = csr_solve(rp, c, v, b, method="CG", precond="none", maxit=1000, eps=EPS)
+    assert status == 0 and np.linalg.norm(y - x) <= 100 * EPS * np.linalg.norm(x)
+    y, it, res, status = csr_solve(rp, c, v, np.zeros_like(b), method="CG", maxit=10, eps=EPS)
+    assert it == 0 and status == 0 and not y.any()
+    bad = b.copy()
+    bad[7] = np.nan
+    _, it, _, status = csr_solve(rp, c, v, bad, method="CG", maxit=10, eps=EPS)
+    assert it == 0 and status == 4
