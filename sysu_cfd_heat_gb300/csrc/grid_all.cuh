@@ -28,7 +28,7 @@
 
 namespace sysu {
 
-constexpr int AX_NVMAX = 6;
+constexpr int AX_NVMAX = 3;
 constexpr int AX_MAX_BLOCKS = 255;  // the arrival count has 8 bits
 
 // 64-bit words of a launch's exchange area: the counter (a 128-byte line of its own), two sets

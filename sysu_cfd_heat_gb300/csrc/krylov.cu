@@ -129,34 +129,6 @@ void SellDev::upload(const SellPattern &p, cudaStream_t s) {
 
 namespace {
 
-// y_c = A (dinv .* x_c) for NR right-hand sides, skipping inactive ones, from
-// the column-scaled values sv[e] = a_e dinv[col e].  MULTI: right-hand side c
-// has its own scaled values svals[c] (same pattern); the column indices are
-// read once.
-template <int NR, bool MULTI>
-__device__ __forceinline__ void row_dot_scaled(const SellView &A, const double *const *svals, int i,
-                                               const double *__restrict__ x, int n, const bool (&act)[3],
-                                               double (&y)[NR]) {
-    int s = i >> 5;
-    int e = A.sl_ptr[s] + (i & 31);
-    int w = A.sl_w[s];
-#pragma unroll
-    for (int c = 0; c < NR; ++c) y[c] = 0.0;
-    for (int k = 0; k < w; ++k, e += 32) {
-        int j = A.col[e];
-        if (MULTI) {
-#pragma unroll
-            for (int c = 0; c < NR; ++c)
-                if (act[c]) y[c] = fma(svals[c][e], x[(size_t)c * n + j], y[c]);
-        } else {
-            double a = svals[0][e];
-#pragma unroll
-            for (int c = 0; c < NR; ++c)
-                if (act[c]) y[c] = fma(a, x[(size_t)c * n + j], y[c]);
-        }
-    }
-}
-
 // sv[e] = val[e] dinv[col e] over all stored entries (padding entries hold 0
 // and their own row as the column).
 __global__ void k_scale_cols(long nnz, const int *__restrict__ col, const double *__restrict__ val,
@@ -450,17 +422,126 @@ struct BicgArgs {
     const SolveInfo *gate;
 };
 
-// Scalar state of a BiCGSTAB solve.  Thread 0 of every block derives it from
-// the global sums (which every block adds up in the same fixed order, so all
-// blocks hold identical copies) and the block reads it from shared memory:
-// the square roots and divisions run once per block instead of in every thread,
-// and the vector loops keep only the few scalars they use in registers.
+// Scalar state of a BiCGSTAB solve, in shared memory.  One thread a component derives it
+// from the global sums (every block adds them in the same order, so all blocks hold the
+// same bits): the divisions run once per block, the components side by side, and the vector
+// loops keep only the scalars they use in registers.  Norms are compared squared: an FP64
+// square root takes 2,600 clocks here, a division 840.
 struct BicgState {
-    double bnorm[3], res[3], rho[3], rho_prev[3], alpha[3], omg[3], beta[3], snorm[3];
-    int it[3], status[3], done[3], act[3], early[3], act2[3];
-    int any;
+    double bb[3], rr[3], thr[3], rho[3], rho_prev[3], alpha[3], omg[3], beta[3];
+    int it[3], status[3], done[3], act[3], early[3];
 };
+__shared__ double g_bicg_smem[9 * (KB / 32)], g_bicg_sum[9];
 
+// One step of the warp's butterfly over NV values with the values dealt out: a lane keeps
+// the half of the values that its side of the step owns and adds its partner's, so NV values
+// cost about NV additions instead of 5 NV.  The additions are those of the butterfly of each
+// value (xor 16, 8, 4, 2, 1): the same bits.  Returns how many values a lane still holds.
+template <int NV>
+__device__ __forceinline__ double deal_sum(const double (&v)[NV], int o) {
+    const int lane = threadIdx.x & 31;
+    if constexpr (NV == 1) {
+        double s = v[0];
+        for (; o > 0; o >>= 1) s += __shfl_xor_sync(FULL_MASK, s, o);
+        return s;
+    } else {
+        constexpr int H = (NV + 1) / 2;  // the lower side keeps values 0..H-1, the upper H..NV-1
+        const bool up = (lane & o) != 0;
+        double k[H];
+#pragma unroll
+        for (int j = 0; j < H; ++j) {
+            const double lo = v[j], hi = H + j < NV ? v[H + j] : 0.0;
+            const double other = __shfl_xor_sync(FULL_MASK, up ? lo : hi, o);
+            k[j] = (up ? hi : lo) + other;
+        }
+        return deal_sum<H>(k, o >> 1);
+    }
+}
+// lane that holds value k's sum after deal_sum<NV>
+template <int NV>
+__device__ __forceinline__ int deal_lane(int k, int o = 16) {
+    if constexpr (NV == 1) {
+        return 0;
+    } else {
+        constexpr int H = (NV + 1) / 2;
+        return k < H ? deal_lane<H>(k, o >> 1) : o + deal_lane<H>(k - H, o >> 1);
+    }
+}
+
+// Grid sums of NV values, to g_bicg_sum for the whole block, in the order of block_sum_t0
+// (warp butterfly, warps) and warp_sum_partials; value k by thread k, then by a warp.
+template <int NV>
+__device__ __forceinline__ bool bicg_sum(const double (&v)[NV], RedCtx &rc, GridBarrier *gb, int *err) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int NW = KB / 32;
+    const double w = deal_sum<NV>(v, 16);
+#pragma unroll
+    for (int k = 0; k < NV; ++k)
+        if (lane == deal_lane<NV>(k)) g_bicg_smem[k * NW + warp] = w;
+    __syncthreads();
+    double *buf = rc.partials + (size_t)rc.parity * 9 * rc.G;
+    rc.parity ^= 1;
+    if (threadIdx.x < NV) {
+        double s = 0.0;
+#pragma unroll
+        for (int q = 0; q < NW; ++q) s += g_bicg_smem[threadIdx.x * NW + q];
+        buf[(size_t)threadIdx.x * rc.G + blockIdx.x] = s;
+    }
+    if (!grid_sync(gb, err)) return false;
+    for (int k = warp; k < NV; k += NW) {
+        const double s = warp_sum_partials(buf + (size_t)k * rc.G, rc.G);
+        if (lane == 0) g_bicg_sum[k] = s;
+    }
+    __syncthreads();
+    return true;
+}
+
+// y_c = A (dinv .* x_c) for NR right-hand sides, skipping inactive ones, from the
+// column-scaled values sv[e] = a_e dinv[col e]; MULTI: right-hand side c has its own values
+// svals[c] (same pattern).  Four entries' columns, values and gathers before their FMAs,
+// which take the entries in order.
+template <int NR, bool MULTI>
+__device__ __forceinline__ void row_dot_scaled(const SellView &A, const double *const *svals, int i,
+                                               const double *__restrict__ x, int n, const bool (&act)[3],
+                                               double (&y)[NR]) {
+    const int s = i >> 5;
+    int e = A.sl_ptr[s] + (i & 31);
+    const int w = A.sl_w[s];
+    constexpr int U = NR == 1 ? 4 : (MULTI ? 1 : 2);
+#pragma unroll
+    for (int c = 0; c < NR; ++c) y[c] = 0.0;
+    for (int k = 0; k < w; k += U, e += 32 * U) {
+        int j[U];
+        double a[U][MULTI ? NR : 1], g[U][NR];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (k + u < w) {
+                j[u] = A.col[e + 32 * u];
+#pragma unroll
+                for (int c = 0; c < (MULTI ? NR : 1); ++c) a[u][c] = svals[c][e + 32 * u];
+            }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (k + u < w)
+#pragma unroll
+                for (int c = 0; c < NR; ++c)
+                    if (act[c]) g[u][c] = x[(size_t)c * n + j[u]];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (k + u < w)
+#pragma unroll
+                for (int c = 0; c < NR; ++c)
+                    if (act[c]) y[c] = fma(a[u][MULTI ? c : 0], g[u][c], y[c]);
+    }
+}
+
+// Rows thread-per-row with a grid stride over up to 608 blocks of 256 threads, FP64 sums in
+// a fixed order that is the same for one and for three right-hand sides, so u, v, w solved
+// together equal three solves to the bit.  BiCGSTAB amplifies the last bit of a sum (another
+// order moved the solution of a 60,680-row convection-diffusion system solved to 1e-10 by
+// 1e-8), so the order stays.  Bounded by the FP64 pipe at 2M rows and by the grid-wide steps
+// below 300k: three sums and two bare barriers an iteration -- s.s, which only decides the
+// early exit, is summed with t.s and t.t.
 template <int NR, bool MULTI>
 __global__ void __launch_bounds__(KB, 4) k_bicgstab(BicgArgs a) {
     if (a.gate && a.gate->status[0] != DEV_STALLED) return;  // the same word for every block
@@ -468,7 +549,7 @@ __global__ void __launch_bounds__(KB, 4) k_bicgstab(BicgArgs a) {
     const int n = a.A.n;
     const int T = gridDim.x * KB;
     const int t0 = blockIdx.x * KB + threadIdx.x;
-    const bool lead = threadIdx.x == 0;
+    const int tid = threadIdx.x;
     int *err = &a.info->err;
     RedCtx rc{a.partials, (int)gridDim.x, 0};
     const double *__restrict__ dinv = a.dinv;
@@ -487,53 +568,50 @@ __global__ void __launch_bounds__(KB, 4) k_bicgstab(BicgArgs a) {
                 double ri = bi - row_dot(Ac, i, a.x[c]);
                 a.r[c * N + i] = ri;
                 a.rt[c * N + i] = ri;
-                v[c] += bi * bi;
-                v[NR + c] += ri * ri;
+                v[c] = fma(bi, bi, v[c]);
+                v[NR + c] = fma(ri, ri, v[NR + c]);
             }
         }
-        if (!grid_reduce_t0<2 * NR>(v, rc, a.gb, err)) return;
-        if (lead) {
-#pragma unroll
-            for (int c = 0; c < NR; ++c) {
-                double bn = sqrt(v[c]);
-                if (bn == 0.0) bn = 1.0;
-                S.bnorm[c] = bn;
-                S.res[c] = sqrt(v[NR + c]) / bn;
-                S.rho[c] = v[NR + c];
-                S.rho_prev[c] = S.alpha[c] = S.omg[c] = 1.0;
-                S.it[c] = 0;
-                S.status[c] = DEV_OK;
-                S.done[c] = 0;
-            }
+        if (!bicg_sum<2 * NR>(v, rc, a.gb, err)) return;
+        if (tid < NR) {
+            const int c = tid;
+            S.bb[c] = g_bicg_sum[c] == 0.0 ? 1.0 : g_bicg_sum[c];
+            S.thr[c] = a.eps * a.eps * S.bb[c];
+            S.rr[c] = S.rho[c] = g_bicg_sum[NR + c];
+            S.rho_prev[c] = S.alpha[c] = S.omg[c] = 1.0;
+            S.it[c] = 0;
+            S.status[c] = DEV_OK;
+            S.done[c] = 0;
         }
+        __syncwarp();
     }
     bool act[3] = {false, false, false};
     for (;;) {
-        if (lead) {
-            int any = 0;
-#pragma unroll
-            for (int c = 0; c < NR; ++c) {
-                bool ac = !S.done[c] && !(S.res[c] < a.eps) && S.it[c] < a.maxit;
-                if (ac && !isfinite(S.res[c])) { S.done[c] = 1; S.status[c] = DEV_NONFINITE; ac = false; }
-                if (ac && S.rho[c] == 0.0) { S.done[c] = 1; S.status[c] = DEV_BREAKDOWN; ac = false; }
-                if (ac) {
-                    ++S.it[c];
-                    any = 1;
-                    S.beta[c] = (S.it[c] == 1) ? 0.0 : (S.rho[c] / S.rho_prev[c]) * (S.alpha[c] / S.omg[c]);
-                }
-                S.act[c] = ac;
+        if (tid < NR) {
+            const int c = tid;
+            bool ac = !S.done[c] && !(S.rr[c] < S.thr[c]) && S.it[c] < a.maxit;
+            if (ac && !isfinite(S.rr[c])) { S.done[c] = 1; S.status[c] = DEV_NONFINITE; ac = false; }
+            if (ac && S.rho[c] == 0.0) { S.done[c] = 1; S.status[c] = DEV_BREAKDOWN; ac = false; }
+            if (ac) {
+                ++S.it[c];
+                S.beta[c] = S.it[c] == 1 ? 0.0 : (S.rho[c] / S.rho_prev[c]) * (S.alpha[c] / S.omg[c]);
             }
-            S.any = any;
+            S.act[c] = ac;
         }
         __syncthreads();
-        if (!S.any) break;
+        bool any = false;
+#pragma unroll
+        for (int c = 0; c < NR; ++c) {
+            act[c] = S.act[c] != 0;
+            any = any || act[c];
+        }
+        if (!any) break;
         // p = r + beta (p - omega v)
         {
             double beta[NR], omg[NR];
             bool first[NR];
 #pragma unroll
             for (int c = 0; c < NR; ++c) {
-                act[c] = S.act[c] != 0;
                 beta[c] = S.beta[c];
                 omg[c] = S.omg[c];
                 first[c] = S.it[c] == 1;
@@ -543,7 +621,7 @@ __global__ void __launch_bounds__(KB, 4) k_bicgstab(BicgArgs a) {
                 for (int c = 0; c < NR; ++c) {
                     if (!act[c]) continue;
                     size_t k = c * N + i;
-                    a.p[k] = first[c] ? a.r[k] : a.r[k] + beta[c] * (a.p[k] - omg[c] * a.v[k]);
+                    a.p[k] = first[c] ? a.r[k] : fma(beta[c], fma(-omg[c], a.v[k], a.p[k]), a.r[k]);
                 }
             }
         }
@@ -560,26 +638,24 @@ __global__ void __launch_bounds__(KB, 4) k_bicgstab(BicgArgs a) {
                 for (int c = 0; c < NR; ++c) {
                     if (!act[c]) continue;
                     a.v[c * N + i] = y[c];
-                    red[c] += a.rt[c * N + i] * y[c];
+                    red[c] = fma(a.rt[c * N + i], y[c], red[c]);
                 }
             }
-            if (!grid_reduce_t0<NR>(red, rc, a.gb, err)) return;
-            if (lead) {
-#pragma unroll
-                for (int c = 0; c < NR; ++c) {
-                    if (!S.act[c]) continue;
-                    if (red[c] == 0.0) { S.done[c] = 1; S.status[c] = DEV_BREAKDOWN; S.act[c] = 0; continue; }
-                    S.alpha[c] = S.rho[c] / red[c];
+            if (!bicg_sum<NR>(red, rc, a.gb, err)) return;
+            if (tid < NR) {
+                const int c = tid;
+                if (S.act[c]) {
+                    if (g_bicg_sum[c] == 0.0) { S.done[c] = 1; S.status[c] = DEV_BREAKDOWN; S.act[c] = 0; }
+                    else S.alpha[c] = S.rho[c] / g_bicg_sum[c];
                 }
             }
             __syncthreads();
         }
-        // s = r - alpha v ; ||s||
+        // s = r - alpha v
         {
-            double red[NR], alpha[NR];
+            double alpha[NR];
 #pragma unroll
             for (int c = 0; c < NR; ++c) {
-                red[c] = 0.0;
                 act[c] = S.act[c] != 0;
                 alpha[c] = S.alpha[c];
             }
@@ -588,50 +664,36 @@ __global__ void __launch_bounds__(KB, 4) k_bicgstab(BicgArgs a) {
                 for (int c = 0; c < NR; ++c) {
                     if (!act[c]) continue;
                     size_t k = c * N + i;
-                    double si = a.r[k] - alpha[c] * a.v[k];
-                    a.s[k] = si;
-                    red[c] += si * si;
+                    a.s[k] = fma(-alpha[c], a.v[k], a.r[k]);
                 }
             }
-            if (!grid_reduce_t0<NR>(red, rc, a.gb, err)) return;
-            if (lead) {
-#pragma unroll
-                for (int c = 0; c < NR; ++c) {
-                    S.early[c] = 0;
-                    S.act2[c] = 0;
-                    if (!S.act[c]) continue;
-                    S.snorm[c] = sqrt(red[c]) / S.bnorm[c];
-                    S.early[c] = S.snorm[c] < a.eps;
-                    S.act2[c] = !S.early[c];
-                }
-            }
-            __syncthreads();
         }
-        // t = A M^-1 s ; t.s, t.t
+        if (!grid_sync(a.gb, err)) return;
+        // t = A M^-1 s ; t.s, t.t, s.s
         {
-            bool act2[3] = {false, false, false};
+            double red[3 * NR];
 #pragma unroll
-            for (int c = 0; c < NR; ++c) act2[c] = S.act2[c] != 0;
-            double red[2 * NR];
-#pragma unroll
-            for (int c = 0; c < 2 * NR; ++c) red[c] = 0.0;
+            for (int c = 0; c < 3 * NR; ++c) red[c] = 0.0;
             for (int i = t0; i < n; i += T) {
                 double y[NR];
-                row_dot_scaled<NR, MULTI>(a.A, a.svals, i, a.s, n, act2, y);
+                row_dot_scaled<NR, MULTI>(a.A, a.svals, i, a.s, n, act, y);
 #pragma unroll
                 for (int c = 0; c < NR; ++c) {
-                    if (!act2[c]) continue;
+                    if (!act[c]) continue;
                     size_t k = c * N + i;
+                    const double si = a.s[k];
                     a.t[k] = y[c];
-                    red[c] += y[c] * a.s[k];
-                    red[NR + c] += y[c] * y[c];
+                    red[c] = fma(y[c], si, red[c]);
+                    red[NR + c] = fma(y[c], y[c], red[NR + c]);
+                    red[2 * NR + c] = fma(si, si, red[2 * NR + c]);
                 }
             }
-            if (!grid_reduce_t0<2 * NR>(red, rc, a.gb, err)) return;
-            if (lead) {
-#pragma unroll
-                for (int c = 0; c < NR; ++c)
-                    if (S.act2[c]) S.omg[c] = red[NR + c] != 0.0 ? red[c] / red[NR + c] : 0.0;
+            if (!bicg_sum<3 * NR>(red, rc, a.gb, err)) return;
+            if (tid < NR) {
+                const int c = tid;
+                S.early[c] = S.act[c] && g_bicg_sum[2 * NR + c] < S.thr[c];
+                if (S.early[c]) S.rr[c] = g_bicg_sum[2 * NR + c];
+                else if (S.act[c]) S.omg[c] = g_bicg_sum[NR + c] != 0.0 ? g_bicg_sum[c] / g_bicg_sum[NR + c] : 0.0;
             }
             __syncthreads();
         }
@@ -653,44 +715,41 @@ __global__ void __launch_bounds__(KB, 4) k_bicgstab(BicgArgs a) {
                     size_t k = c * N + i;
                     double di = MULTI ? dinv[k] : dinv[i];
                     if (early[c]) {
-                        a.x[c][i] += alpha[c] * (di * a.p[k]);
+                        a.x[c][i] = fma(alpha[c], di * a.p[k], a.x[c][i]);
                     } else {
                         double si = a.s[k];
                         a.x[c][i] = fma(di, fma(alpha[c], a.p[k], omg[c] * si), a.x[c][i]);
                         double ri = fma(-omg[c], a.t[k], si);
                         a.r[k] = ri;
-                        red[c] += ri * ri;
-                        red[NR + c] += a.rt[k] * ri;
+                        red[c] = fma(ri, ri, red[c]);
+                        red[NR + c] = fma(a.rt[k], ri, red[NR + c]);
                     }
                 }
             }
-            if (!grid_reduce_t0<2 * NR>(red, rc, a.gb, err)) return;
-            if (lead) {
-#pragma unroll
-                for (int c = 0; c < NR; ++c) {
-                    if (!S.act[c]) continue;
+            if (!bicg_sum<2 * NR>(red, rc, a.gb, err)) return;
+            if (tid < NR) {
+                const int c = tid;
+                if (S.act[c]) {
                     if (S.early[c]) {
-                        S.res[c] = S.snorm[c];
                         S.done[c] = 1;
                     } else {
-                        S.res[c] = sqrt(red[c]) / S.bnorm[c];
+                        S.rr[c] = g_bicg_sum[c];
                         S.rho_prev[c] = S.rho[c];
-                        S.rho[c] = red[NR + c];
-                        if (S.omg[c] == 0.0 && !(S.res[c] < a.eps)) { S.done[c] = 1; S.status[c] = DEV_BREAKDOWN; }
+                        S.rho[c] = g_bicg_sum[NR + c];
+                        if (S.omg[c] == 0.0 && !(S.rr[c] < S.thr[c])) { S.done[c] = 1; S.status[c] = DEV_BREAKDOWN; }
                     }
                 }
             }
+            __syncwarp();
         }
     }
-    if (blockIdx.x == 0 && lead) {
-#pragma unroll
-        for (int c = 0; c < NR; ++c) {
-            int st = S.status[c];
-            if (st == DEV_OK && !(S.res[c] < a.eps)) st = isfinite(S.res[c]) ? DEV_MAXITER : DEV_NONFINITE;
-            a.info->status[c] = st;
-            a.info->iters[c] = S.it[c] + (c == 0 ? it_before : 0);
-            a.info->res[c] = S.res[c];
-        }
+    if (blockIdx.x == 0 && tid < NR) {
+        const int c = tid;
+        int st = S.status[c];
+        if (st == DEV_OK && !(S.rr[c] < S.thr[c])) st = isfinite(S.rr[c]) ? DEV_MAXITER : DEV_NONFINITE;
+        a.info->status[c] = st;
+        a.info->iters[c] = S.it[c] + (c == 0 ? it_before : 0);
+        a.info->res[c] = sqrt(S.rr[c]) / sqrt(S.bb[c]);
     }
 }
 
@@ -716,105 +775,141 @@ struct BicgMixedArgs {
     double *x;
     const double *dinv;    // FP64 Jacobi diagonal inverse
     double *r64;           // FP64 residual scratch
-    float *r, *rt, *p, *v, *s, *t, *e;  // in units of sig (a power of two, sig ||r|| ~ 1)
-    double *partials;
-    GridBarrier *gb;
+    float *r, *rt, *p, *v, *t, *e;  // in units of sig (a power of two, sig ||r|| ~ 1); s in r's storage
+    unsigned long long *slots;
     SolveInfo *info;
     int maxit;
     double eps, inner_tol;
 };
 
 struct BicgMixedState {
-    double bb, thr, rr64, rr_ref, r0in, rho, rho_prev, alpha, omg, beta, snorm2, sig;
+    double bb, thr, rr64, rr_ref, r0in, rho, rho_prev, alpha, omg, beta, sig;
+    double sum[3];
     int it, inner, status, upd, stall, act, early, done;
 };
 
-// y = A_s x over FP32 column-scaled values, one row (FMA order of row_dot_scaled)
-__device__ __forceinline__ float row_dot32(const SellView &A, const float *__restrict__ sv, int i,
-                                           const float *__restrict__ x) {
-    const int s = i >> 5;
-    int e = A.sl_ptr[s] + (i & 31);
-    const int w = A.sl_w[s];
+// y = A_s x over FP32 column-scaled values, one row (FMAs in entry order); local row j
+template <bool RES>
+__device__ __forceinline__ float bicg_row32(const BicgMixedArgs &a, const float *mval, const int *mcol, int ld, int i,
+                                            int j, const float *x) {
+    const int s = i >> 5, w = __ldg(a.A.sl_w + s);
+    const int e = RES ? 0 : __ldg(a.A.sl_ptr + s) + (i & 31);
     float y = 0.f;
-    for (int k = 0; k < w; ++k, e += 32) y = fmaf(sv[e], x[A.col[e]], y);
+    for (int k0 = 0; k0 < w; k0 += 8) {
+        int c[8];
+        float v[8], g[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (k0 + u < w) {
+                c[u] = RES ? mcol[(k0 + u) * ld + j] : __ldg(a.A.col + e + 32 * (k0 + u));
+                v[u] = RES ? mval[(k0 + u) * ld + j] : __ldg(a.sv32 + e + 32 * (k0 + u));
+            }
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (k0 + u < w) g[u] = x[c[u]];
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (k0 + u < w) y = fmaf(v[u], g[u], y);
+    }
     return y;
 }
 
-__global__ void __launch_bounds__(KB, 4) k_bicgstab_mixed(BicgMixedArgs a) {
-    const int n = a.A.n;
-    const int T = gridDim.x * KB;
-    const int t0 = blockIdx.x * KB + threadIdx.x;
-    const bool lead = threadIdx.x == 0;
+// One CTA per SM owns a contiguous range of slices; three grid sums (grid_all.cuh) and two
+// bare barriers an iteration, the FP32 matrix in shared memory where it fits (RES).  s takes
+// r's storage.  Below 300k rows the grid-wide steps bound it: 256,000 rows of a hex mesh took
+// 48 us an iteration on 250 blocks of 256 with FP64 shuffle trees and four sums, here 30.
+constexpr int BICG_NT = 512;
+extern __shared__ __align__(16) unsigned char g_bicg_rows[];
+
+template <bool RES>
+__global__ void __launch_bounds__(BICG_NT, 1) k_bicgstab_mixed(BicgMixedArgs a, int wmax, int ld) {
+    const int n = a.A.n, tid = threadIdx.x;
+    const bool lead = tid == 0;
     int *err = &a.info->err;
-    RedCtx rc{a.partials, (int)gridDim.x, 0};
+    const int sb = (int)((long long)a.A.nslices * blockIdx.x / gridDim.x);
+    const int se = (int)((long long)a.A.nslices * (blockIdx.x + 1) / gridDim.x);
+    const int R0 = sb * 32, R1 = min(se * 32, n);
+    constexpr int RB = 4;
     __shared__ BicgMixedState S;
+    AllCtx gc = all_ctx(a.slots);
+    all_init();
+    float *mval = reinterpret_cast<float *>(g_bicg_rows);
+    int *mcol = reinterpret_cast<int *>(mval + (size_t)wmax * ld);
+    if (RES) {
+        for (int i = R0 + tid; i < R1; i += BICG_NT) {
+            const int s = i >> 5, w = __ldg(a.A.sl_w + s), e = __ldg(a.A.sl_ptr + s) + (i & 31);
+            for (int k = 0; k < w; ++k) {
+                const int c = __ldg(a.A.col + e + 32 * k);
+                mval[k * ld + i - R0] = (float)(__ldg(a.A.val + e + 32 * k) * __ldg(a.dinv + c));
+                mcol[k * ld + i - R0] = c;
+            }
+        }
+    }
+    float *__restrict__ r = a.r, *__restrict__ rt = a.rt, *__restrict__ p = a.p, *__restrict__ v = a.v,
+                        *__restrict__ t = a.t, *__restrict__ ev = a.e;
     // FP64 residual of x into r (FP32), rt = r, e = p = v = 0; ||b||^2 (first
     // call) and ||b - A x||^2.  The lead thread then restarts the inner process.
     auto residual = [&](bool first) -> bool {
-        double v2[2] = {0.0, 0.0}, rf2 = 0.0;
-        for (int i = t0; i < n; i += T) {
+        double v2[2] = {0.0, 0.0};
+        for (int i = R0 + tid; i < R1; i += BICG_NT) {
             const double bi = a.b[i];
             const double ri = bi - row_dot(a.A, i, a.x);
             a.r64[i] = ri;
             if (first) v2[0] = fma(bi, bi, v2[0]);
             v2[1] = fma(ri, ri, v2[1]);
         }
-        if (!grid_reduce_t0<2>(v2, rc, a.gb, err)) return false;
-        if (lead) S.sig = pow2_scale(v2[1]);  // the FP32 vectors hold sig r (exact scaling)
-        __syncthreads();
-        {
-            const double sg = S.sig;
-            float f2 = 0.f;
-            for (int i = t0; i < n; i += T) {
-                const float rf = (float)(sg * a.r64[i]);
-                a.r[i] = rf;
-                a.rt[i] = rf;
-                a.e[i] = 0.f;
-                a.p[i] = 0.f;
-                a.v[i] = 0.f;
-                f2 = fmaf(rf, rf, f2);
-            }
-            double v1[1] = {(double)f2};
-            if (!grid_reduce_t0<1>(v1, rc, a.gb, err)) return false;
-            rf2 = v1[0];
+        if (!all_sum<2>(v2, 0, gc, err, [&](int k, double s) {
+                S.sum[k] = s;
+                if (k == 1) S.sig = pow2_scale(s);  // the FP32 vectors hold sig r (exact scaling)
+            })) return false;
+        const double sg = S.sig;
+        float f2 = 0.f;
+        for (int i = R0 + tid; i < R1; i += BICG_NT) {
+            const float rf = (float)(sg * a.r64[i]);
+            r[i] = rf;
+            rt[i] = rf;
+            ev[i] = 0.f;
+            p[i] = 0.f;
+            v[i] = 0.f;
+            f2 = fmaf(rf, rf, f2);
         }
-        if (lead) {
-            if (first) {
-                S.bb = v2[0] == 0.0 ? 1.0 : v2[0];
-                S.thr = a.eps * a.eps * S.bb;
-                S.it = 0;
-                S.upd = 0;
-                S.stall = 0;
-                S.status = DEV_OK;
-                S.done = 0;
-                S.rr_ref = v2[1];
-            } else {
-                ++S.upd;
-                S.stall = v2[1] < S.rr_ref ? 0 : S.stall + 1;
-                S.rr_ref = fmin(S.rr_ref, v2[1]);
-            }
-            S.rr64 = v2[1];
-            S.r0in = rf2;
-            S.rho = rf2;  // rt . r with rt = r, in the FP32 inner precision (sig^2 units)
-            S.rho_prev = S.alpha = S.omg = 1.0;
-            S.inner = 0;
-            if (!isfinite(v2[1])) { S.status = DEV_NONFINITE; S.done = 1; }
-            else if (v2[1] < S.thr) S.done = 1;
-            else if (S.stall >= 3) { S.status = DEV_STALLED; S.done = 1; }  // FP64 takes over
-            else if (S.it >= a.maxit) { S.status = DEV_MAXITER; S.done = 1; }
-        }
-        __syncthreads();
+        double v1[1] = {(double)f2};
+        if (!all_sum<1>(v1, 2, gc, err, [&](int, double rf2) {
+                const double rr = S.sum[1];
+                if (first) {
+                    S.bb = S.sum[0] == 0.0 ? 1.0 : S.sum[0];
+                    S.thr = a.eps * a.eps * S.bb;
+                    S.it = 0;
+                    S.upd = 0;
+                    S.stall = 0;
+                    S.status = DEV_OK;
+                    S.done = 0;
+                    S.rr_ref = rr;
+                } else {
+                    ++S.upd;
+                    S.stall = rr < S.rr_ref ? 0 : S.stall + 1;
+                    S.rr_ref = fmin(S.rr_ref, rr);
+                }
+                S.rr64 = rr;
+                S.r0in = rf2;
+                S.rho = rf2;  // rt . r with rt = r, in the FP32 inner precision (sig^2 units)
+                S.rho_prev = S.alpha = S.omg = 1.0;
+                S.inner = 0;
+                if (!isfinite(rr)) { S.status = DEV_NONFINITE; S.done = 1; }
+                else if (rr < S.thr) S.done = 1;
+                else if (S.stall >= 3) { S.status = DEV_STALLED; S.done = 1; }  // FP64 takes over
+                else if (S.it >= a.maxit) { S.status = DEV_MAXITER; S.done = 1; }
+            })) return false;
         return true;
     };
     // x += M^-1 e / sig in FP64, then the FP64 residual
     auto update = [&]() -> bool {
         const double isg = 1.0 / S.sig;
-        for (int i = t0; i < n; i += T) a.x[i] = fma(a.dinv[i] * isg, (double)a.e[i], a.x[i]);
-        if (!grid_sync(a.gb, err)) return false;
+        for (int i = R0 + tid; i < R1; i += BICG_NT) a.x[i] = fma(a.dinv[i] * isg, (double)ev[i], a.x[i]);
+        if (!all_sync(gc, err)) return false;
         return residual(false);
     };
     if (!residual(true)) return;
-    const float *__restrict__ sv = a.sv32;
     const double d2 = a.inner_tol * a.inner_tol;
     for (;;) {
         if (S.done) break;
@@ -828,88 +923,82 @@ __global__ void __launch_bounds__(KB, 4) k_bicgstab_mixed(BicgMixedArgs a) {
         {
             const float beta = (float)S.beta, omg = (float)S.omg;
             const bool first = S.inner == 1;
-            for (int i = t0; i < n; i += T)
-                a.p[i] = first ? a.r[i] : fmaf(beta, fmaf(-omg, a.v[i], a.p[i]), a.r[i]);
+#pragma unroll RB
+            for (int i = R0 + tid; i < R1; i += BICG_NT)
+                p[i] = first ? r[i] : fmaf(beta, fmaf(-omg, v[i], p[i]), r[i]);
         }
-        if (!grid_sync(a.gb, err)) return;
+        if (!all_sync(gc, err)) return;
         // v = A M^-1 p ; rt . v
         {
             float f = 0.f;
-            for (int i = t0; i < n; i += T) {
-                const float y = row_dot32(a.A, sv, i, a.p);
-                a.v[i] = y;
-                f = fmaf(a.rt[i], y, f);
+            for (int i = R0 + tid; i < R1; i += BICG_NT) {
+                const float y = bicg_row32<RES>(a, mval, mcol, ld, i, i - R0, p);
+                v[i] = y;
+                f = fmaf(rt[i], y, f);
             }
             double red[1] = {(double)f};
-            if (!grid_reduce_t0<1>(red, rc, a.gb, err)) return;
-            if (lead) {
-                S.act = red[0] != 0.0;  // 0: the recurrence broke down, update and restart
-                if (S.act) S.alpha = S.rho / red[0];
-            }
-            __syncthreads();
+            if (!all_sum<1>(red, 3, gc, err, [&](int, double s) {
+                    S.act = s != 0.0;  // 0: the recurrence broke down, update and restart
+                    if (S.act) S.alpha = S.rho / s;
+                })) return;
         }
         if (!S.act) {
             if (!update()) return;
             continue;
         }
-        // s = r - alpha v ; ||s||
+        // s = r - alpha v
         {
             const float alpha = (float)S.alpha;
-            float f = 0.f;
-            for (int i = t0; i < n; i += T) {
-                const float si = fmaf(-alpha, a.v[i], a.r[i]);
-                a.s[i] = si;
-                f = fmaf(si, si, f);
+#pragma unroll RB
+            for (int i = R0 + tid; i < R1; i += BICG_NT) r[i] = fmaf(-alpha, v[i], r[i]);
+        }
+        if (!all_sync(gc, err)) return;
+        // t = A M^-1 s ; t.s, t.t, s.s
+        {
+            float f0 = 0.f, f1 = 0.f, f2 = 0.f;
+            for (int i = R0 + tid; i < R1; i += BICG_NT) {
+                const float y = bicg_row32<RES>(a, mval, mcol, ld, i, i - R0, r);
+                const float si = r[i];
+                t[i] = y;
+                f0 = fmaf(y, si, f0);
+                f1 = fmaf(y, y, f1);
+                f2 = fmaf(si, si, f2);
             }
-            double red[1] = {(double)f};
-            if (!grid_reduce_t0<1>(red, rc, a.gb, err)) return;
+            double red[3] = {(double)f0, (double)f1, (double)f2};
+            if (!all_sum<3>(red, 4, gc, err, [&](int k, double s) { S.sum[k] = s; })) return;
             if (lead) {
-                S.snorm2 = red[0];
-                S.early = red[0] <= d2 * S.r0in;
+                S.early = S.sum[2] <= d2 * S.r0in;
+                S.omg = S.sum[1] != 0.0 ? S.sum[0] / S.sum[1] : 0.0;
             }
             __syncthreads();
         }
+        const float alpha = (float)S.alpha, omg = (float)S.omg;
         if (S.early) {  // e += alpha p, then the FP64 update
-            const float alpha = (float)S.alpha;
-            for (int i = t0; i < n; i += T) a.e[i] = fmaf(alpha, a.p[i], a.e[i]);
+            for (int i = R0 + tid; i < R1; i += BICG_NT) ev[i] = fmaf(alpha, p[i], ev[i]);
             if (!update()) return;
             continue;
         }
-        // t = A M^-1 s ; t.s, t.t
-        {
-            float f0 = 0.f, f1 = 0.f;
-            for (int i = t0; i < n; i += T) {
-                const float y = row_dot32(a.A, sv, i, a.s);
-                a.t[i] = y;
-                f0 = fmaf(y, a.s[i], f0);
-                f1 = fmaf(y, y, f1);
-            }
-            double red[2] = {(double)f0, (double)f1};
-            if (!grid_reduce_t0<2>(red, rc, a.gb, err)) return;
-            if (lead) S.omg = red[1] != 0.0 ? red[0] / red[1] : 0.0;
-            __syncthreads();
-        }
         // e += alpha p + omega s ; r = s - omega t ; r.r, rt.r
         {
-            const float alpha = (float)S.alpha, omg = (float)S.omg;
             float f0 = 0.f, f1 = 0.f;
-            for (int i = t0; i < n; i += T) {
-                const float si = a.s[i];
-                a.e[i] = fmaf(alpha, a.p[i], fmaf(omg, si, a.e[i]));
-                const float ri = fmaf(-omg, a.t[i], si);
-                a.r[i] = ri;
+#pragma unroll RB
+            for (int i = R0 + tid; i < R1; i += BICG_NT) {
+                const float si = r[i];
+                ev[i] = fmaf(alpha, p[i], fmaf(omg, si, ev[i]));
+                const float ri = fmaf(-omg, t[i], si);
+                r[i] = ri;
                 f0 = fmaf(ri, ri, f0);
-                f1 = fmaf(a.rt[i], ri, f1);
+                f1 = fmaf(rt[i], ri, f1);
             }
             double red[2] = {(double)f0, (double)f1};
-            if (!grid_reduce_t0<2>(red, rc, a.gb, err)) return;
+            if (!all_sum<2>(red, 7, gc, err, [&](int k, double s) { S.sum[k] = s; })) return;
             if (lead) {
                 S.rho_prev = S.rho;
-                S.rho = red[1];
+                S.rho = S.sum[1];
                 // FP64 update once the FP32 residual fell by inner_tol, at the
                 // iteration cap, or when the next step would divide by zero
-                S.act = !(red[0] <= d2 * S.r0in || S.it >= a.maxit || S.omg == 0.0 || S.rho == 0.0 ||
-                          !(red[0] == red[0]));
+                S.act = !(S.sum[0] <= d2 * S.r0in || S.it >= a.maxit || S.omg == 0.0 || S.rho == 0.0 ||
+                          !(S.sum[0] == S.sum[0]));
             }
             __syncthreads();
         }
@@ -933,7 +1022,7 @@ void KrylovWork::ensure(int n_, int nrhs_, int max_blocks_, cudaStream_t st) {
     size_t m = (size_t)n * nrhs;
     r.alloc(m); rt.alloc(m); p.alloc(m); v.alloc(m); s.alloc(m); t.alloc(m);
     dinv.alloc(m);
-    partials.alloc((size_t)8 * NVMAX * max_blocks);  // also the 4-word exact-sum partials
+    partials.alloc((size_t)8 * NVMAX * max_blocks);  // also 2 x 9 sums, and the 4-word exact-sum partials
     barrier.alloc(1);
     barrier.zero(st);
     slots.alloc(AX_WORDS);
@@ -1112,19 +1201,22 @@ void bicgstab_solve_mixed(const SellDev &A, const double *val, const double *b, 
                           KrylovWork &w, SolveInfo *info, cudaStream_t st) {
     const int n = A.n;
     if (n == 0) return;
-    static int maxb = 0;
-    if (!maxb) maxb = coresident_blocks(k_bicgstab_mixed);
-    int mb = maxb;
-    if (w.sm_cap > 0) mb = std::min(mb, w.sm_cap * std::max(1, maxb / num_sms()));
-    w.ensure(n, 1, std::max(bicg_max_blocks(-1, false), maxb), st);
+    // the FP32 matrix stays in shared memory wherever it fits
+    constexpr unsigned budget = 200 * 1024;
+    const int cap = std::min(w.sm_cap > 0 ? std::min(w.sm_cap, num_sms()) : num_sms(), AX_MAX_BLOCKS);
+    const int G = std::max(1, std::min(A.nslices, cap));
+    int wmax = A.wmax, ld = 32 * ((A.nslices + G - 1) / G);
+    const size_t want = (size_t)ld * wmax * 8;
+    const bool res = want <= budget;
+    w.ensure(n, 1, bicg_max_blocks(-1, false), st);
     w.ensure32(n, st);
     if (w.rt32.size() < (size_t)n) {
-        w.rt32.alloc(n); w.v32.alloc(n); w.s32.alloc(n); w.t32.alloc(n);
+        w.rt32.alloc(n); w.v32.alloc(n); w.t32.alloc(n);
     }
-    if (w.sval32.size() < (size_t)A.nnz) w.sval32.alloc(A.nnz);
     SellView V = view(A, val);
     { k_jacobi_dinv<<<(n + KB - 1) / KB, KB, 0, st>>>(V, o.omega, o.jacobi ? 1 : 0, w.dinv.get()); ++::sysu::g_launches; }
-    if (A.nnz > 0) {
+    if (A.nnz > 0 && !res) {
+        if (w.sval32.size() < (size_t)A.nnz) w.sval32.alloc(A.nnz);
         k_scale_cols32<<<(unsigned)((A.nnz + KB - 1) / KB), KB, 0, st>>>(A.nnz, A.col.get(), val, w.dinv.get(),
                                                                         w.sval32.get());
         ++::sysu::g_launches;
@@ -1138,17 +1230,16 @@ void bicgstab_solve_mixed(const SellDev &A, const double *val, const double *b, 
     a.dinv = w.dinv.get();
     a.r64 = w.r.get();
     a.r = w.r32.get(); a.rt = w.rt32.get(); a.p = w.p32.get(); a.v = w.v32.get();
-    a.s = w.s32.get(); a.t = w.t32.get(); a.e = w.e32.get();
-    a.partials = w.partials.get();
-    a.gb = w.barrier.get();
+    a.t = w.t32.get(); a.e = w.e32.get();
+    a.slots = w.clear_slots(st);
     a.info = info;
     a.maxit = o.maxit;
     a.eps = o.eps;
     a.inner_tol = o.inner_tol;
-    void *args[] = {&a};
-    const int G = grid_for(n, bicg_blocks_for(n, mb));
-    SYSU_CUDA(cudaMemsetAsync(w.barrier.get(), 0, sizeof(GridBarrier), st));  // grid_sync starts from 0
-    SYSU_CUDA(cudaLaunchCooperativeKernel((const void *)k_bicgstab_mixed, dim3(G), dim3(KB), args, 0, st));
+    const void *kern = res ? (const void *)k_bicgstab_mixed<true> : (const void *)k_bicgstab_mixed<false>;
+    if (res) SYSU_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget));
+    void *args[] = {&a, &wmax, &ld};
+    SYSU_CUDA(cudaLaunchCooperativeKernel(kern, dim3(G), dim3(BICG_NT), args, res ? want : 0, st));
     ++::sysu::g_launches;
     // FP64 takes over from the current x if the FP32 refinement stalled (the
     // launch returns at once otherwise)
