@@ -283,7 +283,7 @@ const char *sysu_mg_last_error(void);
  * own DEVICE buffers: CSR d_rowptr[n+1], d_col[nnz], d_val[nnz] (0-based), d_b[n],
  * d_x[n] (x0 in, solution out); same algorithm and stopping test as
  * sysu_csr_solve with method CG and precond Jacobi.  Scratch is one static
- * device array of 8.4 MB, present on every GPU that loads the library:
+ * device array of 4.2 MB, present on every GPU that loads the library:
  *   - n must be <= SYSU_NOALLOC_MAX_ROWS, larger systems are rejected
  *     (SYSU_ERR_INPUT, message in sysu_noalloc_last_error());
  *   - every call shares the array; calls that overlap on the GPU race on it;

@@ -12,7 +12,7 @@
 //
 // Limits and rules (also in include/sysu_cfd.h):
 // * at most SYSU_NOALLOC_MAX_ROWS rows (262,144); larger systems are rejected;
-// * the array costs 8.4 MB on every GPU that loads the library, until exit;
+// * the array costs 4.2 MB on every GPU that loads the library, until exit;
 // * all calls share the array and it keeps the last call's contents: each call
 //   clears what must start at zero (barrier counter, status words) itself;
 //   calls that overlap on the GPU (two streams, two threads) race on it;
@@ -36,20 +36,22 @@
 #include <string>
 
 #include "../../include/sysu_cfd.h"
-#include "device.hpp"
+#include "grid_all.cuh"
 
 namespace {
 
 constexpr int NA_MAX_ROWS = 262144;
-constexpr int NA_KB = 256;
-constexpr int NA_MAX_BLOCKS = 1024;
-constexpr int NA_NV = 3;
+constexpr int NA_KB = 256;                 // threads of the check kernel
+constexpr int NA_NT = 512;                 // threads of a solver CTA
+constexpr int NA_ROWS = 4;                 // rows a thread at most
+constexpr unsigned NA_SMEM = 200 * 1024;   // matrix entries a CTA keeps in shared memory
+constexpr int NA_ENTRIES = NA_SMEM / 12;
 
 // what a malformed CSR row was found to hold (low two bits of NaHeader::bad)
 enum NaBad : int { NA_BAD_NONE = 0, NA_BAD_ROWPTR = 1, NA_BAD_COL = 2, NA_BAD_DIAG = 3 };
 
 struct NaHeader {  // at the start of the array, cleared by every call
-    sysu::GridBarrier barrier;
+    int unused[2];
     int err;
     int status;
     int iters;
@@ -60,10 +62,11 @@ struct NaHeader {  // at the start of the array, cleared by every call
     unsigned long long bad;
 };
 
-// layout in doubles: header (64 B) | r | p | q | dinv | partials (2*NA_NV*NA_MAX_BLOCKS)
-constexpr size_t NA_HDR = 8;
-static_assert(sizeof(NaHeader) <= NA_HDR * sizeof(double), "NaHeader must fit its 64-byte slot");
-constexpr size_t NA_DOUBLES = NA_HDR + 4 * (size_t)NA_MAX_ROWS + 2 * (size_t)NA_NV * NA_MAX_BLOCKS;
+// layout in doubles: header (64 B) | z | dinv | exchange area of the grid sums
+constexpr size_t NA_HDR = 16;
+static_assert(sizeof(NaHeader) <= NA_HDR * sizeof(double), "NaHeader must fit its slot");
+constexpr size_t NA_SLOTS = NA_HDR + 2 * (size_t)NA_MAX_ROWS;
+constexpr size_t NA_DOUBLES = NA_SLOTS + sysu::AX_WORDS;
 
 static __device__ __align__(256) double g_noalloc_scratch[NA_DOUBLES];
 
@@ -77,39 +80,6 @@ struct NaArgs {
     double eps;
     double *base;  // device address of g_noalloc_scratch
 };
-
-__shared__ double na_red_smem[NA_NV * (NA_KB / 32)];
-__shared__ double na_red_res[NA_NV];
-
-template <int NV>
-__device__ bool na_reduce(double (&v)[NV], double *partials, int &parity, sysu::GridBarrier *gb, int *err) {
-    sysu::block_sum<NV>(v, na_red_smem);
-    double *buf = partials + (size_t)parity * NA_NV * gridDim.x;
-    parity ^= 1;
-    if (threadIdx.x == 0)
-        for (int k = 0; k < NV; ++k) buf[(size_t)k * gridDim.x + blockIdx.x] = v[k];
-    if (!sysu::grid_sync(gb, err)) return false;
-    if (threadIdx.x < 32)
-        for (int k = 0; k < NV; ++k) {
-            double s = sysu::warp_sum_partials(buf + (size_t)k * gridDim.x, gridDim.x);
-            if (threadIdx.x == 0) na_red_res[k] = s;
-        }
-    __syncthreads();
-    for (int k = 0; k < NV; ++k) v[k] = na_red_res[k];
-    __syncthreads();
-    return true;
-}
-
-// Row i of A times x.  Entries whose column lies outside 0..n-1 are skipped
-// (k_na_dinv has already reported them, and the solve does not run).
-__device__ __forceinline__ double csr_row(const NaArgs &a, int i, const double *x) {
-    double s = 0.0;
-    for (int k = a.rowptr[i]; k < a.rowptr[i + 1]; ++k) {
-        int c = a.col[k];
-        if ((unsigned)c < (unsigned)a.n) s += a.val[k] * x[c];
-    }
-    return s;
-}
 
 constexpr unsigned long long NA_GOOD = ~0ull;
 
@@ -141,76 +111,153 @@ __global__ void k_na_dinv(NaArgs a) {
         na_report(h, i, kind);
         d = 1.0;
     }
-    a.base[NA_HDR + 3 * (size_t)NA_MAX_ROWS + i] = a.omega / d;
+    a.base[NA_HDR + (size_t)NA_MAX_ROWS + i] = a.omega / d;
 }
 
-// Same recurrences as the SELL persistent CG (Templates Fig. 2.5, Jacobi).
-__global__ void __launch_bounds__(NA_KB) k_na_cg(NaArgs a) {
+// Same recurrences as the SELL persistent CG (Templates Fig. 2.5, Jacobi) with w = A z and
+// q = w + beta q in place of the product of p, so that an iteration has two grid-wide steps.
+// Row i's product takes its entries in the caller's order.
+//
+// One CTA per SM owns a contiguous range of rows: their vectors in registers, their part of
+// the caller's CSR in shared memory when it fits (17,066 entries a CTA, so always for the
+// 7-entry rows of a hex mesh; a CTA whose rows hold more reads the caller's arrays).  z, which
+// other CTAs gather, is the only vector in memory.  Latency bounds it at every size up to the
+// limit: two sums (grid_all.cuh) and two FP64 divisions an iteration.  1,716 rows on 7 blocks
+// of 256 threads, with three barriers and FP64 shuffle trees, square roots and divisions in
+// every thread, took 13.7 us an iteration; on 54 CTAs here 6.7 (238,080 rows: 13.0).
+template <int R>
+__global__ void __launch_bounds__(NA_NT, 1) k_na_cg(NaArgs a) {
     NaHeader *h = reinterpret_cast<NaHeader *>(a.base);
-    double *r = a.base + NA_HDR, *p = r + NA_MAX_ROWS, *q = p + NA_MAX_ROWS, *dinv = q + NA_MAX_ROWS;
-    double *partials = dinv + NA_MAX_ROWS;
-    const int n = a.n, T = gridDim.x * NA_KB, t0 = blockIdx.x * NA_KB + threadIdx.x;
+    double *zg = a.base + NA_HDR;
+    const double *dinv = zg + NA_MAX_ROWS;
+    const int n = a.n, tid = threadIdx.x;
     // k_na_dinv ran before this launch on the same stream: every block reads the
     // same check result, so on a malformed matrix all leave together, before any
     // row loop or barrier
     if (__ldcg(&h->bad) != NA_GOOD) return;
-    int parity = 0;
+    const int groups = (n + 31) / 32;
+    const int R0 = 32 * (int)((long long)groups * blockIdx.x / gridDim.x);
+    const int R1 = min(n, 32 * (int)((long long)groups * (blockIdx.x + 1) / gridDim.x));
+    sysu::AllCtx c = sysu::all_ctx(reinterpret_cast<unsigned long long *>(a.base + NA_SLOTS));
+    sysu::all_init();
+    extern __shared__ __align__(16) unsigned char na_smem[];
+    const int E0 = a.rowptr[R0], nent = a.rowptr[R1] - E0;
+    const bool res = nent <= NA_ENTRIES;
+    double *sval = reinterpret_cast<double *>(na_smem);
+    int *scol = reinterpret_cast<int *>(sval + (res ? nent : 0));
+    if (res) {
+        for (int k = tid; k < nent; k += NA_NT) {
+            sval[k] = a.val[E0 + k];
+            scol[k] = a.col[E0 + k];
+        }
+    }
+    const double *mv = res ? sval : a.val + E0;
+    const int *mc = res ? scol : a.col + E0;
+    __shared__ double s_rr, s_rho, s_thr, s_bb, s_alpha, s_beta;
+    __shared__ int s_brk;
+    int *err = &h->err;
+    double x[R], r[R], p[R], q[R], d[R];
+    int e0[R], len[R];
     double v3[3] = {0.0, 0.0, 0.0};
-    for (int i = t0; i < n; i += T) {
-        double bi = a.b[i];
-        double ri = bi - csr_row(a, i, a.x);
-        r[i] = ri;
-        v3[0] += bi * bi;
-        v3[1] += ri * ri;
-        v3[2] += ri * (dinv[i] * ri);
+#pragma unroll
+    for (int u = 0; u < R; ++u) {
+        const int i = R0 + tid + u * NA_NT;
+        x[u] = r[u] = p[u] = q[u] = d[u] = 0.0;
+        e0[u] = len[u] = 0;
+        if (i >= R1) continue;
+        const int k0 = a.rowptr[i], k1 = a.rowptr[i + 1];
+        e0[u] = k0 - E0;
+        len[u] = k1 - k0;
+        double s = 0.0;
+        for (int k = k0; k < k1; ++k) s = fma(a.val[k], a.x[a.col[k]], s);
+        const double bi = a.b[i];
+        x[u] = a.x[i];
+        d[u] = dinv[i];
+        r[u] = bi - s;
+        const double z = d[u] * r[u];
+        zg[i] = z;
+        v3[0] = fma(bi, bi, v3[0]);
+        v3[1] = fma(r[u], r[u], v3[1]);
+        v3[2] = fma(r[u], z, v3[2]);
     }
-    if (!na_reduce<3>(v3, partials, parity, &h->barrier, &h->err)) return;
-    double bnorm = sqrt(v3[0]);
-    if (bnorm == 0.0) bnorm = 1.0;
-    double res = sqrt(v3[1]) / bnorm, rho = v3[2], rho_prev = 1.0;
+    if (!sysu::all_sum<3>(v3, 0, c, err, [&](int k, double s) {
+            if (k == 0) {
+                s_bb = s == 0.0 ? 1.0 : s;
+                s_thr = a.eps * a.eps * s_bb;
+            } else if (k == 1) {
+                s_rr = s;
+            } else {
+                s_rho = s;
+                s_beta = 0.0;
+            }
+        })) return;
     int it = 0, status = sysu::DEV_OK;
-    while (!(res < a.eps) && it < a.maxit) {
-        if (!isfinite(res)) { status = sysu::DEV_NONFINITE; break; }
+    while (!(s_rr < s_thr) && it < a.maxit) {
+        if (!isfinite(s_rr)) { status = sysu::DEV_NONFINITE; break; }
         ++it;
-        double beta = (it == 1) ? 0.0 : rho / rho_prev;
-        for (int i = t0; i < n; i += T) {
-            double z = dinv[i] * r[i];
-            p[i] = (it == 1) ? z : z + beta * p[i];
-        }
-        if (!sysu::grid_sync(&h->barrier, &h->err)) return;
+        const double beta = s_beta;
         double v1[1] = {0.0};
-        for (int i = t0; i < n; i += T) {
-            double qi = csr_row(a, i, p);
-            q[i] = qi;
-            v1[0] += p[i] * qi;
+#pragma unroll
+        for (int u = 0; u < R; ++u) {
+            if (len[u] == 0) continue;
+            double w = 0.0;
+            int k = 0;
+            for (; k + 4 <= len[u]; k += 4) {  // four entries' loads before their FMAs
+                const int e = e0[u] + k;
+                const double g0 = zg[mc[e]], g1 = zg[mc[e + 1]], g2 = zg[mc[e + 2]], g3 = zg[mc[e + 3]];
+                w = fma(mv[e], g0, w);
+                w = fma(mv[e + 1], g1, w);
+                w = fma(mv[e + 2], g2, w);
+                w = fma(mv[e + 3], g3, w);
+            }
+            for (; k < len[u]; ++k) w = fma(mv[e0[u] + k], zg[mc[e0[u] + k]], w);
+            p[u] = fma(beta, p[u], d[u] * r[u]);
+            q[u] = fma(beta, q[u], w);
+            v1[0] = fma(p[u], q[u], v1[0]);
         }
-        if (!na_reduce<1>(v1, partials, parity, &h->barrier, &h->err)) return;
-        if (v1[0] == 0.0) { status = sysu::DEV_BREAKDOWN; break; }
-        double alpha = rho / v1[0];
+        if (!sysu::all_sum<1>(v1, 3, c, err, [&](int, double pq) {
+                s_brk = pq == 0.0;
+                s_alpha = pq == 0.0 ? 0.0 : s_rho / pq;
+            })) return;
+        if (s_brk) { status = sysu::DEV_BREAKDOWN; break; }
+        const double alpha = s_alpha;
         double v2[2] = {0.0, 0.0};
-        for (int i = t0; i < n; i += T) {
-            a.x[i] += alpha * p[i];
-            double ri = r[i] - alpha * q[i];
-            r[i] = ri;
-            v2[0] += ri * ri;
-            v2[1] += ri * (dinv[i] * ri);
+#pragma unroll
+        for (int u = 0; u < R; ++u) {
+            const int i = R0 + tid + u * NA_NT;
+            if (i >= R1) continue;
+            x[u] = fma(alpha, p[u], x[u]);
+            r[u] = fma(-alpha, q[u], r[u]);
+            const double z = d[u] * r[u];
+            zg[i] = z;
+            v2[0] = fma(r[u], r[u], v2[0]);
+            v2[1] = fma(r[u], z, v2[1]);
         }
-        if (!na_reduce<2>(v2, partials, parity, &h->barrier, &h->err)) return;
-        res = sqrt(v2[0]) / bnorm;
-        rho_prev = rho;
-        rho = v2[1];
+        if (!sysu::all_sum<2>(v2, 4, c, err, [&](int k, double s) {
+                if (k == 0) {
+                    s_rr = s;
+                } else {
+                    s_beta = s / s_rho;
+                    s_rho = s;
+                }
+            })) return;
     }
-    if (status == sysu::DEV_OK && !(res < a.eps)) status = isfinite(res) ? sysu::DEV_MAXITER : sysu::DEV_NONFINITE;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+#pragma unroll
+    for (int u = 0; u < R; ++u) {
+        const int i = R0 + tid + u * NA_NT;
+        if (i < R1) a.x[i] = x[u];
+    }
+    if (blockIdx.x == 0 && tid == 0) {
+        if (status == sysu::DEV_OK && !(s_rr < s_thr)) status = isfinite(s_rr) ? sysu::DEV_MAXITER : sysu::DEV_NONFINITE;
         h->status = status;
         h->iters = it;
-        h->res = res;
+        h->res = sqrt(s_rr) / sqrt(s_bb);
     }
 }
 
 thread_local std::string g_na_err;
 std::mutex g_na_mu;
-int g_na_blocks[64] = {0};
+int g_na_blocks[64] = {0};  // SMs of a device, 0: not asked yet
 
 int na_fail(int code, const std::string &m) {
     g_na_err = m;
@@ -251,21 +298,31 @@ int sysu_csr_cg_noalloc(int n, const int *d_rowptr, const int *d_col, const doub
         std::lock_guard<std::mutex> lock(g_na_mu);
         if (!g_na_blocks[dev]) {  // once per device: cooperative-launch occupancy
             int per_sm = 0, sms = 0, coop = 0;
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_na_cg, NA_KB, 0);
+            const void *kernels[] = {(const void *)k_na_cg<1>, (const void *)k_na_cg<2>, (const void *)k_na_cg<NA_ROWS>};
+            for (const void *k : kernels) {
+                if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)NA_SMEM);
+                int ps = 0;
+                if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ps, k, NA_NT, NA_SMEM);
+                per_sm = k == kernels[0] || ps < per_sm ? ps : per_sm;
+            }
             if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
             if (e == cudaSuccess) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
             if (e != cudaSuccess) return na_fail(SYSU_ERR_CUDA, std::string("device query: ") + cudaGetErrorString(e));
             if (!coop || per_sm < 1) return na_fail(SYSU_ERR_CUDA, "cooperative launch unavailable");
-            g_na_blocks[dev] = per_sm * sms < NA_MAX_BLOCKS ? per_sm * sms : NA_MAX_BLOCKS;
+            if ((long long)sms * NA_NT * NA_ROWS < NA_MAX_ROWS)
+                return na_fail(SYSU_ERR_CUDA, "the device has too few SMs for the solver");
+            g_na_blocks[dev] = sms < sysu::AX_MAX_BLOCKS ? sms : sysu::AX_MAX_BLOCKS;
         }
         blocks = g_na_blocks[dev];
     }
-    int G = (n + NA_KB - 1) / NA_KB;
-    if (G > blocks) G = blocks;
+    const int groups = (n + 31) / 32;
+    const int G = groups < blocks ? groups : blocks;
+    const int need = (32 * ((groups + G - 1) / G) + NA_NT - 1) / NA_NT;  // rows a thread
     NaArgs a{n, d_rowptr, d_col, d_val, d_b, d_x, omega, maxit, eps, base};
-    // what must start at zero: the barrier counter and the status words; the
-    // malformed-row key starts at all ones (no row found)
+    // what must start at zero: the exchange area of the grid sums and the status words;
+    // the malformed-row key starts at all ones (no row found)
     e = cudaMemsetAsync(base, 0, offsetof(NaHeader, bad), st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(base + NA_SLOTS, 0, sysu::AX_WORDS * sizeof(double), st);
     if (e == cudaSuccess)
         e = cudaMemsetAsync(reinterpret_cast<char *>(base) + offsetof(NaHeader, bad), 0xff, sizeof(unsigned long long),
                             st);
@@ -274,7 +331,9 @@ int sysu_csr_cg_noalloc(int n, const int *d_rowptr, const int *d_col, const doub
     e = cudaGetLastError();
     if (e != cudaSuccess) return na_fail(SYSU_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(e));
     void *args[] = {&a};
-    e = cudaLaunchCooperativeKernel((const void *)k_na_cg, dim3(G), dim3(NA_KB), args, 0, st);
+    const void *kern = need <= 1 ? (const void *)k_na_cg<1>
+                                 : need <= 2 ? (const void *)k_na_cg<2> : (const void *)k_na_cg<NA_ROWS>;
+    e = cudaLaunchCooperativeKernel(kern, dim3(G), dim3(NA_NT), args, NA_SMEM, st);
     if (e != cudaSuccess) return na_fail(SYSU_ERR_CUDA, std::string("cooperative launch: ") + cudaGetErrorString(e));
     NaHeader h;
     e = cudaMemcpyAsync(&h, base, sizeof(NaHeader), cudaMemcpyDeviceToHost, st);

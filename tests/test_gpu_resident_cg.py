@@ -69,3 +69,44 @@ def test_resident_cg_cap_breakdown_and_no_preconditioner():
     bad[7] = np.nan
     _, it, _, status = csr_solve(rp, c, v, bad, method="CG", maxit=10, eps=EPS)
     assert it == 0 and status == 4
+
+
+@pytest.mark.parametrize("n", [1, 32, 33, 4864, 77824, 77857, 155680, 262144])
+@pytest.mark.parametrize("wide", [0, 20000])
+def test_noalloc_cg_sizes(n, wide):
+    """sysu_csr_cg_noalloc at the sizes where its launch changes (one CTA, 1, 2 and 4 rows a
+    thread, the largest), and with one row so long that its CTA reads the caller's arrays."""
+    torch = pytest.importorskip("torch")
+    import ctypes as C
+
+    from sysu_cfd_heat_gb300._lib import LIB_PATH
+
+    if wide and n < 2 * wide:
+        pytest.skip("the row needs more columns")
+    rng = np.random.default_rng(n)
+    a = np.arange(n - 1)
+    w = rng.uniform(0.5, 1.5, n - 1)
+    far = np.arange(n - wide, n) if wide else np.zeros(0, np.int64)  # couplings of row 0
+    g = rng.uniform(0.5, 1.0, far.size) / max(wide, 1)
+    rows = np.concatenate([a, a + 1, np.zeros(far.size, np.int64), far])
+    cols = np.concatenate([a + 1, a, far, np.zeros(far.size, np.int64)])
+    off = np.concatenate([w, w, g, g])
+    diag = 1.1 * np.maximum(np.bincount(rows, off, n), 1.0)
+    r, c = np.concatenate([np.arange(n), rows]), np.concatenate([np.arange(n), cols])
+    v = np.concatenate([diag, -off])
+    order = np.lexsort((c, r))
+    r, c, v = r[order], c[order].astype(np.int32), v[order]
+    rp = np.concatenate([[0], np.cumsum(np.bincount(r, minlength=n))]).astype(np.int32)
+    x = rng.standard_normal(n)
+    b = np.add.reduceat(v * x[c], rp[:-1])
+    fn = C.CDLL(LIB_PATH).sysu_csr_cg_noalloc
+    fn.argtypes = [C.c_int] + [C.c_void_p] * 5 + [C.c_int, C.c_double, C.c_double] + [C.c_void_p] * 4
+    d = [torch.from_numpy(t).cuda() for t in (rp, c, v, b)]
+    y = torch.zeros(n, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    it, res, st = C.c_int(), C.c_double(), C.c_int()
+    assert fn(n, *(t.data_ptr() for t in d), y.data_ptr(), 1000, EPS, 1.3, None, C.addressof(it), C.addressof(res),
+              C.addressof(st)) == 0
+    assert st.value == 0 and res.value < EPS
+    # cond(A) <= 21 max(d) / min(d) <= 21 * 3.3 / 1.1
+    assert np.linalg.norm(y.cpu().numpy() - x) <= 100 * EPS * np.linalg.norm(x)
