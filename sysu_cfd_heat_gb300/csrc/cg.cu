@@ -90,6 +90,9 @@ struct CgPipeArgs {
     double eps, inner_tol;
     unsigned long long *ts;
     CgPlan plan;
+    // the form with M^-1 behind the scaled one (cg_scaled.cuh): run only if *only_if; null:
+    // always run
+    const int *only_if;
     // FP64 kernel behind a mixed solve: run only if gate->status[0] is
     // DEV_STALLED (the iterations of both are reported); null: always run
     const SolveInfo *gate;
@@ -152,6 +155,14 @@ __shared__ int g_tile_e[CG_TILE_TABLE + 1];
 
 __device__ __forceinline__ int tile_entry(const Part &P, const int *sl_ptr, int t) {
     return t <= CG_TILE_TABLE ? g_tile_e[t] : __ldg(sl_ptr + min(P.sb + t * P.ts, P.se));
+}
+
+// the same for a matrix copy without its diagonal entries (cg_scaled.cuh; the table then
+// holds that copy's entries)
+__device__ __forceinline__ int tile_entry_packed(const Part &P, const int *sl_ptr, int t) {
+    if (t <= CG_TILE_TABLE) return g_tile_e[t];
+    const int s = min(P.sb + t * P.ts, P.se);
+    return __ldg(sl_ptr + s) - 32 * s;
 }
 
 __device__ __forceinline__ int cg_consumers() { return (int)(blockDim.x >> 5) - 1; }
@@ -259,10 +270,13 @@ __device__ __forceinline__ void drain(const Ring &R) {
     }
 }
 
-__device__ __forceinline__ void ring_init(Ring &R, const CgPlan &pl, const Part &P, const int *sl_ptr) {
+__device__ __forceinline__ void ring_init(Ring &R, const CgPlan &pl, const Part &P, const int *sl_ptr,
+                                          bool packed = false) {
     const int nt = P.nt;
-    for (int t = threadIdx.x; t <= min(nt, CG_TILE_TABLE); t += blockDim.x)
-        g_tile_e[t] = __ldg(sl_ptr + min(P.sb + t * P.ts, P.se));
+    for (int t = threadIdx.x; t <= min(nt, CG_TILE_TABLE); t += blockDim.x) {
+        const int s = min(P.sb + t * P.ts, P.se);
+        g_tile_e[t] = __ldg(sl_ptr + s) - (packed ? 32 * s : 0);
+    }
     R.depth = max(1, min(pl.depth, nt));
     R.slot = pl.slot;
     R.cslot = 0;
@@ -570,7 +584,8 @@ __device__ __forceinline__ V s_phase(const Part &P, Ring &R, const SellView &A, 
 template <int WR, bool AHEAD = true>
 __global__ void __launch_bounds__(cg64_threads<WR, AHEAD>(), 1) k_cg_pipe(CgPipeArgs a) {
     constexpr int NT = cg64_threads<WR, AHEAD>();
-    if (a.gate && a.gate->status[0] != DEV_STALLED) return;  // the same word for every block
+    if (a.gate && a.gate->status[0] != DEV_STALLED) return;  // the same words for every block
+    if (a.only_if && !*a.only_if) return;
     const int it_before = a.gate ? a.gate->iters[0] : 0;
     const int n = a.A.n;
     const int tid = threadIdx.x;
@@ -722,6 +737,7 @@ __global__ void __launch_bounds__(cg64_threads<WR, AHEAD>(), 1) k_cg_pipe(CgPipe
 // Convergence is decided on that FP64 residual only.  Per-thread partial dot
 // products run in FP32 over the thread's rows; exact sums across threads.
 __global__ void __launch_bounds__(CGT32, 1) k_cg_mixed_pipe(CgPipeArgs a) {
+    if (a.only_if && !*a.only_if) return;  // the same word for every block
     const int n = a.A.n;
     const int tid = threadIdx.x;
     const bool prod = is_producer();
@@ -960,6 +976,7 @@ __global__ void __launch_bounds__(CGT64, 1) k_spmv_ring(SellView A, const V *val
 }  // namespace sysu
 
 #include "cg_resident.cuh"
+#include "cg_scaled.cuh"
 
 namespace sysu {
 namespace {
@@ -1006,6 +1023,79 @@ int cg_grid(const SellDev &A, const CgPlan &pl, int maxb, int sm_cap) {
 
 }  // namespace
 
+// The scaled form of a streaming solve (cg_scaled.cuh): its matrix copy and its launch.  The
+// caller's launch of the form with M^-1 runs only where the returned word is not 0.  Not for
+// solves capped to a share of the SMs (cases of one CUDA graph), whose second cooperative
+// launch would hold up the graph's other branches.
+template <class V>
+static const int *sym_launch(const SellDev &A, const double *val, const double *b, double *x, const KrylovOpts &o,
+                             KrylovWork &w, SolveInfo *info, const SolveInfo *gate, cudaStream_t st) {
+    constexpr bool fp32 = sizeof(V) == 4;
+    if (!o.jacobi || w.sm_cap > 0) return nullptr;
+    const int n = A.n;
+    if (w.wt.size() < (size_t)n) w.wt.alloc(n);
+    if (w.scol.size() < (size_t)A.nnz) w.scol.alloc(A.nnz);
+    if (!w.sym_bad.size()) w.sym_bad.alloc(1);
+    if (fp32 && w.sval32.size() < (size_t)A.nnz) w.sval32.alloc(A.nnz);
+    if (!fp32 && w.sval.size() < (size_t)A.nnz) w.sval.alloc(A.nnz);
+    CgSymArgs a{};
+    a.A = view(A, val);
+    w.sym_bad.zero(st);
+    k_sym_diag<<<(n + KB - 1) / KB, KB, 0, st>>>(a.A, w.dinv.get(), w.wt.get(), w.sym_bad.get(), gate);
+    V *sv = nullptr;
+    if constexpr (fp32) sv = w.sval32.get();
+    else sv = w.sval.get();
+    k_sym_scale<V><<<(A.nslices * 32 + KB - 1) / KB, KB, 0, st>>>(a.A, w.dinv.get(), sv, w.scol.get(), gate);
+    ::sysu::g_launches += 2;
+    a.val = sv;
+    a.col = w.scol.get();
+    a.s = w.dinv.get();
+    a.wt = w.wt.get();
+    a.bad = w.sym_bad.get();
+    a.b = b;
+    a.x = x;
+    a.slots = w.clear_slots(st);
+    a.info = info;
+    a.maxit = o.maxit;
+    a.eps = o.eps;
+    a.inner_tol = o.inner_tol;
+    a.ts = w.phase_ts;
+    a.gate = gate;
+    check_aligned16({a.val, a.col});
+    const bool narrow = A.wmax <= 5;  // gathers a thread holds: 4 off-diagonals (tets) or 6 (hexes)
+    const void *kern;
+    int threads, maxb;
+    if constexpr (fp32) {
+        static int mb[2] = {0, 0};
+        int &m = mb[narrow ? 0 : 1];
+        kern = narrow ? (const void *)k_cg_mixed_sym<4> : (const void *)k_cg_mixed_sym<6>;
+        if (!m) m = narrow ? cg_max_blocks(k_cg_mixed_sym<4>, SYM_NT32) : cg_max_blocks(k_cg_mixed_sym<6>, SYM_NT32);
+        threads = SYM_NT32;
+        maxb = m;
+        a.r = w.r32.get(); a.p = w.p32.get(); a.q = w.q32.get(); a.y = w.e32.get();
+        a.r64 = w.r.get();
+    } else {
+        static int mb[2] = {0, 0};
+        int &m = mb[narrow ? 0 : 1];
+        kern = narrow ? (const void *)k_cg_sym<4> : (const void *)k_cg_sym<6>;
+        if (!m) m = narrow ? cg_max_blocks(k_cg_sym<4>, SYM_NT) : cg_max_blocks(k_cg_sym<6>, SYM_NT);
+        threads = SYM_NT;
+        maxb = m;
+        a.r = w.r.get(); a.p = w.p.get(); a.q = w.v.get(); a.y = w.t.get();
+    }
+    a.plan = plan_cg(A.wmax - 1, (int)sizeof(V), threads / 32 - 1);
+    void *args[] = {&a};
+    const int G = std::min(cg_grid(A, a.plan, maxb, 0), AX_MAX_BLOCKS);
+    // at least three slots, more up to 118 KB: beyond that the L1 left for the gathers of r
+    // shrinks (2M tets with 512 threads, us an iteration: FP64 50.7 / 49.4 / 49.6 with 4 / 5 / 6
+    // slots of 23 KB; FP32 28.3 / 28.5 with 4 / 5)
+    a.plan.depth = std::max(std::min(a.plan.depth, 3), std::min(a.plan.depth, (int)(118 * 1024 / a.plan.slot)));
+    a.plan.smem = a.plan.depth * a.plan.slot;
+    SYSU_CUDA(cudaLaunchCooperativeKernel(kern, dim3(G), dim3(threads), args, a.plan.smem, st));
+    ++::sysu::g_launches;
+    return w.sym_bad.get();
+}
+
 // The FP64 persistent CG.  gate: see CgPipeArgs (then x is not zeroed and
 // info is not cleared: the solve continues the mixed one's).
 static void cg_launch64(const SellDev &A, const double *val, const double *b, double *x, bool x0_zero,
@@ -1051,10 +1141,11 @@ static void cg_launch64(const SellDev &A, const double *val, const double *b, do
     w.ensure(n, 1, maxb, st);
     check_aligned16({val, A.col.get()});
     SellView V = view(A, val);
-    { k_jacobi_dinv<<<(n + KB - 1) / KB, KB, 0, st>>>(V, o.omega, o.jacobi ? 1 : 0, w.dinv.get()); ++::sysu::g_launches; }
     if (!gate && x0_zero) { k_zero<<<(n + KB - 1) / KB, KB, 0, st>>>(x, n); ++::sysu::g_launches; }
     if (!gate) SYSU_CUDA(cudaMemsetAsync(info, 0, sizeof(SolveInfo), st));
     CgPipeArgs a{};
+    a.only_if = sym_launch<double>(A, val, b, x, o, w, info, gate, st);
+    { k_jacobi_dinv<<<(n + KB - 1) / KB, KB, 0, st>>>(V, o.omega, o.jacobi ? 1 : 0, w.dinv.get()); ++::sysu::g_launches; }
     a.gate = gate;
     a.A = V;
     a.b = b;
@@ -1144,6 +1235,7 @@ void cg_solve_mixed(const SellDev &A, const double *val, const float *val32, con
     if (x0_zero) { k_zero<<<(n + KB - 1) / KB, KB, 0, st>>>(x, n); ++::sysu::g_launches; }
     SYSU_CUDA(cudaMemsetAsync(info, 0, sizeof(SolveInfo), st));
     CgPipeArgs a{};
+    a.only_if = sym_launch<float>(A, val, b, x, o, w, info, nullptr, st);
     a.A = V;
     a.val32 = val32;
     a.b = b;

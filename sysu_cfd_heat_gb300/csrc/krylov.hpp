@@ -77,6 +77,8 @@ struct KrylovWork {
     DevBuf<double> sval;  // BiCGSTAB: matrix values scaled by the Jacobi diagonal inverse of their column
     DevBuf<float> r32, z32, p32, q32, e32, dinv32;  // mixed-precision inner solve
     DevBuf<float> rt32, v32, t32, sval32;      // mixed BiCGSTAB (with r32, p32, e32)
+    DevBuf<float> wt;                                // scaled CG (cg_scaled.cuh): diagonal square roots,
+    DevBuf<int> scol, sym_bad;                       // its copy's columns, rows it cannot take
     DevBuf<double> gV, gZ, gW, ilu;                  // GMRES basis, preconditioned basis, ILU(0) factors
     DevBuf<long long> gpart;                         // exact multi-value partial sums
     DevBuf<GridBarrier> barrier;

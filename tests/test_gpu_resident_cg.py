@@ -57,6 +57,36 @@ def test_resident_cg(shape, method):
     assert it2 == it and res2 == res and np.array_equal(y, z)  # runs are bit-identical
 
 
+@pytest.mark.parametrize("shape", [(13, 17, 19), (80, 80, 101), (128, 100, 82)])
+@pytest.mark.parametrize("method", ["CG", "CG-mixed"])
+@pytest.mark.parametrize("kind", ["negative", "spread", "one_negative"])
+def test_cg_diagonals(shape, method, kind):
+    """Streaming solves run on the scaled system where the diagonal has one sign (a negative
+    definite matrix among them); with a single entry of the other sign (capped: it need not
+    converge) the form with M^-1 runs; row scales spread over 12 decades leave the answer."""
+    rp, c, v, x, b = seven_point(*shape, seed=5)
+    n = len(x)
+    rows = np.repeat(np.arange(n), np.diff(rp))
+    if kind == "spread":  # D A D with D over 6 decades: Jacobi removes it
+        d = 10.0 ** np.random.default_rng(2).uniform(-3, 3, n)
+        v, b, x = v * d[rows] * d[c], d * b, x / d
+    elif kind == "negative":
+        v, b = -v, -b
+    else:
+        v = v.copy()
+        at = rp[n // 2] + int(np.where(c[rp[n // 2]:rp[n // 2 + 1]] == n // 2)[0][0])
+        v[at] = -v[at]
+        _, it, res, status = csr_solve(rp, c, v, b, method=method, maxit=3, eps=EPS)
+        assert it == 3 and status == 1 and np.isfinite(res)
+        return
+    y, it, res, status = csr_solve(rp, c, v, b, method=method, maxit=1000, eps=EPS)
+    assert status == 0 and res < EPS
+    r = b - np.add.reduceat(v * y[c], rp[:-1])
+    assert np.linalg.norm(r) <= 2 * EPS * np.linalg.norm(b)
+    if kind == "negative":
+        assert np.linalg.norm(y - x) <= 100 * EPS * np.linalg.norm(x)
+
+
 def test_resident_cg_cap_breakdown_and_no_preconditioner():
     rp, c, v, x, b = seven_point(20, 19, 18, seed=3)
     _, it, res, status = csr_solve(rp, c, v, b, method="CG", maxit=5, eps=1e-14)
