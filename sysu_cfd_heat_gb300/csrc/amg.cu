@@ -108,7 +108,7 @@ __device__ __forceinline__ float row_part(const MgView &A, int i, const float *x
 #pragma unroll 4
     for (int k = s; k < wd; k += G) {
         const int pos = base + k * 32 + lane;
-        acc += A.val[pos] * x[A.col[pos]];
+        acc = fmaf(A.val[pos], x[A.col[pos]], acc);
     }
     return acc;
 }
@@ -126,10 +126,10 @@ __device__ __forceinline__ void group_loop(int n, F f) {
     }
 }
 
+// The steps of the cycle, over the whole grid.
 // t = r - A (w r)   (pre-smoothing from zero and its residual)
 template <int G>
-__global__ void k_mg_down(MgView A, const float *w, const float *r, float *t, const int *done) {
-    if (done && *done) return;
+__device__ __forceinline__ void down_rows(const MgView &A, const float *w, const float *r, float *t) {
     group_loop<G>(A.n, [&](bool valid, int i, int s) {
         float acc = 0.f;
         if (valid) {
@@ -147,6 +147,7 @@ __global__ void k_mg_down(MgView A, const float *w, const float *r, float *t, co
                     acc += v3 * y3;
                 }
             }
+#pragma unroll 2
             for (; k < wd; k += G) {
                 const int pos = base + k * 32 + lane;
                 const int j = A.col[pos];
@@ -161,9 +162,8 @@ __global__ void k_mg_down(MgView A, const float *w, const float *r, float *t, co
 // rc[I] = sum of t over the rows of aggregate I (members in ascending order,
 // lane s taking members s, s + G, ...)
 template <int G>
-__global__ void k_mg_restrict(int nc, const int *mem_ptr, const int *mem_idx, const float *t, float *rc,
-                              const int *done) {
-    if (done && *done) return;
+__device__ __forceinline__ void restrict_rows(int nc, const int *mem_ptr, const int *mem_idx, const float *t,
+                                              float *rc) {
     group_loop<G>(nc, [&](bool valid, int i, int s) {
         float acc = 0.f;
         if (valid) {
@@ -176,12 +176,16 @@ __global__ void k_mg_restrict(int nc, const int *mem_ptr, const int *mem_idx, co
     });
 }
 
+// the prolonged value w_i r_i + gamma zc[agg(i)], rounded the same way wherever it is formed
+__device__ __forceinline__ float prolonged(float w, float r, float gamma, float zc) {
+    return fmaf(w, r, __fmul_rn(gamma, zc));
+}
+
 // z_i = w_i r_i + gamma zc[agg(i)]; four rows a thread with 16-byte loads (the
 // level's arrays are whole allocations; r may be the caller's fine residual,
 // which is read four rows at a time only when 16-byte aligned)
-__global__ void k_mg_prolong(int n, const float *w, const float *r, const int *agg, const float *zc, float gamma,
-                             float *z, const int *done) {
-    if (done && *done) return;
+__device__ __forceinline__ void prolong_rows(int n, const float *w, const float *r, const int *agg, const float *zc,
+                                             float gamma, float *z) {
     const int T = gridDim.x * blockDim.x, t0 = blockIdx.x * blockDim.x + threadIdx.x;
     int n4 = 0;
     if ((reinterpret_cast<uintptr_t>(r) & 15) == 0 && (reinterpret_cast<uintptr_t>(z) & 15) == 0) {
@@ -190,25 +194,67 @@ __global__ void k_mg_prolong(int n, const float *w, const float *r, const int *a
             const float4 wj = reinterpret_cast<const float4 *>(w)[j], rj = reinterpret_cast<const float4 *>(r)[j];
             const int4 aj = reinterpret_cast<const int4 *>(agg)[j];
             float4 zj;
-            zj.x = wj.x * rj.x + gamma * zc[aj.x];
-            zj.y = wj.y * rj.y + gamma * zc[aj.y];
-            zj.z = wj.z * rj.z + gamma * zc[aj.z];
-            zj.w = wj.w * rj.w + gamma * zc[aj.w];
+            zj.x = prolonged(wj.x, rj.x, gamma, zc[aj.x]);
+            zj.y = prolonged(wj.y, rj.y, gamma, zc[aj.y]);
+            zj.z = prolonged(wj.z, rj.z, gamma, zc[aj.z]);
+            zj.w = prolonged(wj.w, rj.w, gamma, zc[aj.w]);
             reinterpret_cast<float4 *>(z)[j] = zj;
         }
     }
-    for (int i = 4 * n4 + t0; i < n; i += T) z[i] = w[i] * r[i] + gamma * zc[agg[i]];
+    for (int i = 4 * n4 + t0; i < n; i += T) z[i] = prolonged(w[i], r[i], gamma, zc[agg[i]]);
 }
 
 // zout = z + w (r - A z)
 template <int G>
-__global__ void k_mg_post(MgView A, const float *w, const float *r, const float *z, float *zout, const int *done) {
-    if (done && *done) return;
+__device__ __forceinline__ void post_rows(const MgView &A, const float *w, const float *r, const float *z,
+                                          float *zout) {
     group_loop<G>(A.n, [&](bool valid, int i, int s) {
         float acc = valid ? row_part<G>(A, i, z, s) : 0.f;
         acc = group_sum<G>(acc);
-        if (valid && s == 0) zout[i] = z[i] + w[i] * (r[i] - acc);
+        if (valid && s == 0) zout[i] = fmaf(w[i], r[i] - acc, z[i]);
     });
+}
+
+// the same for z = the prolonged coarse correction, formed where it is gathered
+template <int G>
+__device__ __forceinline__ void post_rows_prolong(const MgView &A, const float *w, const float *r, const int *agg,
+                                                  const float *zc, float gamma, float *zout) {
+    group_loop<G>(A.n, [&](bool valid, int i, int s) {
+        float acc = 0.f;
+        if (valid) {
+            const int base = A.sl_ptr[i >> 5], wd = A.sl_w[i >> 5], lane = i & 31;
+#pragma unroll 4
+            for (int k = s; k < wd; k += G) {
+                const int pos = base + k * 32 + lane, j = A.col[pos];
+                acc = fmaf(A.val[pos], prolonged(w[j], r[j], gamma, zc[agg[j]]), acc);
+            }
+        }
+        acc = group_sum<G>(acc);
+        if (valid && s == 0) zout[i] = fmaf(w[i], r[i] - acc, prolonged(w[i], r[i], gamma, zc[agg[i]]));
+    });
+}
+
+// one launch a step (the finest level, and a cycle whose coarse levels do not run as one launch)
+template <int G>
+__global__ void k_mg_down(MgView A, const float *w, const float *r, float *t, const int *done) {
+    if (done && *done) return;
+    down_rows<G>(A, w, r, t);
+}
+template <int G>
+__global__ void k_mg_restrict(int nc, const int *mem_ptr, const int *mem_idx, const float *t, float *rc,
+                              const int *done) {
+    if (done && *done) return;
+    restrict_rows<G>(nc, mem_ptr, mem_idx, t, rc);
+}
+__global__ void k_mg_prolong(int n, const float *w, const float *r, const int *agg, const float *zc, float gamma,
+                             float *z, const int *done) {
+    if (done && *done) return;
+    prolong_rows(n, w, r, agg, zc, gamma, z);
+}
+template <int G>
+__global__ void k_mg_post(MgView A, const float *w, const float *r, const float *z, float *zout, const int *done) {
+    if (done && *done) return;
+    post_rows<G>(A, w, r, z, zout);
 }
 
 // t = r - A z
@@ -243,7 +289,7 @@ __global__ void __launch_bounds__(DENSE_THREADS) k_mg_dense_apply(int nd, const 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     for (int i = warp; i < nd; i += nw) {
         float s = 0.f;
-        for (int j = lane; j < nd; j += 32) s += minv[(size_t)i * nd + j] * rs[j];
+        for (int j = lane; j < nd; j += 32) s = fmaf(minv[(size_t)i * nd + j], rs[j], s);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(FULL_MASK, s, o);
         if (lane == 0) z[i] = s;
@@ -338,24 +384,25 @@ __global__ void __launch_bounds__(DENSE_THREADS) k_mg_dense_inverse(int nd, cons
 MgView view_of(const SellDev &A, const float *val) { return MgView{A.n, A.sl_ptr.get(), A.sl_w.get(), A.col.get(), val}; }
 
 // ---- the coarse levels in one persistent cooperative launch ------------------
-// (option; measured slower than one launch per phase on the 2M-cell p' system:
-// 135 us per cycle against about 110 us, because every phase is a chain of
-// dependent L2 loads that a grid barrier does not shorten, and the finest
-// level's phases run at one 1024-thread block per SM)
-// Phases (each closed by a grid barrier): restriction of the finest level's t into
-// level 1; for l = 1 .. L-2: t_l = r_l - A_l (w_l r_l), restriction into l+1; the
-// coarsest solve; for l = L-2 .. 1: prolongation w_l r_l + gamma z_{l+1}[agg] into
-// t_l, post-smoothing into z_l; finally the finest prolongation
-// z0 = w0 r0 + gamma z_1[agg0].  Every row is computed by the same arithmetic in
-// the same order as the one-kernel-per-phase path, so both give the same bits.
-// Vectors written inside the launch are read with ld.global.cg (L2, not L1): t is
-// gathered again after other blocks rewrote it.
+// A V-cycle's coarse levels are a chain of 13 to 20 steps of one or two microseconds of work
+// each; as one launch a step they took 88 us of a 217 us iteration on the 2M-cell p' system
+// and 65 of 93 on the 256,000-row channel's.  Here a step ends with a grid barrier (1.2 us)
+// instead of a launch.  What made an earlier form of this kernel slower than the launches was
+// its steps: one thread walked a row's 14 entries one dependent L2 load after the other.  The
+// steps are those of the one-launch-per-phase kernels, a group of lanes a row, and give the
+// same bits; on levels below MG_FUSE_ROWS the prolongation is formed while the post-smoother
+// gathers it, a barrier fewer.
+// Phases: restriction of the finest level's t into level 1; for l = 1 .. L-2:
+// t_l = r_l - A_l (w_l r_l), restriction into l+1; the coarsest solve; for l = L-2 .. 1:
+// prolongation and post-smoothing into z_l; finally the finest prolongation
+// z0 = w0 r0 + gamma z_1[agg0].
 constexpr int MGP_THREADS = 1024;
+constexpr int MG_FUSE_ROWS = 65536;
 
 struct MgLvl {
-    int n;
-    const int *sl_ptr, *sl_w, *col;
-    const float *val, *w;
+    MgView A;
+    int grow, gagg;  // lanes per row / per aggregate
+    const float *w;
     float *r, *z, *t;
     const int *agg, *mem_ptr, *mem_idx;  // to the next level
 };
@@ -373,86 +420,70 @@ struct MgPersistArgs {
     const int *done;
 };
 
-__device__ __forceinline__ float lvl_row(const MgLvl &L, int i, const float *x) {
-    const int base = L.sl_ptr[i >> 5], wd = L.sl_w[i >> 5], lane = i & 31;
-    float s = 0.f;
-    for (int k = 0; k < wd; ++k) {
-        const int pos = base + k * 32 + lane;
-        s += L.val[pos] * __ldcg(x + L.col[pos]);
+template <class F>
+__device__ __forceinline__ void with_group_dev(int g, F f) {
+    switch (g) {
+        case 1: f(std::integral_constant<int, 1>{}); break;
+        case 2: f(std::integral_constant<int, 2>{}); break;
+        case 4: f(std::integral_constant<int, 4>{}); break;
+        case 8: f(std::integral_constant<int, 8>{}); break;
+        case 16: f(std::integral_constant<int, 16>{}); break;
+        default: f(std::integral_constant<int, 32>{}); break;
     }
-    return s;
-}
-
-__device__ __forceinline__ float lvl_row_wr(const MgLvl &L, int i) {
-    const int base = L.sl_ptr[i >> 5], wd = L.sl_w[i >> 5], lane = i & 31;
-    float s = 0.f;
-    for (int k = 0; k < wd; ++k) {
-        const int pos = base + k * 32 + lane;
-        const int j = L.col[pos];
-        s += L.val[pos] * (L.w[j] * __ldcg(L.r + j));
-    }
-    return s;
 }
 
 __global__ void __launch_bounds__(MGP_THREADS, 1) k_mg_coarse(MgPersistArgs a) {
     if (a.done && *a.done) return;  // written by earlier launches: every block sees the same value
-    const int T = gridDim.x * blockDim.x, t0 = blockIdx.x * blockDim.x + threadIdx.x;
     const int L = a.nlev;
-    // restriction of the finest level's t into level 1
-    {
-        const MgLvl &f = a.lv[0];
-        const MgLvl &c = a.lv[1];
-        for (int I = t0; I < c.n; I += T) {
-            float s = 0.f;
-            for (int k = f.mem_ptr[I]; k < f.mem_ptr[I + 1]; ++k) s += __ldcg(a.t0 + f.mem_idx[k]);
-            c.r[I] = s;
-        }
-    }
+    with_group_dev(a.lv[0].gagg, [&](auto G) {
+        restrict_rows<G.value>(a.lv[1].A.n, a.lv[0].mem_ptr, a.lv[0].mem_idx, a.t0, a.lv[1].r);
+    });
     if (!grid_sync(a.gb, a.err)) return;
     for (int l = 1; l < L - 1; ++l) {
         const MgLvl &f = a.lv[l];
-        for (int i = t0; i < f.n; i += T) f.t[i] = __ldcg(f.r + i) - lvl_row_wr(f, i);
+        with_group_dev(f.grow, [&](auto G) { down_rows<G.value>(f.A, f.w, f.r, f.t); });
         if (!grid_sync(a.gb, a.err)) return;
-        const MgLvl &c = a.lv[l + 1];
-        for (int I = t0; I < c.n; I += T) {
-            float s = 0.f;
-            for (int k = f.mem_ptr[I]; k < f.mem_ptr[I + 1]; ++k) s += __ldcg(f.t + f.mem_idx[k]);
-            c.r[I] = s;
-        }
+        with_group_dev(f.gagg, [&](auto G) {
+            restrict_rows<G.value>(a.lv[l + 1].A.n, f.mem_ptr, f.mem_idx, f.t, a.lv[l + 1].r);
+        });
         if (!grid_sync(a.gb, a.err)) return;
     }
+    const int T = gridDim.x * blockDim.x, t0 = blockIdx.x * blockDim.x + threadIdx.x;
     const MgLvl &c = a.lv[L - 1];
     if (a.nd > 0) {
         const int warp = t0 >> 5, lane = threadIdx.x & 31, nw = T >> 5;
         for (int i = warp; i < a.nd; i += nw) {
             float s = 0.f;
-            for (int j = lane; j < a.nd; j += 32) s += a.minv[(size_t)i * a.nd + j] * __ldcg(c.r + j);
+#pragma unroll 4
+            for (int j = lane; j < a.nd; j += 32) s = fmaf(a.minv[(size_t)i * a.nd + j], c.r[j], s);
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(FULL_MASK, s, o);
             if (lane == 0) c.z[i] = s;
         }
         if (!grid_sync(a.gb, a.err)) return;
     } else {  // three Jacobi steps from zero
-        for (int i = t0; i < c.n; i += T) c.z[i] = c.w[i] * __ldcg(c.r + i);
+        for (int i = t0; i < c.A.n; i += T) c.z[i] = c.w[i] * c.r[i];
         if (!grid_sync(a.gb, a.err)) return;
-        for (int i = t0; i < c.n; i += T) c.t[i] = __ldcg(c.z + i) + c.w[i] * (__ldcg(c.r + i) - lvl_row(c, i, c.z));
+        with_group_dev(c.grow, [&](auto G) { post_rows<G.value>(c.A, c.w, c.r, c.z, c.t); });
         if (!grid_sync(a.gb, a.err)) return;
-        for (int i = t0; i < c.n; i += T) c.z[i] = __ldcg(c.t + i) + c.w[i] * (__ldcg(c.r + i) - lvl_row(c, i, c.t));
+        with_group_dev(c.grow, [&](auto G) { post_rows<G.value>(c.A, c.w, c.r, c.t, c.z); });
         if (!grid_sync(a.gb, a.err)) return;
     }
     for (int l = L - 2; l >= 1; --l) {
         const MgLvl &f = a.lv[l];
-        const MgLvl &cc = a.lv[l + 1];
-        for (int i = t0; i < f.n; i += T) f.t[i] = f.w[i] * __ldcg(f.r + i) + a.gamma * __ldcg(cc.z + f.agg[i]);
-        if (!grid_sync(a.gb, a.err)) return;
-        for (int i = t0; i < f.n; i += T) f.z[i] = __ldcg(f.t + i) + f.w[i] * (__ldcg(f.r + i) - lvl_row(f, i, f.t));
+        const float *zc = a.lv[l + 1].z;
+        if (f.A.n <= MG_FUSE_ROWS) {
+            with_group_dev(f.grow, [&](auto G) {
+                post_rows_prolong<G.value>(f.A, f.w, f.r, f.agg, zc, a.gamma, f.z);
+            });
+        } else {
+            prolong_rows(f.A.n, f.w, f.r, f.agg, zc, a.gamma, f.t);
+            if (!grid_sync(a.gb, a.err)) return;
+            with_group_dev(f.grow, [&](auto G) { post_rows<G.value>(f.A, f.w, f.r, f.t, f.z); });
+        }
         if (!grid_sync(a.gb, a.err)) return;
     }
-    {
-        const MgLvl &f = a.lv[0];
-        const MgLvl &c1 = a.lv[1];
-        for (int i = t0; i < f.n; i += T) a.z0[i] = f.w[i] * a.r0[i] + a.gamma * __ldcg(c1.z + f.agg[i]);
-    }
+    prolong_rows(a.lv[0].A.n, a.lv[0].w, a.r0, a.lv[0].agg, a.lv[1].z, a.gamma, a.z0);
 }
 
 }  // namespace
@@ -604,7 +635,7 @@ void AggMultigrid::enqueue_cycle_to_fine(const float *r, float *z, const int *do
         ++g_launches;
         return;
     }
-    if (persistent && !(post_hook && post_level >= 1)) {
+    if (one_launch && !(post_hook && post_level >= 1)) {
         MgLevelDev &d0 = *lv_[0];
         with_group(d0.grow, [&](auto G) {
             k_mg_down<G.value><<<flat_blocks((long)f.n * G.value), MB, 0, st>>>(view_of(*A0_, val0_32_), d0.w.get(),
@@ -616,9 +647,8 @@ void AggMultigrid::enqueue_cycle_to_fine(const float *r, float *z, const int *do
         for (int l = 0; l < L; ++l) {
             MgLevelDev &d = *lv_[l];
             const SellDev &A = l == 0 ? *A0_ : d.A;
-            pa.lv[l] = MgLvl{d.n, A.sl_ptr.get(), A.sl_w.get(), A.col.get(), l == 0 ? val0_32_ : d.val32.get(),
-                             d.w.get(), d.r.get(), d.z.get(), d.t.get(), d.agg.get(), d.mem_ptr.get(),
-                             d.mem_idx.get()};
+            pa.lv[l] = MgLvl{view_of(A, l == 0 ? val0_32_ : d.val32.get()), d.grow, d.gagg, d.w.get(), d.r.get(),
+                             d.z.get(), d.t.get(), d.agg.get(), d.mem_ptr.get(), d.mem_idx.get()};
         }
         pa.r0 = r;
         pa.t0 = d0.t.get();

@@ -246,18 +246,20 @@ __global__ void __launch_bounds__(MB) k_m3_replace(M3Args a, int first) {
         a.r[i] = r;
         if (any_rs) a.rtd[i] = rt;
     }
-    double v[6];
-    if (!grid_sums_f<6>(f, v, a.part, &a.st->cnt)) return;
+    if (!grid_totals_f<6>(f, a.part, &a.st->cnt) || threadIdx.x >= 3) return;
     M3State *W = a.st;
-    int all_done = 1;
-    for (int c = 0; c < 3; ++c) {
-        if (want[c]) {
-            const double rr = v[c] / (sg[c] * sg[c]);  // ||b - A x||^2
+    const double *v = g_gt_sum;
+    {
+        const int c = threadIdx.x;  // a thread a component
+        if (W->need[c] && !W->done[c]) {
+            const bool rsc = W->restart[c] != 0;
+            const double sgc = W->sig_next[c];
+            const double rr = v[c] / (sgc * sgc);  // ||b - A x||^2
             if (!first) W->upd[c] += 1;
             W->rr64[c] = rr;
             W->sig[c] = W->sig_next[c];
             W->rref[c] = v[c];
-            if (rs[c]) {
+            if (rsc) {
                 W->rho[c] = v[c];
             } else {
                 // the recurrences go on with the replaced residual: rho on it; the
@@ -281,10 +283,12 @@ __global__ void __launch_bounds__(MB) k_m3_replace(M3Args a, int first) {
             W->need[c] = 0;
             W->skip[c] = 0;
         }
-        all_done &= W->done[c];
+        const int all_done = __all_sync(7u, W->done[c] != 0);
+        if (c == 0) {
+            W->any_need = 0;
+            W->all_done = all_done;
+        }
     }
-    W->any_need = 0;
-    W->all_done = all_done;
 }
 
 // p = r (restart) or r + beta (p - omega v)
@@ -323,11 +327,11 @@ __global__ void __launch_bounds__(MB, 8) k_m3_av(M3Args a) {
         f[1] = fmaf(rt.y, y.y, f[1]);
         f[2] = fmaf(rt.z, y.z, f[2]);
     }
-    double v[3];
-    if (!grid_sums_f<3>(f, v, a.part, &a.st->cnt)) return;
+    if (!grid_totals_f<3>(f, a.part, &a.st->cnt) || threadIdx.x >= 3) return;
     M3State *S = a.st;
-    for (int c = 0; c < 3; ++c) {
-        if (S->done[c]) continue;
+    const double *v = g_gt_sum;
+    const int c = threadIdx.x;  // a thread a component
+    if (!S->done[c]) {
         if (v[c] == 0.0 || !isfinite(v[c])) {  // breakdown: replace and restart
             S->skip[c] = 1;
             S->need[c] = 1;
@@ -366,11 +370,11 @@ __global__ void __launch_bounds__(MB) k_m3_s(M3Args a) {
         }
         a.s[i] = s;
     }
-    double v[3];
-    if (!grid_sums_f<3>(f, v, a.part, &a.st->cnt)) return;
+    if (!grid_totals_f<3>(f, a.part, &a.st->cnt) || threadIdx.x >= 3) return;
     M3State *W = a.st;
-    for (int c = 0; c < 3; ++c) {
-        if (!on[c]) continue;
+    const double *v = g_gt_sum;
+    const int c = threadIdx.x;  // a thread a component
+    if (!W->done[c] && !W->skip[c]) {
         const double sc2 = W->sig[c] * W->sig[c];
         W->early[c] = v[c] <= W->d2 * W->rref[c] || v[c] < W->thr[c] * sc2;
         if (W->early[c]) W->sig_next[c] = pow2_scale(v[c] / sc2);
@@ -392,11 +396,11 @@ __global__ void __launch_bounds__(MB, 6) k_m3_at(M3Args a) {
         f[4] = fmaf(y.y, y.y, f[4]);
         f[5] = fmaf(y.z, y.z, f[5]);
     }
-    double v[6];
-    if (!grid_sums_f<6>(f, v, a.part, &a.st->cnt)) return;
+    if (!grid_totals_f<6>(f, a.part, &a.st->cnt) || threadIdx.x >= 3) return;
     M3State *S = a.st;
-    for (int c = 0; c < 3; ++c)
-        if (!S->done[c] && !S->skip[c] && !S->early[c]) S->omg[c] = v[3 + c] != 0.0 ? v[c] / v[3 + c] : 0.0;
+    const double *v = g_gt_sum;
+    const int c = threadIdx.x;  // a thread a component
+    if (!S->done[c] && !S->skip[c] && !S->early[c]) S->omg[c] = v[3 + c] != 0.0 ? v[c] / v[3 + c] : 0.0;
 }
 
 // e += d (alpha p + omega s) ; r = s - omega t ; r.r, rt.r -> rho, beta, and
@@ -435,24 +439,25 @@ __global__ void __launch_bounds__(MB, 6) k_m3_upd(M3Args a) {
         a.e[i] = e;
         a.r[i] = r;
     }
-    double v[6];
-    if (!grid_sums_f<6>(f, v, a.part, &a.st->cnt)) return;
+    if (!grid_totals_f<6>(f, a.part, &a.st->cnt) || threadIdx.x >= 3) return;
     M3State *W = a.st;
-    int need = W->any_need;
-    for (int c = 0; c < 3; ++c) {
-        if (!on[c]) continue;
+    const double *v = g_gt_sum;
+    const int c = threadIdx.x;  // a thread a component
+    const bool run = !W->done[c] && !W->skip[c], early = W->early[c] != 0;
+    const double rr = v[c], sc2 = W->sig[c] * W->sig[c];
+    if (run) {
         W->it[c] += 1;
-        if (ea[c]) {
+        if (early) {
             W->need[c] = 1;
             W->restart[c] = 1;
             W->early[c] = 0;
         } else {
-            const double rr = v[c], sc2 = W->sig[c] * W->sig[c];
-            W->rho_prev[c] = W->rho[c];
-            W->rho[c] = v[3 + c];
+            const double rho = v[3 + c], before = W->rho[c], omg = W->omg[c];
+            W->rho_prev[c] = before;
+            W->rho[c] = rho;
             W->restart[c] = 0;
-            const bool brk = W->omg[c] == 0.0 || W->rho[c] == 0.0 || W->rho_prev[c] == 0.0 || !isfinite(rr);
-            W->beta[c] = brk ? 0.0 : (W->rho[c] / W->rho_prev[c]) * (W->alpha[c] / W->omg[c]);
+            const bool brk = omg == 0.0 || rho == 0.0 || before == 0.0 || !isfinite(rr);
+            W->beta[c] = brk ? 0.0 : (rho / before) * (W->alpha[c] / omg);
             if (brk) {
                 W->need[c] = 1;
                 W->restart[c] = 1;
@@ -461,22 +466,17 @@ __global__ void __launch_bounds__(MB, 6) k_m3_upd(M3Args a) {
             }
             if (W->need[c]) W->sig_next[c] = isfinite(rr) && rr > 0.0 ? pow2_scale(rr / sc2) : W->sig[c];
         }
-        need |= W->need[c];
     }
+    const bool any = __any_sync(7u, W->any_need || (run && W->need[c]));
     // a replacement costs about as much for one component as for three (the
     // matrix pass is shared): a running component whose FP32 residual has fallen
     // by sqrt(inner_tol) since its last replacement is replaced along with the due
     // ones, which saves the pass it would take an iteration or two later
-    if (need)
-        for (int c = 0; c < 3; ++c) {
-            if (!on[c] || ea[c] || W->need[c]) continue;
-            const double rr = v[c], sc2 = W->sig[c] * W->sig[c];
-            if (isfinite(rr) && rr > 0.0 && rr * rr <= W->d2 * W->rref[c] * W->rref[c]) {
-                W->need[c] = 1;
-                W->sig_next[c] = pow2_scale(rr / sc2);
-            }
-        }
-    W->any_need = need;
+    if (any && run && !early && !W->need[c] && isfinite(rr) && rr > 0.0 && rr * rr <= W->d2 * W->rref[c] * W->rref[c]) {
+        W->need[c] = 1;
+        W->sig_next[c] = pow2_scale(rr / sc2);
+    }
+    if (c == 0) W->any_need = any;
 }
 
 // x += e / sig in FP64 and e = 0 for the components about to be replaced (the

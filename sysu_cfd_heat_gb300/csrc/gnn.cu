@@ -268,8 +268,7 @@ __global__ void __launch_bounds__(GT) k_gnn_fwd(NetArgs a) {
     }
     if (DEC && a.fs) {
         const float fv[1] = {zq};
-        double v[1];
-        if (grid_sums_f<1>(fv, v, a.part, &a.fs->cnt[0])) a.fs->zq = v[0];
+        if (grid_totals_f<1>(fv, a.part, &a.fs->cnt[0]) && threadIdx.x == 0) a.fs->zq = g_gt_sum[0];
     }
     umma::fence_before_sync();
     __syncthreads();
@@ -807,8 +806,7 @@ __global__ void k_fcg_jacobi(FcgArgs a) {
         if (!rs) f0 += zi * a.q[i];
     }
     const float fv[1] = {f0};
-    double v[1];
-    if (grid_sums_f<1>(fv, v, a.part, &a.fs->cnt[0])) a.fs->zq = v[0];
+    if (grid_totals_f<1>(fv, a.part, &a.fs->cnt[0]) && threadIdx.x == 0) a.fs->zq = g_gt_sum[0];
 }
 
 // multigrid form, finest level after the coarse correction z2: t = r - A z2, then
@@ -831,8 +829,8 @@ __global__ void k_fcg_mgfine(FcgArgs a, const float *z2, float *t, const float *
         }
     }
     const float fv[1] = {f0};
-    double v[1];
-    if (grid_sums_f<1>(fv, v, a.part, &a.fs->cnt[0])) {
+    if (grid_totals_f<1>(fv, a.part, &a.fs->cnt[0]) && threadIdx.x == 0) {
+        const double *v = g_gt_sum;
         if (net) {
             double s = sqrt(v[0] / (double)a.g.n);
             a.fs->s2 = (float)s;
@@ -866,8 +864,8 @@ __global__ void k_lvl_resid(GView g, const float *r, const float *zp, float *t, 
     }
     if (!net) return;
     const float fv[1] = {f0};
-    double v[1];
-    if (grid_sums_f<1>(fv, v, part, &fs->cnt[3])) {
+    if (grid_totals_f<1>(fv, part, &fs->cnt[3]) && threadIdx.x == 0) {
+        const double *v = g_gt_sum;
         double s = sqrt(v[0] / (double)g.n);
         fs->s2 = (float)s;
         fs->inv_s2 = s > 0.0 ? (float)(1.0 / s) : 0.f;
@@ -911,8 +909,8 @@ __global__ void k_fcg_dir(FcgArgs a) {
         f1 += pi * a.r[i];
     }
     const float fv[2] = {f0, f1};
-    double v[2];
-    if (grid_sums_f<2>(fv, v, a.part, &a.fs->cnt[1])) {
+    if (grid_totals_f<2>(fv, a.part, &a.fs->cnt[1]) && threadIdx.x == 0) {
+        const double *v = g_gt_sum;
         FcgState *f = a.fs;
         double pq = v[0], pr = v[1];
         double alpha = pr / pq;
@@ -976,14 +974,16 @@ __global__ void k_fcg_upd(FcgArgs a) {
         }
     }
     const float fv[2] = {f0, f1};
-    double v[2];
-    if (grid_sums_f<2>(fv, v, a.part, &a.fs->cnt[2])) {
+    if (grid_totals_f<2>(fv, a.part, &a.fs->cnt[2]) && threadIdx.x == 0) {
+        const double *v = g_gt_sum;
         FcgState *f = a.fs;
         f->iters += 1;
         f->rr = v[0];
-        double s = sqrt(v[1] / (double)a.g.n);
-        f->s = (float)s;
-        f->inv_s = s > 0.0 ? (float)(1.0 / s) : 0.f;
+        if (f->use_gnn) {  // the network's input scale (an FP64 root and a division: 1.8 us of the tail)
+            double s = sqrt(v[1] / (double)a.g.n);
+            f->s = (float)s;
+            f->inv_s = s > 0.0 ? (float)(1.0 / s) : 0.f;
+        }
         f->pq_prev = f->pq;
         if (v[0] < f->rr_best) {
             f->rr_best = v[0];
@@ -1470,7 +1470,7 @@ struct FcgKey {
     const double *b_in;
     double *x_out;
     SolveInfo *info;
-    int x0_zero, maxit, use_gnn, chunk, gflat, net_level, post_level, hook, mg_persistent;
+    int x0_zero, maxit, use_gnn, chunk, gflat, net_level, post_level, hook, mg_one_launch;
     double eps, mg_gamma;
     float skip;
     const void *mg;
@@ -1516,7 +1516,7 @@ void GnnPrecond::fcg(const double *b, double *x, bool x0_zero, const KrylovOpts 
         k.net_level = net_level;
         k.post_level = mg_->post_level;
         k.hook = mg_->post_hook ? 1 : 0;
-        k.mg_persistent = mg_->persistent ? 1 : 0;
+        k.mg_one_launch = mg_->one_launch ? 1 : 0;
         k.mg_gamma = mg_->gamma;
     }
     // b, x0 in; the iterations; x and the statistics out

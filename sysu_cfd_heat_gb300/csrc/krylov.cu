@@ -433,41 +433,6 @@ struct BicgState {
 };
 __shared__ double g_bicg_smem[9 * (KB / 32)], g_bicg_sum[9];
 
-// One step of the warp's butterfly over NV values with the values dealt out: a lane keeps
-// the half of the values that its side of the step owns and adds its partner's, so NV values
-// cost about NV additions instead of 5 NV.  The additions are those of the butterfly of each
-// value (xor 16, 8, 4, 2, 1): the same bits.  Returns how many values a lane still holds.
-template <int NV>
-__device__ __forceinline__ double deal_sum(const double (&v)[NV], int o) {
-    const int lane = threadIdx.x & 31;
-    if constexpr (NV == 1) {
-        double s = v[0];
-        for (; o > 0; o >>= 1) s += __shfl_xor_sync(FULL_MASK, s, o);
-        return s;
-    } else {
-        constexpr int H = (NV + 1) / 2;  // the lower side keeps values 0..H-1, the upper H..NV-1
-        const bool up = (lane & o) != 0;
-        double k[H];
-#pragma unroll
-        for (int j = 0; j < H; ++j) {
-            const double lo = v[j], hi = H + j < NV ? v[H + j] : 0.0;
-            const double other = __shfl_xor_sync(FULL_MASK, up ? lo : hi, o);
-            k[j] = (up ? hi : lo) + other;
-        }
-        return deal_sum<H>(k, o >> 1);
-    }
-}
-// lane that holds value k's sum after deal_sum<NV>
-template <int NV>
-__device__ __forceinline__ int deal_lane(int k, int o = 16) {
-    if constexpr (NV == 1) {
-        return 0;
-    } else {
-        constexpr int H = (NV + 1) / 2;
-        return k < H ? deal_lane<H>(k, o >> 1) : o + deal_lane<H>(k - H, o >> 1);
-    }
-}
-
 // Grid sums of NV values, to g_bicg_sum for the whole block, in the order of block_sum_t0
 // (warp butterfly, warps) and warp_sum_partials; value k by thread k, then by a warp.
 template <int NV>

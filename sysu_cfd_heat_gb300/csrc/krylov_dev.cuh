@@ -287,33 +287,103 @@ __device__ bool grid_sums(double (&v)[NV], double *part, unsigned *cnt) {
     return grid_sums_publish<NV>(v, part, cnt, sm);
 }
 
-// Grid sums of FP32 per-thread partials.  The warp sums stay in FP32 (a fixed
-// butterfly, so lane 0's total is the same on every run); only the warp
-// totals go to FP64 for the block and grid sums.  An FP64 shuffle tree in
-// every thread runs on GB300's FP64 pipe (1/64 of the FP32 rate): 6 FP64
-// operations per value and thread took 10-20 us of a 2M-row vector pass.
+// One step of the warp's butterfly over NV values with the values dealt out: a lane keeps
+// the half of the values that its side of the step owns and adds its partner's, so NV values
+// cost about NV additions instead of 5 NV.  The additions are those of the butterfly of each
+// value (xor 16, 8, 4, 2, 1): the same bits.  Returns how many values a lane still holds.
 template <int NV>
-__device__ bool grid_sums_f(const float (&f)[NV], double (&v)[NV], double *part, unsigned *cnt) {
-    __shared__ double sm[NV * 8];
-    float g[NV];
+__device__ __forceinline__ double deal_sum(const double (&v)[NV], int o) {
+    const int lane = threadIdx.x & 31;
+    if constexpr (NV == 1) {
+        double s = v[0];
+        for (; o > 0; o >>= 1) s += __shfl_xor_sync(FULL_MASK, s, o);
+        return s;
+    } else {
+        constexpr int H = (NV + 1) / 2;  // the lower side keeps values 0..H-1, the upper H..NV-1
+        const bool up = (lane & o) != 0;
+        double k[H];
+#pragma unroll
+        for (int j = 0; j < H; ++j) {
+            const double lo = v[j], hi = H + j < NV ? v[H + j] : 0.0;
+            const double other = __shfl_xor_sync(FULL_MASK, up ? lo : hi, o);
+            k[j] = (up ? hi : lo) + other;
+        }
+        return deal_sum<H>(k, o >> 1);
+    }
+}
+// lane that holds value k's sum after deal_sum<NV>
+template <int NV>
+__device__ __forceinline__ int deal_lane(int k, int o = 16) {
+    if constexpr (NV == 1) {
+        return 0;
+    } else {
+        constexpr int H = (NV + 1) / 2;
+        return k < H ? deal_lane<H>(k, o >> 1) : o + deal_lane<H>(k - H, o >> 1);
+    }
+}
+
+// Grid sums of FP32 per-thread partials, for blocks of up to 256 threads: true in every thread of
+// the last block to arrive, which finds the sums in g_gt_sum.  The warp sums stay in FP32 (a
+// fixed butterfly, so the total is the same on every run); only the warp totals go to FP64 for
+// the block and grid sums.  An FP64 shuffle tree in every thread runs on GB300's FP64 pipe
+// (1/64 of the FP32 rate): 6 FP64 operations per value and thread took 10-20 us of a 2M-row
+// vector pass.  What is left is the tail after the last block's arrival, a chain of FP64
+// additions of 65 clocks each: values side by side in groups of 8 lanes or dealt over the
+// lanes, not one after the other in one thread, and callers work their scalars out with a
+// thread a component.  On 262,144 rows the tail of six sums and three components' scalars
+// (k_m3_upd) went from 14 to 5 us.
+__shared__ double g_gt_warp[NVMAX * 8], g_gt_sum[NVMAX];
+
+// g_gt_warp[k * 8 + w], w < 8, summed over w by 8 lanes a value: to every lane of the group
+__device__ __forceinline__ double sum8(double v) {
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(FULL_MASK, v, o);
+    return v;
+}
+
+template <int NV>
+__device__ bool grid_totals_f(const float (&f)[NV], double *part, unsigned *cnt) {
+    static_assert(NV <= NVMAX && NV * 8 <= 64, "grid_totals_f: too many values");
+    __shared__ float sm[NV * 8];
+    __shared__ int s_last;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5, G = gridDim.x;
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
-        g[k] = f[k];
-        for (int o = 16; o > 0; o >>= 1) g[k] += __shfl_xor_sync(FULL_MASK, g[k], o);
+        float g = f[k];
+        for (int o = 16; o > 0; o >>= 1) g += __shfl_xor_sync(FULL_MASK, g, o);
+        if (lane == 0) sm[k * 8 + warp] = g;
     }
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    if (lane == 0)
-#pragma unroll
-        for (int k = 0; k < NV; ++k) sm[k * nw + warp] = (double)g[k];
     __syncthreads();
-    if (threadIdx.x == 0)
+    if (warp < (NV * 8 + 31) / 32) {
+        const double s = sum8(tid < NV * 8 && (tid & 7) < nw ? (double)sm[tid] : 0.0);
+        if (tid < NV * 8 && (tid & 7) == 0) part[(size_t)(tid >> 3) * G + blockIdx.x] = s;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        __threadfence();
+        s_last = atomicAdd(cnt, 1u) == (unsigned)G - 1u;
+    }
+    __syncthreads();
+    if (!s_last) return false;
+    __threadfence();
+    double t[NV];
 #pragma unroll
-        for (int k = 0; k < NV; ++k) {
-            double s = 0.0;
-            for (int w = 0; w < nw; ++w) s += sm[k * nw + w];
-            v[k] = s;
-        }
-    return grid_sums_publish<NV>(v, part, cnt, sm);
+    for (int k = 0; k < NV; ++k) t[k] = 0.0;
+    for (int b = tid; b < G; b += blockDim.x)
+#pragma unroll
+        for (int k = 0; k < NV; ++k) t[k] += __ldcg(part + (size_t)k * G + b);
+    const double w = deal_sum<NV>(t, 16);
+#pragma unroll
+    for (int k = 0; k < NV; ++k)
+        if (lane == deal_lane<NV>(k)) g_gt_warp[k * 8 + warp] = w;
+    __syncthreads();
+    if (warp < (NV * 8 + 31) / 32) {
+        const double s = sum8(tid < NV * 8 && (tid & 7) < nw ? g_gt_warp[tid] : 0.0);
+        if (tid < NV * 8 && (tid & 7) == 0) g_gt_sum[tid >> 3] = s;
+    }
+    if (tid == 0) *cnt = 0;
+    __syncthreads();
+    return true;
 }
 
 int g_num_sms = 0;

@@ -58,7 +58,7 @@ struct EqOpts {
     double mg_theta = 0.25;
     double mg_omega = 0.8;
     double mg_gamma = 1.8;
-    int mg_persistent = 0;    // 1: the coarse levels as one persistent cooperative launch
+    int mg_persistent = 0;    // 1: the coarse levels as one cooperative launch in shared graphs too
     // learned form with precond PK_AMG: the multigrid level whose post-smoother
     // the network is (0 the finest; deeper than the last coarse level clamps)
     int learn_level = 2;
