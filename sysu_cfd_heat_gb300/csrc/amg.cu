@@ -387,11 +387,13 @@ MgView view_of(const SellDev &A, const float *val) { return MgView{A.n, A.sl_ptr
 // A V-cycle's coarse levels are a chain of 13 to 20 steps of one or two microseconds of work
 // each; as one launch a step they took 88 us of a 217 us iteration on the 2M-cell p' system
 // and 65 of 93 on the 256,000-row channel's.  Here a step ends with a grid barrier (1.2 us)
-// instead of a launch.  What made an earlier form of this kernel slower than the launches was
+// instead of a launch: 55 us a cycle on the channel, 86 on the 2M cells (their levels hold more
+// work, so the launches cost less there).  What made an earlier form of this kernel slower than the launches was
 // its steps: one thread walked a row's 14 entries one dependent L2 load after the other.  The
 // steps are those of the one-launch-per-phase kernels, a group of lanes a row, and give the
 // same bits; on levels below MG_FUSE_ROWS the prolongation is formed while the post-smoother
-// gathers it, a barrier fewer.
+// gathers it, a barrier fewer.  Giving a CTA the members of its own aggregates, so that half of
+// the barriers fall away, is slower (63 and 89 us): the members are scattered over the matrix.
 // Phases: restriction of the finest level's t into level 1; for l = 1 .. L-2:
 // t_l = r_l - A_l (w_l r_l), restriction into l+1; the coarsest solve; for l = L-2 .. 1:
 // prolongation and post-smoothing into z_l; finally the finest prolongation

@@ -56,7 +56,7 @@ __device__ __forceinline__ uint32_t bf_pack(float a, float b) {
 __device__ __forceinline__ float bf_round(float a) { return __bfloat162float(__float2bfloat16_rn(a)); }
 
 // The flexible-CG kernels accumulate each thread's rows (a handful) in FP32 and
-// hand those partials to grid_sums_f (FP32 warp sums, FP64 block and grid
+// hand those partials to grid_totals_f (FP32 warp sums, FP64 block and grid
 // sums): per-row FP64 arithmetic and conversions run on GB300's FP64 pipe (1/64
 // of the FP32 rate) and took half of these kernels' time.  Convergence is
 // decided on the FP64 residual b - A x.
@@ -610,11 +610,6 @@ __global__ void k_gnn_loss(GView g, float sgn, int kind, const float *z, const f
     }
 }
 
-__global__ void k_gnn_store_loss(const GnnScalars *sc, double *out) {
-    double d = sc->loss_den;
-    *out = d > 0.0 ? sc->loss_num / d : 0.0;
-}
-
 __global__ void k_gnn_scale(GView g, const float *r, double *part, GnnScalars *sc) {
     double v[1] = {0.0};
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < g.n; i += gridDim.x * blockDim.x) {
@@ -628,13 +623,40 @@ __global__ void k_gnn_scale(GView g, const float *r, double *part, GnnScalars *s
     }
 }
 
-// Sum the per-CTA gradient records; update (Adam) or just report.
-__global__ void k_gnn_adam(const float *rec, int nrec, float *p, float *m, float *v, uint16_t *wbf, float *grad_out,
-                           double lr, int t, int update) {
-    int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= GNN_NPARAM) return;
+// Sum the per-CTA gradient records; update (Adam) or just report.  What bounds it is the FP64
+// pipe (a conversion and an addition a record and parameter, 64 clocks a warp each): a warp's
+// 32 parameters are split over the block's eight warps, each summing every eighth record, so
+// that all the SMs' pipes work and eight loads are in flight.  One thread a parameter, record
+// after record, took 87 us for 456 records; this takes 22.  corr1, corr2: 1 - beta^t.  The
+// first thread also files the loss of the step.
+constexpr int ADAM_P = 32, ADAM_W = 8;
+
+__global__ void __launch_bounds__(ADAM_P * ADAM_W)
+    k_gnn_adam(const float *rec, int nrec, float *p, float *m, float *v, uint16_t *wbf, float *grad_out, double lr,
+               double corr1, double corr2, int update, const GnnScalars *sc, double *loss_out) {
+    __shared__ double part[ADAM_W][ADAM_P];
+    const int c = threadIdx.x & (ADAM_P - 1), w = threadIdx.x / ADAM_P;
+    const int q = blockIdx.x * ADAM_P + c;
     double g = 0.0;
-    for (int b = 0; b < nrec; ++b) g += rec[(size_t)b * GNN_NPARAM_PAD + q];
+    if (q < GNN_NPARAM) {
+        const float *rq = rec + q;
+        int b = w;
+        for (; b + 7 * ADAM_W < nrec; b += 8 * ADAM_W) {
+            float x[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) x[i] = rq[(size_t)(b + i * ADAM_W) * GNN_NPARAM_PAD];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) g += x[i];
+        }
+        for (; b < nrec; b += ADAM_W) g += rq[(size_t)b * GNN_NPARAM_PAD];
+    }
+    part[w][c] = g;
+    __syncthreads();
+    if (w != 0) return;
+    if (q == 0) *loss_out = sc->loss_den > 0.0 ? sc->loss_num / sc->loss_den : 0.0;
+    if (q >= GNN_NPARAM) return;
+#pragma unroll
+    for (int i = 1; i < ADAM_W; ++i) g += part[i][c];
     if (grad_out) grad_out[q] = (float)g;
     if (!update) return;
     const double b1 = 0.9, b2 = 0.999, eps = 1e-8;
@@ -642,7 +664,7 @@ __global__ void k_gnn_adam(const float *rec, int nrec, float *p, float *m, float
     double vq = b2 * v[q] + (1.0 - b2) * g * g;
     m[q] = (float)mq;
     v[q] = (float)vq;
-    double mh = mq / (1.0 - pow(b1, (double)t)), vh = vq / (1.0 - pow(b2, (double)t));
+    double mh = mq / corr1, vh = vq / corr2;
     float pn = (float)(p[q] - lr * mh / (sqrt(vh) + eps));
     p[q] = pn;
     int rel = q - GNN_OFF_LAYER;
@@ -1402,10 +1424,10 @@ void GnnPrecond::train_step(int k, double lr, cudaStream_t st) {
     ++g_launches;
     backward(r, st);
     ++adam_t_;
-    k_gnn_adam<<<(GNN_NPARAM + FB - 1) / FB, FB, 0, st>>>(rec_.get(), gtiles_, p_.get(), m_.get(), v_.get(),
-                                                          wbf_.get(), nullptr, lr, adam_t_, 1);
-    k_gnn_store_loss<<<1, 1, 0, st>>>(sc_.get(), losses_.get() + ((adam_t_ - 1) & ((1 << 16) - 1)));
-    g_launches += 2;
+    k_gnn_adam<<<(GNN_NPARAM + ADAM_P - 1) / ADAM_P, ADAM_P * ADAM_W, 0, st>>>(
+        rec_.get(), gtiles_, p_.get(), m_.get(), v_.get(), wbf_.get(), nullptr, lr, 1.0 - std::pow(0.9, adam_t_),
+        1.0 - std::pow(0.999, adam_t_), 1, sc_.get(), losses_.get() + ((adam_t_ - 1) & ((1 << 16) - 1)));
+    ++g_launches;
     SYSU_CUDA(cudaGetLastError());
 }
 
@@ -1420,10 +1442,10 @@ void GnnPrecond::loss_grad(int k, double *loss, float *grad_host, cudaStream_t s
     ++g_launches;
     backward(r, st);
     DevBuf<float> g(GNN_NPARAM);
-    k_gnn_adam<<<(GNN_NPARAM + FB - 1) / FB, FB, 0, st>>>(rec_.get(), gtiles_, p_.get(), m_.get(), v_.get(),
-                                                          wbf_.get(), g.get(), 0.0, 1, 0);
-    k_gnn_store_loss<<<1, 1, 0, st>>>(sc_.get(), losses_.get());
-    g_launches += 2;
+    k_gnn_adam<<<(GNN_NPARAM + ADAM_P - 1) / ADAM_P, ADAM_P * ADAM_W, 0, st>>>(
+        rec_.get(), gtiles_, p_.get(), m_.get(), v_.get(), wbf_.get(), g.get(), 0.0, 1.0, 1.0, 0, sc_.get(),
+        losses_.get());
+    ++g_launches;
     SYSU_CUDA(cudaGetLastError());
     g.download(grad_host, GNN_NPARAM, st);
     SYSU_CUDA(cudaMemcpyAsync(loss, losses_.get(), sizeof(double), cudaMemcpyDeviceToHost, st));
