@@ -12,7 +12,7 @@
 // Reductions (scale, loss, the flexible-CG scalars) are per-block partial
 // sums that the last block to finish adds up in block order, so results are
 // run-to-run deterministic; so are the parameter gradients (per-CTA records,
-// summed in CTA order by the Adam kernel).
+// summed in a fixed order by the Adam kernel).
 #include <cuda_bf16.h>
 
 #include <cmath>
@@ -31,10 +31,14 @@ constexpr int GT = 128;  // rows per tile = threads per CTA of the network kerne
 constexpr int FB = 256;  // threads per block of the flat kernels
 constexpr uint32_t IDESC_F = umma::idesc_bf16_f32(128, 32);   // forward: 128 x 32, K = 64
 constexpr uint32_t IDESC_B1 = umma::idesc_bf16_f32(128, 64);  // backward, input gradient: 128 x 64, K = 32
-constexpr uint32_t IDESC_B2 = umma::idesc_bf16_f32(128, 32);  // backward, weight gradient: 128 x 32, K = 128
+// backward, weight gradient: 128 x 32, K = 128, both operands MN-major
+constexpr uint32_t IDESC_B2 = umma::idesc_bf16_f32(128, 32) | umma::IDESC_A_MN | umma::IDESC_B_MN;
 
 constexpr int FWD_SMEM = 16384 + 4096 + 1024;
-constexpr int BWD_SMEM = 8192 + 4096 + 32768 + 8192 + 2048 + 1024;
+// backward: X tile, weights, transposition tiles, dpre tile (the 32 bytes between its groups
+// spread a row's four groups over the banks), parameters and sums
+constexpr int BWD_X = 32768, BWD_W = 4096, BWD_T = 16384, BWD_DG = 2048 + 32, BWD_D = 4 * BWD_DG;
+constexpr int BWD_SMEM = BWD_X + BWD_W + BWD_T + BWD_D + (96 + 256) * 4 + 16;
 // The backward kernel holds 128 TMEM columns; requesting this much shared
 // memory caps it at three resident CTAs per SM (384 of 512 columns).
 constexpr int BWD_SMEM_REQ = 64 * 1024;
@@ -53,7 +57,6 @@ __device__ __forceinline__ uint32_t bf_pack(float a, float b) {
     return (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(a)) |
            ((uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(b)) << 16);
 }
-__device__ __forceinline__ float bf_round(float a) { return __bfloat162float(__float2bfloat16_rn(a)); }
 
 // The flexible-CG kernels accumulate each thread's rows (a handful) in FP32 and
 // hand those partials to grid_totals_f (FP32 warp sums, FP64 block and grid
@@ -298,25 +301,61 @@ struct BwdArgs {
     int *err;
 };
 
+__device__ __forceinline__ float4 f4_add(float4 a, float4 b) {
+    return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+}
+
+// The warp's 32 rows (a thread a row, 32 values each) to chunks: out[s] holds values
+// 4 (lane % 8) .. + 3 of row 4 s + lane / 8.  tile: the warp's 4 KB of shared memory; the
+// 16-byte pieces of a row are swapped about by the row's number, so that neither side has
+// bank conflicts.
+__device__ __forceinline__ void rows_to_chunks(const float *v, float4 *out, uint8_t *tile, int lane) {
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+        *reinterpret_cast<float4 *>(tile + lane * 128 + ((q ^ (lane & 7)) << 4)) =
+            make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+    __syncwarp();
+#pragma unroll
+    for (int s = 0; s < 8; ++s) {
+        const int r = 4 * s + (lane >> 3);
+        out[s] = *reinterpret_cast<const float4 *>(tile + r * 128 + (((lane & 7) ^ (r & 7)) << 4));
+    }
+}
+
+// What bounds this kernel is the traffic of its gathers and streams through L1 and L2 (some
+// 700 bytes a row and layer) and, before, the work of feeding the tensor core.  Rows move as
+// chunks: eight lanes take one row's 32 FP32 features, 16 bytes each, so a load touches four
+// lines where a thread a row touches 32; only the accumulator, a row a lane, goes through
+// shared memory to chunks (rows_to_chunks).  The weight gradient's contraction runs over rows,
+// so its operands are the transposes of X and of dpre: both are read as MN-major operands from
+// the row-by-row tiles, and dpre's tile serves the input gradient's MMA as K-major operand as
+// well; nothing is transposed by 2-byte stores (96 a thread and tile), and BF16 activations go
+// from memory to the tile unconverted.  126,720 rows of a 7-point graph: 55 -> 33 us a
+// middle layer, 48 -> 29 the first, 34 -> 18 the last.
+// Encoder and decoder gradients are summed over a tile's rows pairwise, then over the tiles.
 template <bool TOP, bool L1>
-__global__ void __launch_bounds__(GT) k_gnn_bwd(BwdArgs a) {
+__global__ void __launch_bounds__(GT, 3) k_gnn_bwd(BwdArgs a) {
     extern __shared__ __align__(1024) uint8_t smem[];
-    uint8_t *sA1 = smem;                  // dpre: 128 rows x 32 (K = 32)
-    uint8_t *sB1 = smem + 8192;           // W: 64 inputs x 32 outputs (K = 32)
-    uint8_t *sA2 = smem + 12288;          // [X^T; 1; 0]: 128 x 128 rows (K = 128)
-    uint8_t *sB2 = smem + 45056;          // dpre^T: 32 outputs x 128 rows (K = 128)
-    float *sprm = reinterpret_cast<float *>(smem + 53248);  // e, c, w_d
-    float *sred = sprm + 96;                                 // [4 warps][64]
-    uint64_t *bar = reinterpret_cast<uint64_t *>(smem + 53248 + 2048);
+    uint8_t *sX = smem;                         // [X, 1, 0]: 16 groups of 8 features x 128 rows x 16 bytes
+    uint8_t *sW = smem + BWD_X;                 // W: 64 inputs x 32 outputs (K = 32)
+    uint8_t *sT = sW + BWD_W;                   // 4 KB a warp: accumulator rows to chunks
+    uint8_t *sD = sT + BWD_T;                   // dpre: 4 groups of 8 outputs x 128 rows x 16 bytes, padded
+    float *sprm = reinterpret_cast<float *>(sD + BWD_D);  // e, c, w_d
+    float *sred = sprm + 96;                              // [4 warps][64]
+    uint64_t *bar = reinterpret_cast<uint64_t *>(sprm + 96 + 256);
     uint32_t *tslot = reinterpret_cast<uint32_t *>(bar + 1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int q8 = lane & 7, r4 = lane >> 3;  // chunk of a row, row within a step of four
 
     for (int q = tid; q < 64 * 4; q += GT) {
         int i = q >> 2, c = q & 3;
         uint4 w = *reinterpret_cast<const uint4 *>(a.wbf + 2048 + i * 32 + c * 8);
-        *reinterpret_cast<uint4 *>(sB1 + ((i >> 3) * 4 + c) * 128 + (i & 7) * 16) = w;
+        *reinterpret_cast<uint4 *>(sW + ((i >> 3) * 4 + c) * 128 + (i & 7) * 16) = w;
     }
-    for (int q = tid; q < 32768 / 16; q += GT) reinterpret_cast<uint4 *>(sA2)[q] = make_uint4(0, 0, 0, 0);
+    // features 64 (1: the bias gradient; rows past the end have dpre = 0) and 65 .. 127 (0)
+    for (int g = 8; g < 16; ++g)
+        *reinterpret_cast<uint4 *>(sX + g * 2048 + tid * 16) = make_uint4(g == 8 ? 0x3F80u : 0u, 0, 0, 0);
     if (tid < 32) {
         sprm[tid] = a.prm[GNN_OFF_ENC + tid];
         sprm[32 + tid] = a.prm[GNN_OFF_ENC + 32 + tid];
@@ -332,34 +371,35 @@ __global__ void __launch_bounds__(GT) k_gnn_bwd(BwdArgs a) {
     __syncthreads();
     umma::fence_after_sync();
     const uint32_t tmem = *tslot;
-    const float inv_s = *a.inv_s_p, s = *a.s_p;
+    const float inv_s = *a.inv_s_p, s_net = *a.s_p;
     const int n = a.g.n, ntiles = (n + GT - 1) / GT;
-    const uint32_t a1 = umma::smem_addr(sA1), b1 = umma::smem_addr(sB1);
-    const uint32_t a2 = umma::smem_addr(sA2), b2 = umma::smem_addr(sB2);
+    const uint32_t x0 = umma::smem_addr(sX), w0 = umma::smem_addr(sW), d0 = umma::smem_addr(sD);
     const double den = TOP ? a.sc->loss_den : 1.0;
     const float gscale = TOP ? (float)(2.0 / (den > 0.0 ? den : 1.0)) : 0.f;
-    // per-CTA sums kept by lane c % 32 of each warp: [0] value c, [1] value c + 32
-    float acc0 = 0.f, acc1 = 0.f, acc2 = 0.f;
+    // sums over the CTA's rows: TOP: the decoder's weights (this lane's chunk) and bias;
+    // L1: the encoder's e and c (this lane's chunk)
+    float4 acc_a = make_float4(0.f, 0.f, 0.f, 0.f), acc_b = acc_a;
+    float acc_s = 0.f;
     int it = 0;
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++it) {
-        const int row = t * GT + tid;
+        const int row0 = t * GT + warp * 32;  // the warp's rows: one slice
+        const int row = row0 + lane;
         const bool valid = row < n;
-        float delta[32];
-        float xh[32], xm[32];
-        float ui = 0.f, ai = 0.f, wi = 0.f, di = 0.f, gs = 0.f;
-#pragma unroll
-        for (int c = 0; c < 32; ++c) {
-            delta[c] = 0.f;
-            xh[c] = 0.f;
-            xm[c] = 0.f;
-        }
+        float4 delta[8];
+        float ui = 0.f, ai = 0.f, wi = 0.f, di = 0.f;
         uint32_t mbits = 0;
+        int base = 0, w = 0;
+        if (row0 < n) {
+            base = a.g.sl_ptr[row0 >> 5];
+            w = a.g.sl_w[row0 >> 5];
+        }
         if (valid) {
-            const int sl = row >> 5;
-            const int base = a.g.sl_ptr[sl], w = a.g.sl_w[sl];
             di = a.g.dinv[row];
             mbits = a.mask[row];
-            if (TOP) {
+        }
+        if (TOP) {
+            float gs = 0.f;
+            if (valid) {
                 float gz;
                 if (a.kind == 0) {
                     gz = gscale * a.y[row];
@@ -371,119 +411,98 @@ __global__ void __launch_bounds__(GT) k_gnn_bwd(BwdArgs a) {
                     }
                     gz = gscale * a.sgn * sy;
                 }
-                gs = gz * s;
+                gs = gz * s_net;
+            }
+            const float4 wd = *reinterpret_cast<const float4 *>(sprm + 64 + 4 * q8);
+            float4 pair[8];
 #pragma unroll
-                for (int c = 0; c < 32; ++c) delta[c] = gs * sprm[64 + c];
-            } else {
-                const float4 *dp = reinterpret_cast<const float4 *>(a.dIn + (size_t)row * 32);
+            for (int s = 0; s < 8; ++s) {
+                const int r = 4 * s + r4;
+                const float gr = __shfl_sync(FULL_MASK, gs, r);
+                delta[s] = make_float4(gr * wd.x, gr * wd.y, gr * wd.z, gr * wd.w);
+                uint2 h = make_uint2(0, 0);
+                if (row0 + r < n) h = *reinterpret_cast<const uint2 *>(a.h4 + (size_t)(row0 + r) * 32 + 4 * q8);
+                pair[s] = make_float4(gr * bf_lo(h.x), gr * bf_hi(h.x), gr * bf_lo(h.y), gr * bf_hi(h.y));
+            }
 #pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    float4 d4 = dp[q];
-                    delta[4 * q] = d4.x;
-                    delta[4 * q + 1] = d4.y;
-                    delta[4 * q + 2] = d4.z;
-                    delta[4 * q + 3] = d4.w;
+            for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+                for (int s = 0; s < o; ++s) pair[s] = f4_add(pair[s], pair[s + o]);
+            acc_a = f4_add(acc_a, pair[0]);
+            acc_s += gs;
+        } else {
+#pragma unroll
+            for (int s = 0; s < 8; ++s) {
+                const int r = row0 + 4 * s + r4;
+                delta[s] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (r < n) delta[s] = *reinterpret_cast<const float4 *>(a.dIn + (size_t)r * 32 + 4 * q8);
+            }
+            int cn = 0;
+            float vn = 0.f;
+            if (valid && w > 1) {
+                cn = a.g.col[base + 32 + lane];
+                vn = a.g.val[base + 32 + lane];
+            }
+            for (int k = 1; k < w; ++k) {
+                const int c = cn;
+                const float v = vn;
+                if (valid && k + 1 < w) {
+                    cn = a.g.col[base + (k + 1) * 32 + lane];
+                    vn = a.g.val[base + (k + 1) * 32 + lane];
                 }
-                for (int k = 1; k < w; ++k) {
-                    int pos = base + k * 32 + lane;
-                    int j = a.g.col[pos];
-                    float v = a.g.val[pos];
-                    const float4 *gp = reinterpret_cast<const float4 *>(a.gIn + (size_t)j * 32);
 #pragma unroll
-                    for (int q = 0; q < 8; ++q) {
-                        float4 g4 = gp[q];
-                        delta[4 * q] += v * g4.x;
-                        delta[4 * q + 1] += v * g4.y;
-                        delta[4 * q + 2] += v * g4.z;
-                        delta[4 * q + 3] += v * g4.w;
-                    }
+                for (int s = 0; s < 8; ++s) {
+                    const int j = __shfl_sync(FULL_MASK, c, 4 * s + r4);
+                    const float vj = __shfl_sync(FULL_MASK, v, 4 * s + r4);
+                    const float4 g4 = *reinterpret_cast<const float4 *>(a.gIn + (size_t)j * 32 + 4 * q8);
+                    delta[s].x += vj * g4.x;
+                    delta[s].y += vj * g4.y;
+                    delta[s].z += vj * g4.z;
+                    delta[s].w += vj * g4.w;
                 }
             }
-            if (L1) {
+        }
+        // the operand tiles
+        if (L1) {
+            if (valid) {
                 ai = a.aw[2 * (size_t)row];
                 wi = a.aw[2 * (size_t)row + 1];
                 ui = di * a.r[row] * inv_s;
+            }
 #pragma unroll
-                for (int c = 0; c < 32; ++c) {
-                    xh[c] = bf_round(ui * sprm[c] + sprm[32 + c]);
-                    xm[c] = bf_round(ai * sprm[c] + wi * sprm[32 + c]);
+            for (int g = 0; g < 4; ++g) {
+                uint32_t h[4], m[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int c = 8 * g + 2 * e;
+                    h[e] = valid ? bf_pack(ui * sprm[c] + sprm[32 + c], ui * sprm[c + 1] + sprm[33 + c]) : 0u;
+                    m[e] = bf_pack(ai * sprm[c] + wi * sprm[32 + c], ai * sprm[c + 1] + wi * sprm[33 + c]);
                 }
-            } else {
-                const uint4 *hp = reinterpret_cast<const uint4 *>(a.hprev + (size_t)row * 32);
-                const uint4 *mp = reinterpret_cast<const uint4 *>(a.mcur + (size_t)row * 32);
+                *reinterpret_cast<uint4 *>(sX + g * 2048 + tid * 16) = make_uint4(h[0], h[1], h[2], h[3]);
+                *reinterpret_cast<uint4 *>(sX + (4 + g) * 2048 + tid * 16) = make_uint4(m[0], m[1], m[2], m[3]);
+            }
+        } else {
+            // eight rows of 64 bytes a load
+            const int g = lane >> 3;
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    uint4 h4 = hp[q], m4 = mp[q];
-                    uint32_t hw[4] = {h4.x, h4.y, h4.z, h4.w}, mw[4] = {m4.x, m4.y, m4.z, m4.w};
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        xh[8 * q + 2 * e] = bf_lo(hw[e]);
-                        xh[8 * q + 2 * e + 1] = bf_hi(hw[e]);
-                        xm[8 * q + 2 * e] = bf_lo(mw[e]);
-                        xm[8 * q + 2 * e + 1] = bf_hi(mw[e]);
-                    }
+            for (int s = 0; s < 4; ++s) {
+                const int r = 8 * s + (lane & 7);
+                uint4 h = make_uint4(0, 0, 0, 0), m = h;
+                if (row0 + r < n) {
+                    h = *reinterpret_cast<const uint4 *>(a.hprev + (size_t)(row0 + r) * 32 + 8 * g);
+                    m = *reinterpret_cast<const uint4 *>(a.mcur + (size_t)(row0 + r) * 32 + 8 * g);
                 }
+                *reinterpret_cast<uint4 *>(sX + g * 2048 + (warp * 32 + r) * 16) = h;
+                *reinterpret_cast<uint4 *>(sX + (4 + g) * 2048 + (warp * 32 + r) * 16) = m;
             }
         }
-        // decoder gradient (w_d, b_d) from the stored h4
-        if (TOP) {
-            float h4v[32];
 #pragma unroll
-            for (int c = 0; c < 32; ++c) h4v[c] = 0.f;
-            if (valid) {
-                const uint4 *hp = reinterpret_cast<const uint4 *>(a.h4 + (size_t)row * 32);
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    uint4 h4 = hp[q];
-                    uint32_t hw[4] = {h4.x, h4.y, h4.z, h4.w};
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        h4v[8 * q + 2 * e] = bf_lo(hw[e]);
-                        h4v[8 * q + 2 * e + 1] = bf_hi(hw[e]);
-                    }
-                }
-            }
-#pragma unroll
-            for (int c = 0; c < 32; ++c) {
-                float v = gs * h4v[c];
-                for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULL_MASK, v, o);
-                if (lane == c) acc0 += v;
-            }
-            float v = gs;
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULL_MASK, v, o);
-            if (lane == 0) acc2 += v;
-        }
-        // operand tiles
-        uint32_t dp16[16];
-#pragma unroll
-        for (int c = 0; c < 32; c += 2) {
-            float d0 = (mbits >> c) & 1u ? delta[c] : 0.f;
-            float d1 = (mbits >> (c + 1)) & 1u ? delta[c + 1] : 0.f;
-            dp16[c >> 1] = bf_pack(d0, d1);
-        }
-        {
-            uint8_t *rowp = sA1 + (tid >> 3) * 4 * 128 + (tid & 7) * 16;
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-                *reinterpret_cast<uint4 *>(rowp + q * 128) =
-                    make_uint4(dp16[4 * q], dp16[4 * q + 1], dp16[4 * q + 2], dp16[4 * q + 3]);
-        }
-        {
-            // transposed tiles: element (feature, row = tid)
-            const uint32_t colo = ((tid >> 3) << 7) + ((tid & 7) << 1);
-#pragma unroll
-            for (int c = 0; c < 32; ++c) {
-                uint16_t v = (uint16_t)((c & 1) ? (dp16[c >> 1] >> 16) : (dp16[c >> 1] & 0xFFFFu));
-                *reinterpret_cast<uint16_t *>(sB2 + ((c >> 3) * 16) * 128 + ((c & 7) << 4) + colo) = v;
-            }
-#pragma unroll
-            for (int c = 0; c < 32; ++c) {
-                *reinterpret_cast<uint16_t *>(sA2 + ((c >> 3) * 16) * 128 + ((c & 7) << 4) + colo) =
-                    __bfloat16_as_ushort(__float2bfloat16_rn(xh[c]));
-                *reinterpret_cast<uint16_t *>(sA2 + (((c + 32) >> 3) * 16) * 128 + ((c & 7) << 4) + colo) =
-                    __bfloat16_as_ushort(__float2bfloat16_rn(xm[c]));
-            }
-            *reinterpret_cast<uint16_t *>(sA2 + (8 * 16) * 128 + colo) = valid ? (uint16_t)0x3F80u : (uint16_t)0u;
+        for (int s = 0; s < 8; ++s) {
+            const int r = 4 * s + r4;
+            const uint32_t mb = __shfl_sync(FULL_MASK, mbits, r) >> (4 * q8);
+            const uint2 dp = make_uint2(bf_pack(mb & 1u ? delta[s].x : 0.f, mb & 2u ? delta[s].y : 0.f),
+                                        bf_pack(mb & 4u ? delta[s].z : 0.f, mb & 8u ? delta[s].w : 0.f));
+            *reinterpret_cast<uint2 *>(sD + (q8 >> 1) * BWD_DG + (warp * 32 + r) * 16 + (q8 & 1) * 8) = dp;
         }
         umma::fence_smem_to_async();
         umma::fence_before_sync();
@@ -492,12 +511,12 @@ __global__ void __launch_bounds__(GT) k_gnn_bwd(BwdArgs a) {
             umma::fence_after_sync();
 #pragma unroll
             for (int kk = 0; kk < 2; ++kk)
-                umma::mma_bf16(tmem, umma::smem_desc(a1 + kk * 256, 128, 512), umma::smem_desc(b1 + kk * 256, 128, 512),
-                               IDESC_B1, kk > 0);
+                umma::mma_bf16(tmem, umma::smem_desc(d0 + kk * 2 * BWD_DG, BWD_DG, 128),
+                               umma::smem_desc(w0 + kk * 256, 128, 512), IDESC_B1, kk > 0);
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk)
-                umma::mma_bf16(tmem + 64, umma::smem_desc(a2 + kk * 256, 128, 2048),
-                               umma::smem_desc(b2 + kk * 256, 128, 2048), IDESC_B2, it > 0 || kk > 0);
+                umma::mma_bf16(tmem + 64, umma::smem_desc(x0 + kk * 256, 128, 2048),
+                               umma::smem_desc(d0 + kk * 256, 128, BWD_DG), IDESC_B2, it > 0 || kk > 0);
             umma::commit(bar);
         }
         __syncwarp();
@@ -507,36 +526,53 @@ __global__ void __launch_bounds__(GT) k_gnn_bwd(BwdArgs a) {
             break;
         }
         umma::fence_after_sync();
-        float dxh[32], dxm[32];
+        uint8_t *tile = sT + warp * 4096;
         const uint32_t lb = (uint32_t)(warp * 32) << 16;
-        umma::ld32(tmem + lb, dxh);
-        umma::ld32(tmem + lb + 32, dxm);
-        if (!L1) {
-            if (valid) {
-                float4 *dp = reinterpret_cast<float4 *>(a.dOut + (size_t)row * 32);
-                float4 *gp = reinterpret_cast<float4 *>(a.gOut + (size_t)row * 32);
+        {
+            float acc[32];
+            float4 dx[8];
+            umma::ld32(tmem + lb, acc);
+            rows_to_chunks(acc, dx, tile, lane);
 #pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    dp[q] = make_float4(delta[4 * q] + dxh[4 * q], delta[4 * q + 1] + dxh[4 * q + 1],
-                                        delta[4 * q + 2] + dxh[4 * q + 2], delta[4 * q + 3] + dxh[4 * q + 3]);
-                    gp[q] = make_float4(di * dxm[4 * q], di * dxm[4 * q + 1], di * dxm[4 * q + 2], di * dxm[4 * q + 3]);
-                }
+            for (int s = 0; s < 8; ++s) {
+                delta[s] = f4_add(delta[s], dx[s]);
+                const int r = row0 + 4 * s + r4;
+                if (!L1 && r < n) *reinterpret_cast<float4 *>(a.dOut + (size_t)r * 32 + 4 * q8) = delta[s];
             }
-        } else {
-            // encoder: h0 = u e + c, m1 = a e + w c
+            umma::ld32(tmem + lb + 32, acc);
+            rows_to_chunks(acc, dx, tile, lane);
+            if (!L1) {
 #pragma unroll
-            for (int c = 0; c < 32; ++c) {
-                float dh0 = valid ? delta[c] + dxh[c] : 0.f;
-                float dm1 = valid ? dxm[c] : 0.f;
-                float ve = ui * dh0 + ai * dm1, vc = dh0 + wi * dm1;
-                for (int o = 16; o > 0; o >>= 1) {
-                    ve += __shfl_xor_sync(FULL_MASK, ve, o);
-                    vc += __shfl_xor_sync(FULL_MASK, vc, o);
+                for (int s = 0; s < 8; ++s) {
+                    const int r = row0 + 4 * s + r4;
+                    const float d = __shfl_sync(FULL_MASK, di, 4 * s + r4);
+                    if (r < n)
+                        *reinterpret_cast<float4 *>(a.gOut + (size_t)r * 32 + 4 * q8) =
+                            make_float4(d * dx[s].x, d * dx[s].y, d * dx[s].z, d * dx[s].w);
                 }
-                if (lane == c) {
-                    acc0 += ve;
-                    acc1 += vc;
+            } else {
+                // encoder: h0 = u e + c, m1 = a e + w c; rows past the end count as zero
+                float4 ce[8];
+#pragma unroll
+                for (int s = 0; s < 8; ++s) {
+                    const int r = 4 * s + r4;
+                    const bool in = row0 + r < n;
+                    const float u = __shfl_sync(FULL_MASK, ui, r), aa = __shfl_sync(FULL_MASK, ai, r),
+                                ww = __shfl_sync(FULL_MASK, wi, r);
+                    const float4 h = in ? delta[s] : make_float4(0.f, 0.f, 0.f, 0.f);
+                    const float4 m = in ? dx[s] : make_float4(0.f, 0.f, 0.f, 0.f);
+                    ce[s] = make_float4(u * h.x + aa * m.x, u * h.y + aa * m.y, u * h.z + aa * m.z, u * h.w + aa * m.w);
+                    dx[s] = make_float4(h.x + ww * m.x, h.y + ww * m.y, h.z + ww * m.z, h.w + ww * m.w);
                 }
+#pragma unroll
+                for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+                    for (int s = 0; s < o; ++s) {
+                        ce[s] = f4_add(ce[s], ce[s + o]);
+                        dx[s] = f4_add(dx[s], dx[s + o]);
+                    }
+                acc_a = f4_add(acc_a, ce[0]);
+                acc_b = f4_add(acc_b, dx[0]);
             }
         }
         umma::fence_before_sync();
@@ -549,24 +585,39 @@ __global__ void __launch_bounds__(GT) k_gnn_bwd(BwdArgs a) {
     if (warp < 3) {
         float dw[32];
         umma::ld32(tmem + ((uint32_t)(warp * 32) << 16) + 64, dw);
-        const int m = warp * 32 + lane;
-        if (m < 64) {
 #pragma unroll
-            for (int o = 0; o < 32; ++o) lrec[m * 32 + o] = it > 0 ? dw[o] : 0.f;
-        } else if (m == 64) {
+        for (int o = 0; o < 32; ++o) dw[o] = it > 0 ? dw[o] : 0.f;
+        if (warp < 2) {
+            float4 ch[8];
+            rows_to_chunks(dw, ch, sT + warp * 4096, lane);
 #pragma unroll
-            for (int o = 0; o < 32; ++o) lrec[2048 + o] = it > 0 ? dw[o] : 0.f;
+            for (int s = 0; s < 8; ++s)
+                *reinterpret_cast<float4 *>(lrec + (warp * 32 + 4 * s + r4) * 32 + 4 * q8) = ch[s];
+        } else if (lane == 0) {
+#pragma unroll
+            for (int o = 0; o < 32; ++o) lrec[2048 + o] = dw[o];
         }
     }
     if (TOP || L1) {
-        sred[warp * 64 + lane] = acc0;
-        sred[warp * 64 + 32 + lane] = TOP ? (lane == 0 ? acc2 : 0.f) : acc1;
+#pragma unroll
+        for (int o = 16; o >= 8; o >>= 1) {  // over the four rows of a step
+            acc_a = f4_add(acc_a, make_float4(__shfl_xor_sync(FULL_MASK, acc_a.x, o), __shfl_xor_sync(FULL_MASK, acc_a.y, o),
+                                              __shfl_xor_sync(FULL_MASK, acc_a.z, o), __shfl_xor_sync(FULL_MASK, acc_a.w, o)));
+            if (L1)
+                acc_b = f4_add(acc_b, make_float4(__shfl_xor_sync(FULL_MASK, acc_b.x, o), __shfl_xor_sync(FULL_MASK, acc_b.y, o),
+                                                  __shfl_xor_sync(FULL_MASK, acc_b.z, o), __shfl_xor_sync(FULL_MASK, acc_b.w, o)));
+        }
+        if (TOP)
+            for (int o = 16; o > 0; o >>= 1) acc_s += __shfl_xor_sync(FULL_MASK, acc_s, o);
+        if (r4 == 0) {
+            *reinterpret_cast<float4 *>(sred + warp * 64 + 4 * q8) = acc_a;
+            *reinterpret_cast<float4 *>(sred + warp * 64 + 32 + 4 * q8) = TOP ? make_float4(acc_s, 0.f, 0.f, 0.f) : acc_b;
+        }
         __syncthreads();
         if (tid < 64) {
             float v = sred[tid] + sred[64 + tid] + sred[128 + tid] + sred[192 + tid];
             if (TOP) {
-                if (tid < 32) rec[GNN_OFF_DEC + tid] = v;
-                else if (tid == 32) rec[GNN_OFF_DEC + 32] = v;
+                if (tid <= 32) rec[GNN_OFF_DEC + tid] = v;
             } else {
                 rec[GNN_OFF_ENC + tid] = v;
             }

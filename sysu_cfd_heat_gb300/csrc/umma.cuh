@@ -12,6 +12,13 @@
 // adjacent in K) is 128 and the stride-dimension byte offset (between adjacent
 // 8-row groups) is K / 8 * 128.  One MMA consumes K = 16 (two core matrices), so
 // step kk starts 256 * kk bytes further.
+//
+// MN-major operand (the transpose of what lies in memory; IDESC_A_MN / IDESC_B_MN): a core
+// matrix is 8 values of K of 16 bytes each, 8 neighbours along M or N; the leading-dimension
+// offset is between core matrices adjacent in K, the stride-dimension offset between those
+// adjacent along M or N.  So one tile stored as groups of 8 columns, byte(r, c) =
+// (c / 8) * G + r * 16 + (c % 8) * 2, is a K-major operand of its rows (leading G, stride 128)
+// and an MN-major one of its columns (leading 128, stride G).
 #pragma once
 
 #include <cstdint>
@@ -44,6 +51,9 @@ __host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N) {
            | ((uint32_t)(N >> 3) << 17)      // N / 8
            | ((uint32_t)(M >> 4) << 24);     // M / 16
 }
+
+// operand stored MN-major (transposed) instead of K-major
+constexpr uint32_t IDESC_A_MN = 1u << 15, IDESC_B_MN = 1u << 16;
 
 // Tensor-memory allocation by one full warp; the column base is written to
 // *dst (shared memory).  ncols: a power of two >= 32.
