@@ -34,7 +34,8 @@ constexpr uint32_t IDESC_B1 = umma::idesc_bf16_f32(128, 64);  // backward, input
 // backward, weight gradient: 128 x 32, K = 128, both operands MN-major
 constexpr uint32_t IDESC_B2 = umma::idesc_bf16_f32(128, 32) | umma::IDESC_A_MN | umma::IDESC_B_MN;
 
-constexpr int FWD_SMEM = 16384 + 4096 + 1024;
+constexpr int FWD_G = 2048 + 32;  // forward: a group of the operand tile
+constexpr int FWD_SMEM = 8 * FWD_G + 4096 + 136 * 4 + 16;
 // backward: X tile, weights, transposition tiles, dpre tile (the 32 bytes between its groups
 // spread a row's four groups over the banks), parameters and sums
 constexpr int BWD_X = 32768, BWD_W = 4096, BWD_T = 16384, BWD_DG = 2048 + 32, BWD_D = 4 * BWD_DG;
@@ -86,15 +87,29 @@ struct NetArgs {
     int *err;
 };
 
-template <bool L1, bool TRAIN, bool DEC>
+// What bounds this kernel is its gathers: a row's neighbours, 64 bytes of BF16 features each.
+// TR, the rows of a tile:
+//   128  a thread gathers and finishes its own row; 28 warps an SM hide the latencies.
+//   32   four lanes take a row, 16 bytes each, and the four warps eight rows each; eight
+//        neighbours' features are in flight and the next eight columns on their way.  The
+//        MMA's other 96 rows go unused, and one warp finishes the 32 rows.  For levels of a few
+//        thousand rows, where 128-row tiles leave most SMs without work and the time is one
+//        thread's chain of gathers: 7 to 9 us a layer where that took 16 to 18 (second coarse
+//        level of a 264,000-cell tetrahedral mesh).
+// The operand tile is stored as groups of 8 features, byte(r, c) = (c / 8) * FWD_G + 16 r +
+// 2 (c % 8); the 32 bytes between groups keep a row's four lanes on different banks, and the
+// new features leave through it, four lanes a row (126,720 rows, four layers: 64 -> 61 us).
+template <bool L1, bool TRAIN, bool DEC, int TR>
 __global__ void __launch_bounds__(GT) k_gnn_fwd(NetArgs a) {
     extern __shared__ __align__(1024) uint8_t smem[];
-    uint8_t *sA = smem;          // X tile: 128 rows x 64 (K-adjacent, K = 64)
-    uint8_t *sB = smem + 16384;  // Wt: 32 outputs x 64 inputs
-    float *sprm = reinterpret_cast<float *>(smem + 20480);  // bias, e, c, w_d, b_d
-    uint64_t *bar = reinterpret_cast<uint64_t *>(smem + 20480 + 136 * 4);
+    uint8_t *sX = smem;          // [h, m]: 8 groups of 8 features x 128 rows
+    uint8_t *sB = smem + 8 * FWD_G;  // Wt: 32 outputs x 64 inputs
+    float *sprm = reinterpret_cast<float *>(sB + 4096);  // bias, e, c, w_d, b_d
+    uint64_t *bar = reinterpret_cast<uint64_t *>(sprm + 136);
     uint32_t *tslot = reinterpret_cast<uint32_t *>(bar + 1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int q4 = lane & 3, l8 = 8 * warp + (lane >> 2);  // 32-row tiles: this lane's chunk and row
+    const int s0 = TR == 128 ? 32 * warp : 0;              // the warp's slice in the tile
     if (a.fs && (a.fs->done || !a.fs->use_gnn)) return;
 
     for (int q = tid; q < 32 * 8; q += GT) {
@@ -120,27 +135,30 @@ __global__ void __launch_bounds__(GT) k_gnn_fwd(NetArgs a) {
     __syncthreads();
     umma::fence_after_sync();
     const uint32_t tmem = *tslot;
-    const float inv_s = *a.inv_s_p, s = *a.s_p;
-    const int n = a.g.n, ntiles = (n + GT - 1) / GT;
-    const uint32_t a0 = umma::smem_addr(sA), b0 = umma::smem_addr(sB);
+    const float inv_s = *a.inv_s_p, s_net = *a.s_p;
+    const int n = a.g.n, ntiles = (n + TR - 1) / TR;
+    const uint32_t x0 = umma::smem_addr(sX), b0 = umma::smem_addr(sB);
+    const bool rows = TR == 128 || warp == 0;                // has a row a thread
+    uint8_t *xrow = sX + tid * 16;                           // this thread's row
+    uint8_t *xchunk = sX + q4 * FWD_G + l8 * 16;             // 32-row tiles: this lane's chunk
     float zq = 0.f;
     int it = 0;
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++it) {
-        const int row = t * GT + tid;
+        const int row0 = t * TR + s0;  // the warp's slice
+        const int row = row0 + lane;
         const bool valid = row < n;
-        float mv[32];
-        uint32_t hs[16];
-#pragma unroll
-        for (int c = 0; c < 32; ++c) mv[c] = 0.f;
-#pragma unroll
-        for (int c = 0; c < 16; ++c) hs[c] = 0u;
-        float ui = 0.f, di = 0.f;
-        if (valid) {
-            const int sl = row >> 5;
-            const int base = a.g.sl_ptr[sl], w = a.g.sl_w[sl];
-            di = a.g.dinv[row];
-            if (L1) {
+        int base = 0, w = 0;
+        if (row0 < n) {
+            base = a.g.sl_ptr[row0 >> 5];
+            w = a.g.sl_w[row0 >> 5];
+        }
+        const float di = valid ? a.g.dinv[row] : 0.f;
+        uint32_t hs[16];  // the row's h (BF16 pairs)
+        if (L1 && rows) {
+            float ui = 0.f, ai = 0.f, wi = 0.f;
+            if (valid) {
                 float su = 0.f, sw = 0.f;
+#pragma unroll 4
                 for (int k = 1; k < w; ++k) {
                     int pos = base + k * 32 + lane;
                     int j = a.g.col[pos];
@@ -148,30 +166,44 @@ __global__ void __launch_bounds__(GT) k_gnn_fwd(NetArgs a) {
                     su += v * (a.g.dinv[j] * a.r[j]);
                     sw += v;
                 }
-                float ai = di * su * inv_s, wi = di * sw;
+                ai = di * su * inv_s;
+                wi = di * sw;
                 ui = di * a.r[row] * inv_s;
-#pragma unroll
-                for (int c = 0; c < 32; c += 2) {
-                    float e0 = sprm[32 + c], e1 = sprm[33 + c], c0 = sprm[64 + c], c1 = sprm[65 + c];
-                    hs[c >> 1] = bf_pack(ui * e0 + c0, ui * e1 + c1);
-                    mv[c] = ai * e0 + wi * c0;
-                    mv[c + 1] = ai * e1 + wi * c1;
-                }
                 if (TRAIN) {
                     a.aw[2 * (size_t)row] = ai;
                     a.aw[2 * (size_t)row + 1] = wi;
                 }
-            } else {
-                {
-                    const uint4 *hp = reinterpret_cast<const uint4 *>(a.hin + (size_t)row * 32);
+            }
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        uint4 h4 = __ldg(hp + q);
-                        hs[4 * q] = h4.x;
-                        hs[4 * q + 1] = h4.y;
-                        hs[4 * q + 2] = h4.z;
-                        hs[4 * q + 3] = h4.w;
-                    }
+            for (int g = 0; g < 4; ++g) {
+                uint32_t m[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int c = 8 * g + 2 * e;
+                    const float e0 = sprm[32 + c], e1 = sprm[33 + c], c0 = sprm[64 + c], c1 = sprm[65 + c];
+                    hs[4 * g + e] = valid ? bf_pack(ui * e0 + c0, ui * e1 + c1) : 0u;
+                    m[e] = bf_pack(ai * e0 + wi * c0, ai * e1 + wi * c1);
+                }
+                *reinterpret_cast<uint4 *>(xrow + g * FWD_G) =
+                    make_uint4(hs[4 * g], hs[4 * g + 1], hs[4 * g + 2], hs[4 * g + 3]);
+                *reinterpret_cast<uint4 *>(xrow + (4 + g) * FWD_G) = make_uint4(m[0], m[1], m[2], m[3]);
+            }
+        }
+        if (!L1 && TR == 128) {
+            float mv[32];
+#pragma unroll
+            for (int c = 0; c < 32; ++c) mv[c] = 0.f;
+#pragma unroll
+            for (int c = 0; c < 16; ++c) hs[c] = 0u;
+            if (valid) {
+                const uint4 *hp = reinterpret_cast<const uint4 *>(a.hin + (size_t)row * 32);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const uint4 h4 = __ldg(hp + q);
+                    hs[4 * q] = h4.x;
+                    hs[4 * q + 1] = h4.y;
+                    hs[4 * q + 2] = h4.z;
+                    hs[4 * q + 3] = h4.w;
                 }
                 // two neighbours per step: eight 16-byte loads in flight per thread
                 for (int k = 1; k < w; k += 2) {
@@ -191,8 +223,8 @@ __global__ void __launch_bounds__(GT) k_gnn_fwd(NetArgs a) {
                     }
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
-                        uint32_t xw[4] = {x[q].x, x[q].y, x[q].z, x[q].w};
-                        uint32_t yw[4] = {y[q].x, y[q].y, y[q].z, y[q].w};
+                        const uint32_t xw[4] = {x[q].x, x[q].y, x[q].z, x[q].w};
+                        const uint32_t yw[4] = {y[q].x, y[q].y, y[q].z, y[q].w};
 #pragma unroll
                         for (int e = 0; e < 4; ++e) {
                             mv[8 * q + 2 * e] += v0 * bf_lo(xw[e]) + v1 * bf_lo(yw[e]);
@@ -200,24 +232,70 @@ __global__ void __launch_bounds__(GT) k_gnn_fwd(NetArgs a) {
                         }
                     }
                 }
+            }
 #pragma unroll
-                for (int c = 0; c < 32; ++c) mv[c] *= di;
+            for (int g = 0; g < 4; ++g) {
+                uint32_t m[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) m[e] = bf_pack(mv[8 * g + 2 * e] * di, mv[8 * g + 2 * e + 1] * di);
+                const uint4 m4 = make_uint4(m[0], m[1], m[2], m[3]);
+                *reinterpret_cast<uint4 *>(xrow + g * FWD_G) =
+                    make_uint4(hs[4 * g], hs[4 * g + 1], hs[4 * g + 2], hs[4 * g + 3]);
+                *reinterpret_cast<uint4 *>(xrow + (4 + g) * FWD_G) = m4;
+                if (TRAIN && valid) reinterpret_cast<uint4 *>(a.mout + (size_t)row * 32)[g] = m4;
             }
         }
-        uint32_t mp[16];
+        if (!L1 && TR == 32) {
+            const uint16_t *hq = a.hin + 8 * q4;
+            const bool in = row0 + l8 < n;
+            float mv[8];
 #pragma unroll
-        for (int c = 0; c < 16; ++c) mp[c] = bf_pack(mv[2 * c], mv[2 * c + 1]);
-        uint8_t *rowp = sA + (tid >> 3) * 8 * 128 + (tid & 7) * 16;
+            for (int e = 0; e < 8; ++e) mv[e] = 0.f;
+            int c[8];
+            float v[8];
+            auto entries = [&](int k) {  // columns and values of the row's neighbours k .. k + 7
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            *reinterpret_cast<uint4 *>(rowp + q * 128) = make_uint4(hs[4 * q], hs[4 * q + 1], hs[4 * q + 2], hs[4 * q + 3]);
-            *reinterpret_cast<uint4 *>(rowp + (4 + q) * 128) =
-                make_uint4(mp[4 * q], mp[4 * q + 1], mp[4 * q + 2], mp[4 * q + 3]);
-        }
-        if (TRAIN && !L1 && valid) {
-            uint4 *mo = reinterpret_cast<uint4 *>(a.mout + (size_t)row * 32);
+                for (int i = 0; i < 8; ++i) {
+                    c[i] = 0;
+                    v[i] = 0.f;
+                    if (in && k + i < w) {
+                        c[i] = a.g.col[base + (k + i) * 32 + l8];
+                        v[i] = a.g.val[base + (k + i) * 32 + l8];
+                    }
+                }
+            };
+            entries(1);
+            uint4 h = make_uint4(0, 0, 0, 0);
+            if (in) h = __ldg(reinterpret_cast<const uint4 *>(hq + (size_t)(row0 + l8) * 32));
+            // eight gathers in flight, the next eight neighbours' columns on their way
+            for (int k = 1; k < w; k += 8) {
+                uint4 x[8];
+                float u[8];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) mo[q] = make_uint4(mp[4 * q], mp[4 * q + 1], mp[4 * q + 2], mp[4 * q + 3]);
+                for (int i = 0; i < 8; ++i) {
+                    x[i] = __ldg(reinterpret_cast<const uint4 *>(hq + (size_t)c[i] * 32));
+                    u[i] = v[i];
+                }
+                entries(k + 8);
+#pragma unroll
+                for (int i = 0; i < 8; i += 2) {
+                    const uint32_t xw[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
+                    const uint32_t yw[4] = {x[i + 1].x, x[i + 1].y, x[i + 1].z, x[i + 1].w};
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        mv[2 * e] += u[i] * bf_lo(xw[e]) + u[i + 1] * bf_lo(yw[e]);
+                        mv[2 * e + 1] += u[i] * bf_hi(xw[e]) + u[i + 1] * bf_hi(yw[e]);
+                    }
+                }
+            }
+            const float d = __shfl_sync(FULL_MASK, di, l8);
+            uint32_t m[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) m[e] = in ? bf_pack(mv[2 * e] * d, mv[2 * e + 1] * d) : 0u;
+            const uint4 m4 = make_uint4(m[0], m[1], m[2], m[3]);
+            *reinterpret_cast<uint4 *>(xchunk) = h;
+            *reinterpret_cast<uint4 *>(xchunk + 4 * FWD_G) = m4;
+            if (TRAIN && in) *reinterpret_cast<uint4 *>(a.mout + (size_t)(row0 + l8) * 32 + 8 * q4) = m4;
         }
         umma::fence_smem_to_async();
         umma::fence_before_sync();
@@ -226,8 +304,8 @@ __global__ void __launch_bounds__(GT) k_gnn_fwd(NetArgs a) {
             umma::fence_after_sync();
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk)
-                umma::mma_bf16(tmem, umma::smem_desc(a0 + kk * 256, 128, 1024), umma::smem_desc(b0 + kk * 256, 128, 1024),
-                               IDESC_F, kk > 0);
+                umma::mma_bf16(tmem, umma::smem_desc(x0 + kk * 2 * FWD_G, FWD_G, 128),
+                               umma::smem_desc(b0 + kk * 256, 128, 1024), IDESC_F, kk > 0);
             umma::commit(bar);
         }
         __syncwarp();
@@ -237,9 +315,19 @@ __global__ void __launch_bounds__(GT) k_gnn_fwd(NetArgs a) {
             break;
         }
         umma::fence_after_sync();
-        float pre[32];
-        umma::ld32(tmem + ((uint32_t)(warp * 32) << 16), pre);
-        if (valid) {
+        if (rows) {
+            float pre[32];
+            umma::ld32(tmem + ((uint32_t)(warp * 32) << 16), pre);
+            if (!L1 && TR == 32) {
+#pragma unroll
+                for (int g = 0; g < 4; ++g) {
+                    const uint4 h = *reinterpret_cast<const uint4 *>(xrow + g * FWD_G);
+                    hs[4 * g] = h.x;
+                    hs[4 * g + 1] = h.y;
+                    hs[4 * g + 2] = h.z;
+                    hs[4 * g + 3] = h.w;
+                }
+            }
             uint32_t ho[16];
             uint32_t mbits = 0;
 #pragma unroll
@@ -251,23 +339,35 @@ __global__ void __launch_bounds__(GT) k_gnn_fwd(NetArgs a) {
                 mbits |= (p1 > 0.f ? 1u : 0u) << (c + 1);
                 ho[c >> 1] = bf_pack(h0, h1);
             }
-            if (!DEC || TRAIN) {
-                uint4 *hp = reinterpret_cast<uint4 *>(a.hout + (size_t)row * 32);
+            if (!DEC || TRAIN) {  // rows to chunks through the tile (this warp's rows only)
 #pragma unroll
-                for (int q = 0; q < 4; ++q) hp[q] = make_uint4(ho[4 * q], ho[4 * q + 1], ho[4 * q + 2], ho[4 * q + 3]);
+                for (int g = 0; g < 4; ++g)
+                    *reinterpret_cast<uint4 *>(xrow + g * FWD_G) =
+                        make_uint4(ho[4 * g], ho[4 * g + 1], ho[4 * g + 2], ho[4 * g + 3]);
+                __syncwarp();
+#pragma unroll
+                for (int s = 0; s < 4; ++s)
+                    if (row0 + 8 * s + (lane >> 2) < n)
+                        *reinterpret_cast<uint4 *>(a.hout + (size_t)(row0 + 8 * s + (lane >> 2)) * 32 + 8 * q4) =
+                            *reinterpret_cast<const uint4 *>(sX + q4 * FWD_G + (s0 + 8 * s + (lane >> 2)) * 16);
             }
-            if (TRAIN) a.mask[row] = mbits;
-            if (DEC) {
-                float acc = sprm[128];
+            if (valid) {
+                if (TRAIN) a.mask[row] = mbits;
+                if (DEC) {
+                    float acc = sprm[128];
 #pragma unroll
-                for (int c = 0; c < 32; c += 2) acc += sprm[96 + c] * bf_lo(ho[c >> 1]) + sprm[97 + c] * bf_hi(ho[c >> 1]);
-                float u = di * a.r[row] * inv_s;
-                float zi = s * (a.skip * u + acc);
-                if (a.zbase) zi += a.zbase[row];
-                a.z[row] = zi;
-                if (a.qprev) zq = fmaf(zi, a.qprev[row], zq);
+                    for (int c = 0; c < 32; c += 2) acc += sprm[96 + c] * bf_lo(ho[c >> 1]) + sprm[97 + c] * bf_hi(ho[c >> 1]);
+                    float u = di * a.r[row] * inv_s;
+                    float zi = s_net * (a.skip * u + acc);
+                    if (a.zbase) zi += a.zbase[row];
+                    a.z[row] = zi;
+                    if (a.qprev) zq = fmaf(zi, a.qprev[row], zq);
+                }
             }
         }
+        // the tile's rows are read before the next tile's are written
+        if (TR == 128) __syncwarp();
+        else __syncthreads();
     }
     if (DEC && a.fs) {
         const float fv[1] = {zq};
@@ -1170,12 +1270,16 @@ void GnnPrecond::bind(const SellDev &A, const double *val64, const float *val32,
     // the runtime's occupancy query reports one CTA per SM for kernels that
     // allocate tensor memory.
     cudaFuncAttributes fa{};
-    SYSU_CUDA(cudaFuncGetAttributes(&fa, k_gnn_fwd<false, true, true>));
+    SYSU_CUDA(cudaFuncGetAttributes(&fa, k_gnn_fwd<false, true, true, 128>));
     int by_regs = 65536 / std::max(1, fa.numRegs * GT);
     int by_smem = (227 * 1024) / (FWD_SMEM + (int)fa.sharedSizeBytes + 1024);
     int occ = std::max(1, std::min(std::min(by_regs, by_smem), 8));
     if (fwd_per_sm > 0) occ = fwd_per_sm;
-    gfwd_ = std::max(1, std::min(ntiles_, num_sms() * occ));
+    // 32-row tiles up to two CTAs an SM (9,728 rows on 152 SMs).  Four layers and their flat
+    // kernels on a 7-point graph, 32-row against 128-row tiles: 1,300 rows 24.6 and 30.7 us,
+    // 4,096 rows 26.6 and 30.7, 13,824 rows 32.8 and 31.8; wider rows gain more.
+    small_ = (n_ + 31) / 32 <= num_sms() * 2;
+    gfwd_ = std::max(1, std::min(small_ ? (n_ + 31) / 32 : ntiles_, num_sms() * occ));
     gtiles_ = std::max(1, std::min(ntiles_, num_sms() * 3));
     gflat_ = blocks_flat(n_);
     const size_t n = (size_t)n_;
@@ -1306,16 +1410,20 @@ void GnnPrecond::forward(const float *r32, float *z32, bool train, FcgState *fs,
             a.mask = nullptr;
         }
         dim3 grid(gfwd_), blk(GT);
-        if (l == 0) {
-            if (train) k_gnn_fwd<true, true, false><<<grid, blk, FWD_SMEM, st>>>(a);
-            else k_gnn_fwd<true, false, false><<<grid, blk, FWD_SMEM, st>>>(a);
-        } else if (l == GNN_LAYERS - 1) {
-            if (train) k_gnn_fwd<false, true, true><<<grid, blk, FWD_SMEM, st>>>(a);
-            else k_gnn_fwd<false, false, true><<<grid, blk, FWD_SMEM, st>>>(a);
-        } else {
-            if (train) k_gnn_fwd<false, true, false><<<grid, blk, FWD_SMEM, st>>>(a);
-            else k_gnn_fwd<false, false, false><<<grid, blk, FWD_SMEM, st>>>(a);
-        }
+        auto run = [&](auto TR) {
+            if (l == 0) {
+                if (train) k_gnn_fwd<true, true, false, TR.value><<<grid, blk, FWD_SMEM, st>>>(a);
+                else k_gnn_fwd<true, false, false, TR.value><<<grid, blk, FWD_SMEM, st>>>(a);
+            } else if (l == GNN_LAYERS - 1) {
+                if (train) k_gnn_fwd<false, true, true, TR.value><<<grid, blk, FWD_SMEM, st>>>(a);
+                else k_gnn_fwd<false, false, true, TR.value><<<grid, blk, FWD_SMEM, st>>>(a);
+            } else {
+                if (train) k_gnn_fwd<false, true, false, TR.value><<<grid, blk, FWD_SMEM, st>>>(a);
+                else k_gnn_fwd<false, false, false, TR.value><<<grid, blk, FWD_SMEM, st>>>(a);
+            }
+        };
+        if (small_) run(std::integral_constant<int, 32>{});
+        else run(std::integral_constant<int, 128>{});
         ++g_launches;
         SYSU_CUDA(cudaGetLastError());
     }

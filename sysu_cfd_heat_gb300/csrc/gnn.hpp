@@ -183,6 +183,7 @@ class GnnPrecond {
     const double *val64_ = nullptr;
     const float *val32_ = nullptr;
     int n_ = 0, ntiles_ = 0, gtiles_ = 0, gfwd_ = 0, gflat_ = 0;
+    bool small_ = false;  // the forward kernels take 32-row tiles
     float sgn_ = 1.0f;
     int capacity_ = 32, count_ = 0, next_ = 0, adam_t_ = 0;
 
