@@ -65,7 +65,8 @@ int sysu_csr_solve(int method, int precond, int n, const int *rowptr, const int 
         cudaStream_t st = os.st;
         {
             sysu::CsrDevice M;
-            M.load(n, rowptr, col, val, st);
+            if (precond <= 1 && method != 3) M.load_on_device(n, rowptr, col, val, st);
+            else M.load(n, rowptr, col, val, st);
             sysu::DevBuf<double> db(n), dx(n);
             db.upload(b, n, st);
             dx.upload(x, n, st);
@@ -149,7 +150,7 @@ int sysu_csr_spmv(int n, const int *rowptr, const int *col, const double *val, c
         cudaStream_t st = os.st;
         {
             sysu::CsrDevice M;
-            M.load(n, rowptr, col, val, st);
+            M.load_on_device(n, rowptr, col, val, st);
             sysu::DevBuf<double> dx(n), dy(n);
             dx.upload(x, n, st);
             sysu::DevBuf<int> err(1);
@@ -184,7 +185,7 @@ int sysu_csr_spmv_timing(int n, const int *rowptr, const int *col, const double 
         cudaStream_t st = os.st;
         {
             sysu::CsrDevice M;
-            M.load(n, rowptr, col, val, st);
+            M.load_on_device(n, rowptr, col, val, st);
             sysu::DevBuf<double> x64(n), y64(n);
             sysu::DevBuf<float> x32(n), y32(n), v32;
             sysu::DevBuf<unsigned char> flush((size_t)256 << 20);
@@ -302,7 +303,7 @@ int sysu_csr_bicgstab3(int n, const int *rowptr, const int *col, const double *v
         cudaStream_t st = os.st;
         {
             sysu::CsrDevice M;
-            M.load(n, rowptr, col, val, st);
+            M.load_on_device(n, rowptr, col, val, st);
             sysu::DevBuf<double> db[3], dx[3];
             for (int c = 0; c < 3; ++c) {
                 db[c].alloc(n);

@@ -2,6 +2,7 @@
 // entry points of the C ABI: csr_api.cpp, gnn_api.cpp).
 #pragma once
 
+#include <algorithm>
 #include <vector>
 
 #include "krylov.hpp"
@@ -44,6 +45,9 @@ struct CsrDevice {
         A.upload(pat, st);
         upload_values(vl, st);
     }
+    // The same device arrays without pat, rp, cl and the sweeps' level schedules: for solves without
+    // SSOR, ILU(0) or multigrid, and products (csr_device.cu).
+    void load_on_device(int n, const int *rowptr, const int *col, const double *v, cudaStream_t st);
     // new values for the same pattern (same rowptr and col as load)
     void reload_values(int n, const int *rowptr, const int *col, const double *v, cudaStream_t st) {
         std::vector<int> rp2, cl2;

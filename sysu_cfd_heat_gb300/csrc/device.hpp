@@ -33,9 +33,9 @@ class DevBuf {
     explicit DevBuf(size_t n) { alloc(n); }
     DevBuf(const DevBuf &) = delete;
     DevBuf &operator=(const DevBuf &) = delete;
-    DevBuf(DevBuf &&o) noexcept : p_(o.p_), n_(o.n_) { o.p_ = nullptr; o.n_ = 0; }
+    DevBuf(DevBuf &&o) noexcept : p_(o.p_), n_(o.n_), owned_(o.owned_) { o.p_ = nullptr; o.n_ = 0; }
     DevBuf &operator=(DevBuf &&o) noexcept {
-        if (this != &o) { release(); p_ = o.p_; n_ = o.n_; o.p_ = nullptr; o.n_ = 0; }
+        if (this != &o) { release(); p_ = o.p_; n_ = o.n_; owned_ = o.owned_; o.p_ = nullptr; o.n_ = 0; }
         return *this;
     }
     ~DevBuf() { release(); }
@@ -44,10 +44,18 @@ class DevBuf {
         n_ = n;
         if (n) SYSU_CUDA(cudaMalloc((void **)&p_, n * sizeof(T)));
     }
+    // n values of another buffer, which outlives this one
+    void view(T *p, size_t n) {
+        release();
+        p_ = p;
+        n_ = n;
+        owned_ = false;
+    }
     void release() {
-        if (p_) cudaFree(p_);
+        if (p_ && owned_) cudaFree(p_);
         p_ = nullptr;
         n_ = 0;
+        owned_ = true;
     }
     void upload(const T *h, size_t n, cudaStream_t s) {
         if (n > n_) throw CaseError{"upload larger than buffer"};
@@ -70,6 +78,7 @@ class DevBuf {
   private:
     T *p_ = nullptr;
     size_t n_ = 0;
+    bool owned_ = true;
 };
 
 // Grid barrier state for persistent (cooperatively launched) kernels.

@@ -981,16 +981,21 @@ __global__ void __launch_bounds__(BICG_NT, 1) k_bicgstab_mixed(BicgMixedArgs a, 
 
 void KrylovWork::ensure(int n_, int nrhs_, int max_blocks_, cudaStream_t st) {
     if (n_ <= n && nrhs_ <= nrhs && max_blocks_ <= max_blocks) return;
-    n = std::max(n, n_);
-    nrhs = std::max(nrhs, nrhs_);
-    max_blocks = std::max(max_blocks, max_blocks_);
-    size_t m = (size_t)n * nrhs;
-    r.alloc(m); rt.alloc(m); p.alloc(m); v.alloc(m); s.alloc(m); t.alloc(m);
-    dinv.alloc(m);
-    partials.alloc((size_t)8 * NVMAX * max_blocks);  // also 2 x 9 sums, and the 4-word exact-sum partials
+    const int n1 = std::max(n, n_), nrhs1 = std::max(nrhs, nrhs_), blocks1 = std::max(max_blocks, max_blocks_);
+    const size_t m = (size_t)n1 * nrhs1;
+    n = nrhs = max_blocks = 0;  // until everything is there
+    // one allocation for the vectors (a cudaMalloc and cudaFree of half a megabyte are 25 us)
+    const size_t pad = (m + 31) / 32 * 32, np = (size_t)8 * NVMAX * blocks1;
+    DevBuf<double> *const vec[] = {&r, &rt, &p, &v, &s, &t, &dinv};
+    slab.alloc(7 * pad + np);
+    for (int k = 0; k < 7; ++k) vec[k]->view(slab.get() + k * pad, m);
+    partials.view(slab.get() + 7 * pad, np);  // also 2 x 9 sums, and the 4-word exact-sum partials
     barrier.alloc(1);
     barrier.zero(st);
     slots.alloc(AX_WORDS);
+    n = n1;
+    nrhs = nrhs1;
+    max_blocks = blocks1;
 }
 
 unsigned long long *KrylovWork::clear_slots(cudaStream_t st) {

@@ -73,6 +73,7 @@ struct SolveInfo {
 // Scratch of the persistent solvers, sized for n rows and up to 3 RHS.
 struct KrylovWork {
     int n = 0, nrhs = 0, max_blocks = 0;
+    DevBuf<double> slab;  // r .. partials are views of it
     DevBuf<double> r, rt, p, v, s, t, dinv, partials;
     DevBuf<double> sval;  // BiCGSTAB: matrix values scaled by the Jacobi diagonal inverse of their column
     DevBuf<float> r32, z32, p32, q32, e32, dinv32;  // mixed-precision inner solve
