@@ -46,6 +46,7 @@ constexpr int NA_NT = 512;                 // threads of a solver CTA
 constexpr int NA_ROWS = 4;                 // rows a thread at most
 constexpr unsigned NA_SMEM = 200 * 1024;   // matrix entries a CTA keeps in shared memory
 constexpr int NA_ENTRIES = NA_SMEM / 12;
+constexpr int NA_CL_ROWS = 16 * NA_NT;     // up to here one cluster of at most 16 CTAs solves the system
 
 // what a malformed CSR row was found to hold (low two bits of NaHeader::bad)
 enum NaBad : int { NA_BAD_NONE = 0, NA_BAD_ROWPTR = 1, NA_BAD_COL = 2, NA_BAD_DIAG = 3 };
@@ -124,8 +125,10 @@ __global__ void k_na_dinv(NaArgs a) {
 // other CTAs gather, is the only vector in memory.  Latency bounds it at every size up to the
 // limit: two sums (grid_all.cuh) and two FP64 divisions an iteration.  1,716 rows on 7 blocks
 // of 256 threads, with three barriers and FP64 shuffle trees, square roots and divisions in
-// every thread, took 13.7 us an iteration; on 54 CTAs here 6.7 (238,080 rows: 13.0).
-template <int R>
+// every thread, took 13.7 us an iteration; on 54 CTAs here 6.9 (238,080 rows: 13.0).
+// CL: the grid is one cluster.  z lies in its CTAs' shared memory, the columns there are turned
+// into shared addresses of the cluster, and the sums meet at the cluster's barrier: 5.3.
+template <int R, bool CL>
 __global__ void __launch_bounds__(NA_NT, 1) k_na_cg(NaArgs a) {
     NaHeader *h = reinterpret_cast<NaHeader *>(a.base);
     double *zg = a.base + NA_HDR;
@@ -139,29 +142,47 @@ __global__ void __launch_bounds__(NA_NT, 1) k_na_cg(NaArgs a) {
     const int R0 = 32 * (int)((long long)groups * blockIdx.x / gridDim.x);
     const int R1 = min(n, 32 * (int)((long long)groups * (blockIdx.x + 1) / gridDim.x));
     sysu::AllCtx c = sysu::all_ctx(reinterpret_cast<unsigned long long *>(a.base + NA_SLOTS));
-    sysu::all_init();
+    sysu::ClCtx cl = sysu::cl_ctx();
+    if (CL) sysu::cl_sync();  // every block has started before its shared memory is written to
+    else sysu::all_init();
+    auto sum = [&](auto &v, int ch, auto fin) {
+        if (!CL) return sysu::all_sum(v, ch, c, &h->err, fin);
+        sysu::cl_sum(v, cl, fin);
+        return true;
+    };
+    const int NT = CL ? (int)blockDim.x : NA_NT;
     extern __shared__ __align__(16) unsigned char na_smem[];
+    // CL: this block's z, and where the cluster keeps row j's
+    __shared__ double zs[CL ? R * NA_NT : 1];
+    auto at = [&](int j) {
+        const int g = j >> 5, G = (int)gridDim.x;
+        int o = (int)(((long long)(g + 1) * G - 1) / groups);
+        return sysu::cl_addr(zs + (j - 32 * (int)((long long)groups * o / G)), o);
+    };
     const int E0 = a.rowptr[R0], nent = a.rowptr[R1] - E0;
     const bool res = nent <= NA_ENTRIES;
     double *sval = reinterpret_cast<double *>(na_smem);
     int *scol = reinterpret_cast<int *>(sval + (res ? nent : 0));
     if (res) {
-        for (int k = tid; k < nent; k += NA_NT) {
+        for (int k = tid; k < nent; k += NT) {
             sval[k] = a.val[E0 + k];
-            scol[k] = a.col[E0 + k];
+            scol[k] = CL ? (int)at(a.col[E0 + k]) : a.col[E0 + k];
         }
     }
     const double *mv = res ? sval : a.val + E0;
     const int *mc = res ? scol : a.col + E0;
+    auto zat = [&](int e) {
+        if (!CL) return zg[mc[e]];
+        return sysu::cl_load(res ? (unsigned)mc[e] : at(mc[e]));
+    };
     __shared__ double s_rr, s_rho, s_thr, s_bb, s_alpha, s_beta;
     __shared__ int s_brk;
-    int *err = &h->err;
     double x[R], r[R], p[R], q[R], d[R];
     int e0[R], len[R];
     double v3[3] = {0.0, 0.0, 0.0};
 #pragma unroll
     for (int u = 0; u < R; ++u) {
-        const int i = R0 + tid + u * NA_NT;
+        const int i = R0 + tid + u * NT;
         x[u] = r[u] = p[u] = q[u] = d[u] = 0.0;
         e0[u] = len[u] = 0;
         if (i >= R1) continue;
@@ -175,12 +196,13 @@ __global__ void __launch_bounds__(NA_NT, 1) k_na_cg(NaArgs a) {
         d[u] = dinv[i];
         r[u] = bi - s;
         const double z = d[u] * r[u];
-        zg[i] = z;
+        if (CL) zs[i - R0] = z;
+        else zg[i] = z;
         v3[0] = fma(bi, bi, v3[0]);
         v3[1] = fma(r[u], r[u], v3[1]);
         v3[2] = fma(r[u], z, v3[2]);
     }
-    if (!sysu::all_sum<3>(v3, 0, c, err, [&](int k, double s) {
+    if (!sum(v3, 0, [&](int k, double s) {
             if (k == 0) {
                 s_bb = s == 0.0 ? 1.0 : s;
                 s_thr = a.eps * a.eps * s_bb;
@@ -204,18 +226,18 @@ __global__ void __launch_bounds__(NA_NT, 1) k_na_cg(NaArgs a) {
             int k = 0;
             for (; k + 4 <= len[u]; k += 4) {  // four entries' loads before their FMAs
                 const int e = e0[u] + k;
-                const double g0 = zg[mc[e]], g1 = zg[mc[e + 1]], g2 = zg[mc[e + 2]], g3 = zg[mc[e + 3]];
+                const double g0 = zat(e), g1 = zat(e + 1), g2 = zat(e + 2), g3 = zat(e + 3);
                 w = fma(mv[e], g0, w);
                 w = fma(mv[e + 1], g1, w);
                 w = fma(mv[e + 2], g2, w);
                 w = fma(mv[e + 3], g3, w);
             }
-            for (; k < len[u]; ++k) w = fma(mv[e0[u] + k], zg[mc[e0[u] + k]], w);
+            for (; k < len[u]; ++k) w = fma(mv[e0[u] + k], zat(e0[u] + k), w);
             p[u] = fma(beta, p[u], d[u] * r[u]);
             q[u] = fma(beta, q[u], w);
             v1[0] = fma(p[u], q[u], v1[0]);
         }
-        if (!sysu::all_sum<1>(v1, 3, c, err, [&](int, double pq) {
+        if (!sum(v1, 3, [&](int, double pq) {
                 s_brk = pq == 0.0;
                 s_alpha = pq == 0.0 ? 0.0 : s_rho / pq;
             })) return;
@@ -224,16 +246,17 @@ __global__ void __launch_bounds__(NA_NT, 1) k_na_cg(NaArgs a) {
         double v2[2] = {0.0, 0.0};
 #pragma unroll
         for (int u = 0; u < R; ++u) {
-            const int i = R0 + tid + u * NA_NT;
+            const int i = R0 + tid + u * NT;
             if (i >= R1) continue;
             x[u] = fma(alpha, p[u], x[u]);
             r[u] = fma(-alpha, q[u], r[u]);
             const double z = d[u] * r[u];
-            zg[i] = z;
+            if (CL) zs[i - R0] = z;
+            else zg[i] = z;
             v2[0] = fma(r[u], r[u], v2[0]);
             v2[1] = fma(r[u], z, v2[1]);
         }
-        if (!sysu::all_sum<2>(v2, 4, c, err, [&](int k, double s) {
+        if (!sum(v2, 4, [&](int k, double s) {
                 if (k == 0) {
                     s_rr = s;
                 } else {
@@ -244,7 +267,7 @@ __global__ void __launch_bounds__(NA_NT, 1) k_na_cg(NaArgs a) {
     }
 #pragma unroll
     for (int u = 0; u < R; ++u) {
-        const int i = R0 + tid + u * NA_NT;
+        const int i = R0 + tid + u * NT;
         if (i < R1) a.x[i] = x[u];
     }
     if (blockIdx.x == 0 && tid == 0) {
@@ -257,7 +280,8 @@ __global__ void __launch_bounds__(NA_NT, 1) k_na_cg(NaArgs a) {
 
 thread_local std::string g_na_err;
 std::mutex g_na_mu;
-int g_na_blocks[64] = {0};  // SMs of a device, 0: not asked yet
+int g_na_blocks[64] = {0};   // SMs of a device, 0: not asked yet
+int g_na_cluster[64] = {0};  // CTAs of its largest cluster of the solver
 
 int na_fail(int code, const std::string &m) {
     g_na_err = m;
@@ -298,19 +322,40 @@ int sysu_csr_cg_noalloc(int n, const int *d_rowptr, const int *d_col, const doub
         std::lock_guard<std::mutex> lock(g_na_mu);
         if (!g_na_blocks[dev]) {  // once per device: cooperative-launch occupancy
             int per_sm = 0, sms = 0, coop = 0;
-            const void *kernels[] = {(const void *)k_na_cg<1>, (const void *)k_na_cg<2>, (const void *)k_na_cg<NA_ROWS>};
+            const void *kernels[] = {(const void *)k_na_cg<1, false>, (const void *)k_na_cg<2, false>,
+                                     (const void *)k_na_cg<NA_ROWS, false>};
             for (const void *k : kernels) {
                 if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)NA_SMEM);
                 int ps = 0;
                 if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ps, k, NA_NT, NA_SMEM);
                 per_sm = k == kernels[0] || ps < per_sm ? ps : per_sm;
             }
+            const void *clk = (const void *)k_na_cg<1, true>;
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(clk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)NA_SMEM);
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(clk, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
             if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
             if (e == cudaSuccess) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
             if (e != cudaSuccess) return na_fail(SYSU_ERR_CUDA, std::string("device query: ") + cudaGetErrorString(e));
             if (!coop || per_sm < 1) return na_fail(SYSU_ERR_CUDA, "cooperative launch unavailable");
             if ((long long)sms * NA_NT * NA_ROWS < NA_MAX_ROWS)
                 return na_fail(SYSU_ERR_CUDA, "the device has too few SMs for the solver");
+            // the largest cluster the device takes, 0: none
+            for (int cs = sysu::CL_MAX; cs >= 1 && !g_na_cluster[dev]; cs /= 2) {
+                cudaLaunchAttribute at{};
+                at.id = cudaLaunchAttributeClusterDimension;
+                at.val.clusterDim.x = (unsigned)cs;
+                at.val.clusterDim.y = at.val.clusterDim.z = 1;
+                cudaLaunchConfig_t lc{};
+                lc.gridDim = dim3(cs);
+                lc.blockDim = dim3(NA_NT);
+                lc.dynamicSmemBytes = NA_SMEM;
+                lc.attrs = &at;
+                lc.numAttrs = 1;
+                int fit = 0;
+                if (cudaOccupancyMaxActiveClusters(&fit, k_na_cg<1, true>, &lc) == cudaSuccess && fit > 0)
+                    g_na_cluster[dev] = cs;
+            }
+            (void)cudaGetLastError();
             g_na_blocks[dev] = sms < sysu::AX_MAX_BLOCKS ? sms : sysu::AX_MAX_BLOCKS;
         }
         blocks = g_na_blocks[dev];
@@ -318,6 +363,18 @@ int sysu_csr_cg_noalloc(int n, const int *d_rowptr, const int *d_col, const doub
     const int groups = (n + 31) / 32;
     const int G = groups < blocks ? groups : blocks;
     const int need = (32 * ((groups + G - 1) / G) + NA_NT - 1) / NA_NT;  // rows a thread
+    // One cluster where a thread a row suffices: CTAs of 128 rows, one warp a scheduler, up to 16
+    // of them, then more rows each.  Cluster against whole GPU, us an iteration: 512 rows 5.0 and
+    // 7.2, 1,716 rows 5.3 and 6.9, 4,096 rows 5.6 and 6.9, 8,000 rows 6.7 and 6.9; with two rows a
+    // thread (13,824 rows) 8.5 and 6.8.
+    int cluster = 0;
+    if (n <= NA_CL_ROWS && g_na_cluster[dev] > 0) {
+        cluster = 1;
+        while (cluster < g_na_cluster[dev] && 4 * cluster < groups) cluster *= 2;
+    }
+    const int rows = cluster ? 32 * ((groups + cluster - 1) / cluster) : 0;
+    if (rows > NA_NT) cluster = 0;
+    const int threads = rows < 128 ? 128 : rows;
     NaArgs a{n, d_rowptr, d_col, d_val, d_b, d_x, omega, maxit, eps, base};
     // what must start at zero: the exchange area of the grid sums and the status words;
     // the malformed-row key starts at all ones (no row found)
@@ -331,9 +388,24 @@ int sysu_csr_cg_noalloc(int n, const int *d_rowptr, const int *d_col, const doub
     e = cudaGetLastError();
     if (e != cudaSuccess) return na_fail(SYSU_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(e));
     void *args[] = {&a};
-    const void *kern = need <= 1 ? (const void *)k_na_cg<1>
-                                 : need <= 2 ? (const void *)k_na_cg<2> : (const void *)k_na_cg<NA_ROWS>;
-    e = cudaLaunchCooperativeKernel(kern, dim3(G), dim3(NA_NT), args, NA_SMEM, st);
+    const void *kern = need <= 1 ? (const void *)k_na_cg<1, false>
+                                 : need <= 2 ? (const void *)k_na_cg<2, false> : (const void *)k_na_cg<NA_ROWS, false>;
+    if (cluster) {
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = (unsigned)cluster;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cudaLaunchConfig_t lc{};
+        lc.gridDim = dim3(cluster);
+        lc.blockDim = dim3(threads);
+        lc.dynamicSmemBytes = NA_SMEM;
+        lc.stream = st;
+        lc.attrs = &at;
+        lc.numAttrs = 1;
+        e = cudaLaunchKernelEx(&lc, k_na_cg<1, true>, a);
+    } else {
+        e = cudaLaunchCooperativeKernel(kern, dim3(G), dim3(NA_NT), args, NA_SMEM, st);
+    }
     if (e != cudaSuccess) return na_fail(SYSU_ERR_CUDA, std::string("cooperative launch: ") + cudaGetErrorString(e));
     NaHeader h;
     e = cudaMemcpyAsync(&h, base, sizeof(NaHeader), cudaMemcpyDeviceToHost, st);
