@@ -13,7 +13,7 @@
 // and reported figures as k_cg_pipe / k_cg_mixed_pipe.
 //
 // Measured, us per iteration, streaming kernels before -> here: 13,824 rows of a hex mesh in
-// FP64 13.2 -> 6.6 (two sums of 2.2 us, the FP64 latencies of a row and of alpha and beta),
+// FP64 13.2 -> 6.6 (two sums of 2 us, the FP64 latencies of a row and of alpha),
 // 51,200 rows 13.8 -> 7.7, 256,000 rows 19.3 -> 13.2 (5.7 us of it FP64 pipe); 262,144 rows in
 // FP32 16.2 -> 8.2.  The line to the streaming kernels is the shared memory: there is no size
 // that fits and was faster streamed.
@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(CR_NT, 1) k_cg_res(CgResArgs a, int wmax) {
     }
     if (!all_sum<3>(v3, CH_INIT, c, err)) return;
     // thread-0 scalar state in shared memory
-    __shared__ double s_bb, s_rr, s_rho, s_thr, s_unit;
+    __shared__ double s_bb, s_rr, s_rho, s_thr, s_unit, s_inv;
     __shared__ int s_bias, s_rr_est;
     if (tid == 0) {
         s_bb = g_ax_sum[0] == 0.0 ? 1.0 : g_ax_sum[0];
@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(CR_NT, 1) k_cg_res(CgResArgs a, int wmax) {
         if (!all_sum<1>(v1, CH_PQ, c, err, [&](int, double pq) {
                 g_bc[2] = pq == 0.0 ? 0.0 : s_rho / pq;
                 g_bc[3] = pq == 0.0 ? 1.0 : 0.0;
-            })) { ok = false; break; }
+            }, [&] { s_inv = 1.0 / s_rho; })) { ok = false; break; }
         stamp(a.ts, it, 1);
         if (g_bc[3] != 0.0) { status = DEV_BREAKDOWN; break; }
         const double alpha = g_bc[2];
@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(CR_NT, 1) k_cg_res(CgResArgs a, int wmax) {
         if (bias) v2[0] = (double)rr32;
         if (!all_sum<2>(v2, CH_RZ, c, err, [&](int k, double sum) {
                 if (k == 1) {
-                    g_bc[1] = sum / s_rho;
+                    g_bc[1] = sum * s_inv;
                     s_rho = sum;
                 } else if (bias) {
                     // the estimate decides only when it is clearly above the threshold
@@ -278,7 +278,7 @@ __global__ void __launch_bounds__(CR_NT, 1) k_cg_mixed_res(CgResArgs a, int wmax
     int wd[R];
     res_load<float, R>(M, a.A, a.val32, R0, nrow, wd);
     float r[R], p[R], q[R], e[R], d[R];
-    __shared__ double s_bb, s_thr, s_rho, s_rz, s_rr, s_sig, s_sig_next;
+    __shared__ double s_bb, s_thr, s_rho, s_rz, s_rr, s_sig, s_sig_next, s_inv;
     __shared__ int s_stalls;
     {
         double r64[R], v2[2] = {0.0, 0.0};
@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(CR_NT, 1) k_cg_mixed_res(CgResArgs a, int wmax
         if (!all_sum<1>(v1, CH_PQ, c, err, [&](int, double pq) {
                 g_bc[2] = pq == 0.0 ? 0.0 : s_rho / pq;
                 g_bc[3] = pq == 0.0 ? 1.0 : 0.0;
-            })) return;
+            }, [&] { s_inv = 1.0 / s_rho; })) return;
         stamp(a.ts, total, 1);
         if (g_bc[3] != 0.0) { status = DEV_BREAKDOWN; break; }
         const float alpha = (float)g_bc[2];
@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(CR_NT, 1) k_cg_mixed_res(CgResArgs a, int wmax
         double w2[2] = {(double)h0, (double)h1};
         if (!all_sum<2>(w2, CH_RZ, c, err, [&](int k, double sum) {
                 if (k == 1) {
-                    g_bc[1] = sum / s_rho;  // the next beta, unless an update replaces r
+                    g_bc[1] = sum * s_inv;  // the next beta, unless an update replaces r
                     s_rz = sum;
                 } else {
                     // reliable update: as k_cg_mixed_pipe (the FP32 sums are in sig^2 units)

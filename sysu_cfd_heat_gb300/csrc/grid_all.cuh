@@ -355,10 +355,16 @@ __device__ __forceinline__ AxNum ax_block(int k, int &nf) {
 // Exact sums of NV values per thread over the grid, and a barrier: what any thread wrote
 // before the call, every thread may read after it.  Value k is combined by warp k, whose
 // lane 0 calls fin(k, sum) before the block goes on (what it writes to shared memory, every
-// thread may read after the call); the last warp orders the block's data: the block needs
+// thread may read after the call); idle() runs meanwhile in a thread with nothing to do (a
+// division that the next step needs); the last warp orders the block's data: the block needs
 // NV + 1 warps.  ch: the first of the NV channels of this place in the code.
-template <int NV, class Fin>
-__device__ __forceinline__ bool all_sum(const double (&v)[NV], int ch, AllCtx &c, int *err, Fin &&fin) {
+struct AxNone {
+    __device__ void operator()() const {}
+};
+
+template <int NV, class Fin, class Idle = AxNone>
+__device__ __forceinline__ bool all_sum(const double (&v)[NV], int ch, AllCtx &c, int *err, Fin &&fin,
+                                        Idle &&idle = Idle()) {
     static_assert(NV <= AX_NVMAX, "all_sum: too many values");
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     ax_warps<NV>(v);
@@ -378,6 +384,8 @@ __device__ __forceinline__ bool all_sum(const double (&v)[NV], int ch, AllCtx &c
         const AxNum a = ax_block(warp, f);
         const double s = ax_grid(a, f, warp, ch + warp, c, err);
         if (lane == 0) fin(warp, s);
+    } else if (warp == NV && lane == 0) {
+        idle();
     }
     __syncthreads();
     return *reinterpret_cast<volatile int *>(&g_ax_bad) == 0;
@@ -432,11 +440,21 @@ __device__ __forceinline__ void cl_store(unsigned a, int x, int y, int z, int w)
     asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w)
                  : "memory");
 }
-// Barrier of the cluster's threads: what any of them wrote before, all may read after.
+// Barrier of the cluster's threads: what any of them wrote before, all may read after, and
+// what idle() writes to shared memory, the block's threads (by a barrier of their own).
 __device__ __forceinline__ void cl_sync() {
     __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+template <class Idle>
+__device__ __forceinline__ void cl_sync(Idle &&idle) {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    if (threadIdx.x == 32) idle();
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    __syncthreads();
 }
 
 // all_sum over the cluster; at least NV warps a block.
@@ -472,6 +490,27 @@ __device__ __forceinline__ void cl_sum(const double (&v)[NV], ClCtx &c, Fin &&fi
     }
     c.parity ^= 1;
     __syncthreads();
+}
+
+// ---- CG with one sum an iteration ----------------------------------------------
+// Chronopoulos and Gear's form of CG's two scalars: with w = A z, gamma = r.z, delta = w.z,
+//     beta = gamma / gamma_old,   alpha = gamma / (delta - beta gamma / alpha_old)
+// (p.q in the denominator: r is orthogonal to the old z), so both sums and the residual's are
+// taken at once and an iteration has one sum and one bare barrier.  The quotients that only
+// the next iteration needs are formed by an idle thread during the barrier.
+struct CgScalars {
+    double gamma, delta, beta, alpha, den;
+    double inv_gamma, inv_alpha;  // of the iteration before; 0 in the first
+};
+
+__device__ __forceinline__ void cg_scalars(CgScalars &S) {
+    S.beta = S.gamma * S.inv_gamma;
+    S.den = fma(-(S.beta * S.inv_alpha), S.gamma, S.delta);
+    S.alpha = S.den == 0.0 ? 0.0 : S.gamma / S.den;
+}
+__device__ __forceinline__ void cg_next(CgScalars &S) {
+    S.inv_gamma = 1.0 / S.gamma;
+    S.inv_alpha = S.den * S.inv_gamma;
 }
 
 }  // namespace

@@ -127,7 +127,10 @@ __global__ void k_na_dinv(NaArgs a) {
 // of 256 threads, with three barriers and FP64 shuffle trees, square roots and divisions in
 // every thread, took 13.7 us an iteration; on 54 CTAs here 6.9 (238,080 rows: 13.0).
 // CL: the grid is one cluster.  z lies in its CTAs' shared memory, the columns there are turned
-// into shared addresses of the cluster, and the sums meet at the cluster's barrier: 5.3.
+// into shared addresses of the cluster, and the sums meet at the cluster's barrier: 5.3 us with
+// the two sums, 4.6 with one (CgScalars) and a barrier.  Over the whole GPU that form is not
+// faster (6.9 either way at 32,768 rows, 7.5 against 7.2 at 60,680): three values at once and a
+// bare barrier take as long as the two sums.
 template <int R, bool CL>
 __global__ void __launch_bounds__(NA_NT, 1) k_na_cg(NaArgs a) {
     NaHeader *h = reinterpret_cast<NaHeader *>(a.base);
@@ -175,7 +178,8 @@ __global__ void __launch_bounds__(NA_NT, 1) k_na_cg(NaArgs a) {
         if (!CL) return zg[mc[e]];
         return sysu::cl_load(res ? (unsigned)mc[e] : at(mc[e]));
     };
-    __shared__ double s_rr, s_rho, s_thr, s_bb, s_alpha, s_beta;
+    __shared__ double s_rr, s_rho, s_thr, s_bb, s_alpha, s_beta, s_inv;
+    __shared__ sysu::CgScalars S;
     __shared__ int s_brk;
     double x[R], r[R], p[R], q[R], d[R];
     int e0[R], len[R];
@@ -211,10 +215,61 @@ __global__ void __launch_bounds__(NA_NT, 1) k_na_cg(NaArgs a) {
             } else {
                 s_rho = s;
                 s_beta = 0.0;
+                S.inv_gamma = S.inv_alpha = 0.0;
             }
         })) return;
+    auto product = [&](int u) {  // row u of A z
+        double w = 0.0;
+        int k = 0;
+        for (; k + 4 <= len[u]; k += 4) {  // four entries' loads before their FMAs
+            const int e = e0[u] + k;
+            const double g0 = zat(e), g1 = zat(e + 1), g2 = zat(e + 2), g3 = zat(e + 3);
+            w = fma(mv[e], g0, w);
+            w = fma(mv[e + 1], g1, w);
+            w = fma(mv[e + 2], g2, w);
+            w = fma(mv[e + 3], g3, w);
+        }
+        for (; k < len[u]; ++k) w = fma(mv[e0[u] + k], zat(e0[u] + k), w);
+        return w;
+    };
     int it = 0, status = sysu::DEV_OK;
-    while (!(s_rr < s_thr) && it < a.maxit) {
+    while (CL) {  // one sum and one barrier an iteration
+        double w[R], v[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+        for (int u = 0; u < R; ++u) {
+            w[u] = 0.0;
+            if (len[u] == 0) continue;
+            w[u] = product(u);
+            const double z = d[u] * r[u];
+            v[0] = fma(r[u], r[u], v[0]);
+            v[1] = fma(r[u], z, v[1]);
+            v[2] = fma(w[u], z, v[2]);
+        }
+        sysu::cl_sum(v, cl, [&](int k, double s) {
+            if (k == 0) s_rr = s;
+            else if (k == 1) S.gamma = s;
+            else S.delta = s;
+        });
+        if (s_rr < s_thr || it >= a.maxit) break;
+        if (!isfinite(s_rr)) { status = sysu::DEV_NONFINITE; break; }
+        ++it;
+        if (tid == 0) sysu::cg_scalars(S);
+        __syncthreads();
+        if (S.den == 0.0) { status = sysu::DEV_BREAKDOWN; break; }
+        const double alpha = S.alpha, beta = S.beta;
+#pragma unroll
+        for (int u = 0; u < R; ++u) {
+            const int i = R0 + tid + u * NT;
+            if (i >= R1) continue;
+            p[u] = fma(beta, p[u], d[u] * r[u]);
+            q[u] = fma(beta, q[u], w[u]);
+            x[u] = fma(alpha, p[u], x[u]);
+            r[u] = fma(-alpha, q[u], r[u]);
+            zs[i - R0] = d[u] * r[u];
+        }
+        sysu::cl_sync([&] { sysu::cg_next(S); });
+    }
+    while (!CL && !(s_rr < s_thr) && it < a.maxit) {
         if (!isfinite(s_rr)) { status = sysu::DEV_NONFINITE; break; }
         ++it;
         const double beta = s_beta;
@@ -222,25 +277,15 @@ __global__ void __launch_bounds__(NA_NT, 1) k_na_cg(NaArgs a) {
 #pragma unroll
         for (int u = 0; u < R; ++u) {
             if (len[u] == 0) continue;
-            double w = 0.0;
-            int k = 0;
-            for (; k + 4 <= len[u]; k += 4) {  // four entries' loads before their FMAs
-                const int e = e0[u] + k;
-                const double g0 = zat(e), g1 = zat(e + 1), g2 = zat(e + 2), g3 = zat(e + 3);
-                w = fma(mv[e], g0, w);
-                w = fma(mv[e + 1], g1, w);
-                w = fma(mv[e + 2], g2, w);
-                w = fma(mv[e + 3], g3, w);
-            }
-            for (; k < len[u]; ++k) w = fma(mv[e0[u] + k], zat(e0[u] + k), w);
+            const double w = product(u);
             p[u] = fma(beta, p[u], d[u] * r[u]);
             q[u] = fma(beta, q[u], w);
             v1[0] = fma(p[u], q[u], v1[0]);
         }
-        if (!sum(v1, 3, [&](int, double pq) {
+        if (!sysu::all_sum(v1, 3, c, &h->err, [&](int, double pq) {
                 s_brk = pq == 0.0;
                 s_alpha = pq == 0.0 ? 0.0 : s_rho / pq;
-            })) return;
+            }, [&] { s_inv = 1.0 / s_rho; })) return;
         if (s_brk) { status = sysu::DEV_BREAKDOWN; break; }
         const double alpha = s_alpha;
         double v2[2] = {0.0, 0.0};
@@ -251,16 +296,15 @@ __global__ void __launch_bounds__(NA_NT, 1) k_na_cg(NaArgs a) {
             x[u] = fma(alpha, p[u], x[u]);
             r[u] = fma(-alpha, q[u], r[u]);
             const double z = d[u] * r[u];
-            if (CL) zs[i - R0] = z;
-            else zg[i] = z;
+            zg[i] = z;
             v2[0] = fma(r[u], r[u], v2[0]);
             v2[1] = fma(r[u], z, v2[1]);
         }
-        if (!sum(v2, 4, [&](int k, double s) {
+        if (!sysu::all_sum(v2, 4, c, &h->err, [&](int k, double s) {
                 if (k == 0) {
                     s_rr = s;
                 } else {
-                    s_beta = s / s_rho;
+                    s_beta = s * s_inv;
                     s_rho = s;
                 }
             })) return;
@@ -364,9 +408,9 @@ int sysu_csr_cg_noalloc(int n, const int *d_rowptr, const int *d_col, const doub
     const int G = groups < blocks ? groups : blocks;
     const int need = (32 * ((groups + G - 1) / G) + NA_NT - 1) / NA_NT;  // rows a thread
     // One cluster where a thread a row suffices: CTAs of 128 rows, one warp a scheduler, up to 16
-    // of them, then more rows each.  Cluster against whole GPU, us an iteration: 512 rows 5.0 and
-    // 7.2, 1,716 rows 5.3 and 6.9, 4,096 rows 5.6 and 6.9, 8,000 rows 6.7 and 6.9; with two rows a
-    // thread (13,824 rows) 8.5 and 6.8.
+    // of them, then more rows each.  Cluster against whole GPU, us an iteration: 512 rows 4.6 and
+    // 7.2, 1,716 rows 4.6 and 6.9, 4,096 rows 5.0 and 6.9, 8,000 rows 6.3 and 6.9; with two rows a
+    // thread and two sums (13,824 rows) 8.5 and 6.8.
     int cluster = 0;
     if (n <= NA_CL_ROWS && g_na_cluster[dev] > 0) {
         cluster = 1;
