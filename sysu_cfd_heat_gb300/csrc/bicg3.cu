@@ -206,8 +206,8 @@ __global__ void __launch_bounds__(MB) k_m3_init(M3Args a, int maxit, double eps,
 // FP64 residual replacement for the components that need it: r_c = sig (b - A x)
 // with the scale chosen from the FP32 residual that triggered it; rt_c = r_c
 // when the component restarts.  first: the set-up pass (the residual of x0 from
-// r0, no stall bookkeeping).
-__global__ void __launch_bounds__(MB) k_m3_replace(M3Args a, int first) {
+// r0, no stall bookkeeping).  Five blocks an SM: the grid decides which rows a thread sums.
+__global__ void __launch_bounds__(MB, 5) k_m3_replace(M3Args a, int first) {
     const M3State *S = a.st;
     if (S->all_done || !S->any_need) return;
     bool want[3], rs[3];

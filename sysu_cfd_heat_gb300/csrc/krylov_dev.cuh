@@ -328,18 +328,12 @@ __device__ __forceinline__ int deal_lane(int k, int o = 16) {
 // the block and grid sums.  An FP64 shuffle tree in every thread runs on GB300's FP64 pipe
 // (1/64 of the FP32 rate): 6 FP64 operations per value and thread took 10-20 us of a 2M-row
 // vector pass.  What is left is the tail after the last block's arrival, a chain of FP64
-// additions of 65 clocks each: values side by side in groups of 8 lanes or dealt over the
-// lanes, not one after the other in one thread, and callers work their scalars out with a
-// thread a component.  On 262,144 rows k_m3_upd (six sums, three components' scalars) went
+// additions of 65 clocks each: values side by side, a lane each or dealt over the lanes, not
+// one after the other in one thread, and callers work their scalars out with a thread a
+// component.  The order of each value's additions (warp butterflies, then the warps one after
+// the other) is part of the results: BiCGSTAB amplifies a last bit to 1e-9 of the solution.  On 262,144 rows k_m3_upd (six sums, three components' scalars) went
 // from 21.8 to 12.8 us, k_m3_at from 17.0 to 11.4 and k_fcg_upd from 11.1 to 8.1.
 __shared__ double g_gt_warp[NVMAX * 8], g_gt_sum[NVMAX];
-
-// g_gt_warp[k * 8 + w], w < 8, summed over w by 8 lanes a value: to every lane of the group
-__device__ __forceinline__ double sum8(double v) {
-#pragma unroll
-    for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(FULL_MASK, v, o);
-    return v;
-}
 
 template <int NV>
 __device__ bool grid_totals_f(const float (&f)[NV], double *part, unsigned *cnt) {
@@ -354,9 +348,10 @@ __device__ bool grid_totals_f(const float (&f)[NV], double *part, unsigned *cnt)
         if (lane == 0) sm[k * 8 + warp] = g;
     }
     __syncthreads();
-    if (warp < (NV * 8 + 31) / 32) {
-        const double s = sum8(tid < NV * 8 && (tid & 7) < nw ? (double)sm[tid] : 0.0);
-        if (tid < NV * 8 && (tid & 7) == 0) part[(size_t)(tid >> 3) * G + blockIdx.x] = s;
+    if (tid < NV) {
+        double s = 0.0;
+        for (int w = 0; w < nw; ++w) s += (double)sm[tid * 8 + w];
+        part[(size_t)tid * G + blockIdx.x] = s;
     }
     __syncthreads();
     if (tid == 0) {
@@ -377,9 +372,10 @@ __device__ bool grid_totals_f(const float (&f)[NV], double *part, unsigned *cnt)
     for (int k = 0; k < NV; ++k)
         if (lane == deal_lane<NV>(k)) g_gt_warp[k * 8 + warp] = w;
     __syncthreads();
-    if (warp < (NV * 8 + 31) / 32) {
-        const double s = sum8(tid < NV * 8 && (tid & 7) < nw ? g_gt_warp[tid] : 0.0);
-        if (tid < NV * 8 && (tid & 7) == 0) g_gt_sum[tid >> 3] = s;
+    if (tid < NV) {
+        double s = 0.0;
+        for (int w = 0; w < nw; ++w) s += g_gt_warp[tid * 8 + w];
+        g_gt_sum[tid] = s;
     }
     if (tid == 0) *cnt = 0;
     __syncthreads();
