@@ -420,6 +420,8 @@ struct BicgArgs {
     // behind a mixed solve: run only if gate->status[0] is DEV_STALLED (one
     // system; the iterations of both are reported); null: always run
     const SolveInfo *gate;
+    int G;     // blocks of KB rows and sums (the grid, or dealt to the CTAs of the resident form)
+    int wmax;  // resident form: widest slice
 };
 
 // Scalar state of a BiCGSTAB solve, in shared memory.  One thread a component derives it
@@ -431,10 +433,12 @@ struct BicgState {
     double bb[3], rr[3], thr[3], rho[3], rho_prev[3], alpha[3], omg[3], beta[3];
     int it[3], status[3], done[3], act[3], early[3];
 };
-__shared__ double g_bicg_smem[9 * (KB / 32)], g_bicg_sum[9];
+constexpr int BICG_RES_NT = 2 * KB;  // threads of the resident form's CTA at most
+__shared__ double g_bicg_smem[9 * (BICG_RES_NT / 32)], g_bicg_sum[9];
 
-// Grid sums of NV values, to g_bicg_sum for the whole block, in the order of block_sum_t0
-// (warp butterfly, warps) and warp_sum_partials; value k by thread k, then by a warp.
+// Grid sums of NV values, to g_bicg_sum for the whole CTA, in the order of block_sum_t0
+// (warp butterfly, warps) and warp_sum_partials; a CTA holds one or several blocks of KB
+// threads, every gridDim.x-th of the rc.G.
 template <int NV>
 __device__ __forceinline__ bool bicg_sum(const double (&v)[NV], RedCtx &rc, GridBarrier *gb, int *err) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -442,23 +446,78 @@ __device__ __forceinline__ bool bicg_sum(const double (&v)[NV], RedCtx &rc, Grid
     const double w = deal_sum<NV>(v, 16);
 #pragma unroll
     for (int k = 0; k < NV; ++k)
-        if (lane == deal_lane<NV>(k)) g_bicg_smem[k * NW + warp] = w;
+        if (lane == deal_lane<NV>(k)) g_bicg_smem[k * (BICG_RES_NT / 32) + warp] = w;
     __syncthreads();
     double *buf = rc.partials + (size_t)rc.parity * 9 * rc.G;
     rc.parity ^= 1;
-    if (threadIdx.x < NV) {
+    const int nh = blockDim.x / KB;
+    if ((int)threadIdx.x < NV * nh) {
+        const int k = (int)threadIdx.x / nh, h = (int)threadIdx.x % nh, blk = blockIdx.x + h * gridDim.x;
         double s = 0.0;
 #pragma unroll
-        for (int q = 0; q < NW; ++q) s += g_bicg_smem[threadIdx.x * NW + q];
-        buf[(size_t)threadIdx.x * rc.G + blockIdx.x] = s;
+        for (int q = 0; q < NW; ++q) s += g_bicg_smem[k * (BICG_RES_NT / 32) + h * NW + q];
+        if (blk < rc.G) buf[(size_t)k * rc.G + blk] = s;
     }
     if (!grid_sync(gb, err)) return false;
-    for (int k = warp; k < NV; k += NW) {
+    for (int k = warp; k < NV; k += (int)blockDim.x / 32) {
         const double s = warp_sum_partials(buf + (size_t)k * rc.G, rc.G);
         if (lane == 0) g_bicg_sum[k] = s;
     }
     __syncthreads();
     return true;
+}
+
+// The resident form's rows in shared memory: entry k of a thread's u-th row at
+// (u wmax + k) blockDim.x + threadIdx.x.
+struct BicgRows {
+    double *val;
+    int *col;
+    unsigned w;  // widths of the thread's rows, a byte each
+    BicgRows() = default;
+    __device__ __forceinline__ BicgRows(const BicgArgs &a, int t0, int T, unsigned char *smem) {
+        const int R = (a.A.n + T - 1) / T, NT = blockDim.x;
+        val = reinterpret_cast<double *>(smem);
+        col = reinterpret_cast<int *>(val + (size_t)R * a.wmax * NT);
+        w = 0;
+        for (int u = 0, i = t0; i < a.A.n; ++u, i += T) {
+            const int e = a.A.sl_ptr[i >> 5] + (i & 31), wu = a.A.sl_w[i >> 5];
+            w |= (unsigned)wu << (8 * u);
+            for (int k = 0; k < wu; ++k) {
+                val[(u * a.wmax + k) * NT + threadIdx.x] = a.svals[0][e + 32 * k];
+                col[(u * a.wmax + k) * NT + threadIdx.x] = a.A.col[e + 32 * k];
+            }
+        }
+    }
+};
+
+// row_dot_scaled from the rows in shared memory, the FMAs in entry order
+template <int NR>
+__device__ __forceinline__ void row_dot_resident(const BicgRows &M, int wmax, int u, const double *x, int n,
+                                                 const bool (&act)[3], double (&y)[NR]) {
+    constexpr int U = NR == 1 ? 4 : 2;
+    const int NT = blockDim.x, w = (int)(M.w >> (8 * u)) & 255;
+    int e = u * wmax * NT + (int)threadIdx.x;
+#pragma unroll
+    for (int c = 0; c < NR; ++c) y[c] = 0.0;
+    for (int k = 0; k < w; k += U, e += U * NT) {
+        double g[U][NR];
+#pragma unroll
+        for (int q = 0; q < U; ++q)
+            if (k + q < w) {
+                const int j = M.col[e + q * NT];
+#pragma unroll
+                for (int c = 0; c < NR; ++c)
+                    if (act[c]) g[q][c] = x[(size_t)c * n + j];
+            }
+#pragma unroll
+        for (int q = 0; q < U; ++q)
+            if (k + q < w) {
+                const double v = M.val[e + q * NT];
+#pragma unroll
+                for (int c = 0; c < NR; ++c)
+                    if (act[c]) y[c] = fma(v, g[q][c], y[c]);
+            }
+    }
 }
 
 // y_c = A (dinv .* x_c) for NR right-hand sides, skipping inactive ones, from the
@@ -507,16 +566,24 @@ __device__ __forceinline__ void row_dot_scaled(const SellView &A, const double *
 // 1e-8), so the order stays.  Bounded by the FP64 pipe at 2M rows and by the grid-wide steps
 // below 300k: three sums and two bare barriers an iteration -- s.s, which only decides the
 // early exit, is summed with t.s and t.t.
-template <int NR, bool MULTI>
-__global__ void __launch_bounds__(KB, 4) k_bicgstab(BicgArgs a) {
+//
+// RES: the column-scaled matrix stays in shared memory, up to two blocks of KB threads in a
+// CTA, one CTA an SM: fewer arrivals at a barrier and no trips to L2 for the matrix.  Rows and
+// sums are dealt to the same (virtual) threads and blocks as without, so the bits are the same.
+// BICG_US
+template <int NR, bool MULTI, bool RES>
+__global__ void __launch_bounds__(RES ? BICG_RES_NT : KB, RES ? 1 : 4) k_bicgstab(BicgArgs a) {
+    static_assert(!(MULTI && RES), "the resident form takes one matrix");
     if (a.gate && a.gate->status[0] != DEV_STALLED) return;  // the same word for every block
     const int it_before = a.gate ? a.gate->iters[0] : 0;
     const int n = a.A.n;
-    const int T = gridDim.x * KB;
-    const int t0 = blockIdx.x * KB + threadIdx.x;
     const int tid = threadIdx.x;
+    const int T = a.G * KB, blk = RES ? blockIdx.x + (tid / KB) * gridDim.x : blockIdx.x;
+    const int t0 = blk < a.G ? blk * KB + tid % KB : n;
     int *err = &a.info->err;
-    RedCtx rc{a.partials, (int)gridDim.x, 0};
+    RedCtx rc{a.partials, a.G, 0};
+    extern __shared__ __align__(16) unsigned char bicg_smem[];
+    BicgRows M = RES ? BicgRows(a, t0, T, bicg_smem) : BicgRows();
     const double *__restrict__ dinv = a.dinv;
     const size_t N = (size_t)n;
     __shared__ BicgState S;
@@ -596,9 +663,10 @@ __global__ void __launch_bounds__(KB, 4) k_bicgstab(BicgArgs a) {
             double red[NR];
 #pragma unroll
             for (int c = 0; c < NR; ++c) red[c] = 0.0;
-            for (int i = t0; i < n; i += T) {
+            for (int i = t0, u = 0; i < n; i += T, ++u) {
                 double y[NR];
-                row_dot_scaled<NR, MULTI>(a.A, a.svals, i, a.p, n, act, y);
+                if constexpr (RES) row_dot_resident<NR>(M, a.wmax, u, a.p, n, act, y);
+                else row_dot_scaled<NR, MULTI>(a.A, a.svals, i, a.p, n, act, y);
 #pragma unroll
                 for (int c = 0; c < NR; ++c) {
                     if (!act[c]) continue;
@@ -639,9 +707,10 @@ __global__ void __launch_bounds__(KB, 4) k_bicgstab(BicgArgs a) {
             double red[3 * NR];
 #pragma unroll
             for (int c = 0; c < 3 * NR; ++c) red[c] = 0.0;
-            for (int i = t0; i < n; i += T) {
+            for (int i = t0, u = 0; i < n; i += T, ++u) {
                 double y[NR];
-                row_dot_scaled<NR, MULTI>(a.A, a.svals, i, a.s, n, act, y);
+                if constexpr (RES) row_dot_resident<NR>(M, a.wmax, u, a.s, n, act, y);
+                else row_dot_scaled<NR, MULTI>(a.A, a.svals, i, a.s, n, act, y);
 #pragma unroll
                 for (int c = 0; c < NR; ++c) {
                     if (!act[c]) continue;
@@ -1099,14 +1168,16 @@ static int bicg_blocks_for(int n, int maxb) {
 static int bicg_max_blocks(int nrhs, bool multi) {
     static int mb[4] = {0, 0, 0, 0};
     if (!mb[0]) {
-        mb[0] = coresident_blocks(k_bicgstab<1, false>);
-        mb[1] = coresident_blocks(k_bicgstab<3, false>);
-        mb[2] = coresident_blocks(k_bicgstab<3, true>);
+        mb[0] = coresident_blocks(k_bicgstab<1, false, false>);
+        mb[1] = coresident_blocks(k_bicgstab<3, false, false>);
+        mb[2] = coresident_blocks(k_bicgstab<3, true, false>);
         mb[3] = std::max(std::max(mb[0], mb[1]), mb[2]);
     }
     if (nrhs < 0) return mb[3];
     return nrhs == 1 ? mb[0] : (multi ? mb[2] : mb[1]);
 }
+
+constexpr unsigned BICG_SMEM = 210 * 1024;  // shared memory of the resident form's CTA
 
 static void bicg_launch(const SellDev &A, const double *const *vals, bool multi, int nrhs, const double *const *b,
                         double *const *x, const KrylovOpts &o, KrylovWork &w, SolveInfo *info, cudaStream_t st,
@@ -1145,11 +1216,20 @@ static void bicg_launch(const SellDev &A, const double *const *vals, bool multi,
     a.maxit = o.maxit;
     a.eps = o.eps;
     void *args[] = {&a};
-    int G = grid_for(n, bicg_blocks_for(n, maxb));
-    const void *k = nrhs == 1 ? (const void *)k_bicgstab<1, false>
-                              : (multi ? (const void *)k_bicgstab<3, true> : (const void *)k_bicgstab<3, false>);
+    a.G = grid_for(n, bicg_blocks_for(n, maxb));
+    a.wmax = A.wmax;
+    // the resident form wherever the CTAs' rows fit
+    const int C = std::min(a.G, w.sm_cap > 0 ? std::min(w.sm_cap, num_sms()) : num_sms());
+    const int nt = KB * ((a.G + C - 1) / C), R = (n + a.G * KB - 1) / (a.G * KB);
+    const size_t smem = (size_t)nt * R * A.wmax * 12;
+    const bool res = !multi && nt <= BICG_RES_NT && R <= 4 && A.wmax <= 255 && smem <= BICG_SMEM;
+    const void *k;
+    if (res) k = nrhs == 1 ? (const void *)k_bicgstab<1, false, true> : (const void *)k_bicgstab<3, false, true>;
+    else if (nrhs == 1) k = (const void *)k_bicgstab<1, false, false>;
+    else k = multi ? (const void *)k_bicgstab<3, true, false> : (const void *)k_bicgstab<3, false, false>;
+    if (res) SYSU_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BICG_SMEM));
     SYSU_CUDA(cudaMemsetAsync(w.barrier.get(), 0, sizeof(GridBarrier), st));  // grid_sync starts from 0
-    SYSU_CUDA(cudaLaunchCooperativeKernel(k, dim3(G), dim3(KB), args, 0, st));
+    SYSU_CUDA(cudaLaunchCooperativeKernel(k, dim3(res ? C : a.G), dim3(res ? nt : KB), args, res ? smem : 0, st));
     ++::sysu::g_launches;
 }
 
