@@ -559,6 +559,31 @@ __device__ __forceinline__ void row_dot_scaled(const SellView &A, const double *
     }
 }
 
+// A vector of the resident form: R > 0: a thread's own rows in registers (u-th row at [u]); R = 0:
+// in global memory.
+template <int NR, int R>
+struct BicgVec {
+    double own[NR][R > 0 ? R : 1];
+    double *mem;
+    __device__ __forceinline__ double get(int c, int u, size_t k) const { return R > 0 ? own[c][u] : mem[k]; }
+    __device__ __forceinline__ void set(int c, int u, size_t k, double v) {
+        if (R > 0) own[c][u] = v;
+        else mem[k] = v;
+    }
+};
+
+// f(i, u): the thread's u-th row i
+template <int R, class F>
+__device__ __forceinline__ void bicg_rows(int t0, int T, int n, F &&f) {
+    if constexpr (R > 0) {
+#pragma unroll
+        for (int u = 0; u < R; ++u)
+            if (t0 + u * T < n) f(t0 + u * T, u);
+    } else {
+        for (int i = t0, u = 0; i < n; i += T, ++u) f(i, u);
+    }
+}
+
 // Rows thread-per-row with a grid stride over up to 608 blocks of 256 threads, FP64 sums in
 // a fixed order that is the same for one and for three right-hand sides, so u, v, w solved
 // together equal three solves to the bit.  BiCGSTAB amplifies the last bit of a sum (another
@@ -568,12 +593,13 @@ __device__ __forceinline__ void row_dot_scaled(const SellView &A, const double *
 // early exit, is summed with t.s and t.t.
 //
 // RES: the column-scaled matrix stays in shared memory, up to two blocks of KB threads in a
-// CTA, one CTA an SM: fewer arrivals at a barrier and no trips to L2 for the matrix.  Rows and
+// CTA, one CTA an SM: fewer arrivals at a barrier and no trips to L2 for the matrix; R > 0: the
+// vectors but for p and s, which other threads gather, in registers (R rows a thread).  Rows and
 // sums are dealt to the same (virtual) threads and blocks as without, so the bits are the same.
-// BICG_US
-template <int NR, bool MULTI, bool RES>
+// 60,680 rows, us an iteration: 23.6 without, 19.6 with the matrix, 17.6 with the vectors.
+template <int NR, bool MULTI, bool RES, int R>
 __global__ void __launch_bounds__(RES ? BICG_RES_NT : KB, RES ? 1 : 4) k_bicgstab(BicgArgs a) {
-    static_assert(!(MULTI && RES), "the resident form takes one matrix");
+    static_assert(!(MULTI && RES) && (RES || R == 0), "the resident form takes one matrix");
     if (a.gate && a.gate->status[0] != DEV_STALLED) return;  // the same word for every block
     const int it_before = a.gate ? a.gate->iters[0] : 0;
     const int n = a.A.n;
@@ -587,24 +613,35 @@ __global__ void __launch_bounds__(RES ? BICG_RES_NT : KB, RES ? 1 : 4) k_bicgsta
     const double *__restrict__ dinv = a.dinv;
     const size_t N = (size_t)n;
     __shared__ BicgState S;
+    BicgVec<NR, R> r, rt, v, t, x, p, sv;
+    double dg[R > 0 ? R : 1];
+    r.mem = a.r;
+    rt.mem = a.rt;
+    v.mem = a.v;
+    t.mem = a.t;
     {
-        double v[2 * NR];
+        double w[2 * NR];
 #pragma unroll
-        for (int c = 0; c < 2 * NR; ++c) v[c] = 0.0;
-        for (int i = t0; i < n; i += T) {
+        for (int c = 0; c < 2 * NR; ++c) w[c] = 0.0;
+        bicg_rows<R>(t0, T, n, [&](int i, int u) {
+            if (R > 0) dg[u] = dinv[i];
 #pragma unroll
             for (int c = 0; c < NR; ++c) {
                 double bi = a.b[c][i];
                 SellView Ac = a.A;
                 if (MULTI) Ac.val = a.vals[c];
                 double ri = bi - row_dot(Ac, i, a.x[c]);
-                a.r[c * N + i] = ri;
-                a.rt[c * N + i] = ri;
-                v[c] = fma(bi, bi, v[c]);
-                v[NR + c] = fma(ri, ri, v[NR + c]);
+                r.set(c, u, c * N + i, ri);
+                rt.set(c, u, c * N + i, ri);
+                if (R > 0) {
+                    x.own[c][u] = a.x[c][i];
+                    p.own[c][u] = sv.own[c][u] = v.own[c][u] = t.own[c][u] = 0.0;
+                }
+                w[c] = fma(bi, bi, w[c]);
+                w[NR + c] = fma(ri, ri, w[NR + c]);
             }
-        }
-        if (!bicg_sum<2 * NR>(v, rc, a.gb, err)) return;
+        });
+        if (!bicg_sum<2 * NR>(w, rc, a.gb, err)) return;
         if (tid < NR) {
             const int c = tid;
             S.bb[c] = g_bicg_sum[c] == 0.0 ? 1.0 : g_bicg_sum[c];
@@ -648,14 +685,17 @@ __global__ void __launch_bounds__(RES ? BICG_RES_NT : KB, RES ? 1 : 4) k_bicgsta
                 omg[c] = S.omg[c];
                 first[c] = S.it[c] == 1;
             }
-            for (int i = t0; i < n; i += T) {
+            bicg_rows<R>(t0, T, n, [&](int i, int u) {
 #pragma unroll
                 for (int c = 0; c < NR; ++c) {
                     if (!act[c]) continue;
                     size_t k = c * N + i;
-                    a.p[k] = first[c] ? a.r[k] : fma(beta[c], fma(-omg[c], a.v[k], a.p[k]), a.r[k]);
+                    const double ri = r.get(c, u, k);
+                    const double pi = first[c] ? ri : fma(beta[c], fma(-omg[c], v.get(c, u, k), R > 0 ? p.own[c][u] : a.p[k]), ri);
+                    a.p[k] = pi;
+                    if (R > 0) p.own[c][u] = pi;
                 }
-            }
+            });
         }
         if (!grid_sync(a.gb, err)) return;
         // v = A M^-1 p ; rt . v
@@ -663,17 +703,17 @@ __global__ void __launch_bounds__(RES ? BICG_RES_NT : KB, RES ? 1 : 4) k_bicgsta
             double red[NR];
 #pragma unroll
             for (int c = 0; c < NR; ++c) red[c] = 0.0;
-            for (int i = t0, u = 0; i < n; i += T, ++u) {
+            bicg_rows<R>(t0, T, n, [&](int i, int u) {
                 double y[NR];
                 if constexpr (RES) row_dot_resident<NR>(M, a.wmax, u, a.p, n, act, y);
                 else row_dot_scaled<NR, MULTI>(a.A, a.svals, i, a.p, n, act, y);
 #pragma unroll
                 for (int c = 0; c < NR; ++c) {
                     if (!act[c]) continue;
-                    a.v[c * N + i] = y[c];
-                    red[c] = fma(a.rt[c * N + i], y[c], red[c]);
+                    v.set(c, u, c * N + i, y[c]);
+                    red[c] = fma(rt.get(c, u, c * N + i), y[c], red[c]);
                 }
-            }
+            });
             if (!bicg_sum<NR>(red, rc, a.gb, err)) return;
             if (tid < NR) {
                 const int c = tid;
@@ -692,14 +732,16 @@ __global__ void __launch_bounds__(RES ? BICG_RES_NT : KB, RES ? 1 : 4) k_bicgsta
                 act[c] = S.act[c] != 0;
                 alpha[c] = S.alpha[c];
             }
-            for (int i = t0; i < n; i += T) {
+            bicg_rows<R>(t0, T, n, [&](int i, int u) {
 #pragma unroll
                 for (int c = 0; c < NR; ++c) {
                     if (!act[c]) continue;
                     size_t k = c * N + i;
-                    a.s[k] = fma(-alpha[c], a.v[k], a.r[k]);
+                    const double si = fma(-alpha[c], v.get(c, u, k), r.get(c, u, k));
+                    a.s[k] = si;
+                    if (R > 0) sv.own[c][u] = si;
                 }
-            }
+            });
         }
         if (!grid_sync(a.gb, err)) return;
         // t = A M^-1 s ; t.s, t.t, s.s
@@ -707,7 +749,7 @@ __global__ void __launch_bounds__(RES ? BICG_RES_NT : KB, RES ? 1 : 4) k_bicgsta
             double red[3 * NR];
 #pragma unroll
             for (int c = 0; c < 3 * NR; ++c) red[c] = 0.0;
-            for (int i = t0, u = 0; i < n; i += T, ++u) {
+            bicg_rows<R>(t0, T, n, [&](int i, int u) {
                 double y[NR];
                 if constexpr (RES) row_dot_resident<NR>(M, a.wmax, u, a.s, n, act, y);
                 else row_dot_scaled<NR, MULTI>(a.A, a.svals, i, a.s, n, act, y);
@@ -715,13 +757,13 @@ __global__ void __launch_bounds__(RES ? BICG_RES_NT : KB, RES ? 1 : 4) k_bicgsta
                 for (int c = 0; c < NR; ++c) {
                     if (!act[c]) continue;
                     size_t k = c * N + i;
-                    const double si = a.s[k];
-                    a.t[k] = y[c];
+                    const double si = R > 0 ? sv.own[c][u] : a.s[k];
+                    t.set(c, u, k, y[c]);
                     red[c] = fma(y[c], si, red[c]);
                     red[NR + c] = fma(y[c], y[c], red[NR + c]);
                     red[2 * NR + c] = fma(si, si, red[2 * NR + c]);
                 }
-            }
+            });
             if (!bicg_sum<3 * NR>(red, rc, a.gb, err)) return;
             if (tid < NR) {
                 const int c = tid;
@@ -742,24 +784,28 @@ __global__ void __launch_bounds__(RES ? BICG_RES_NT : KB, RES ? 1 : 4) k_bicgsta
                 omg[c] = S.omg[c];
                 early[c] = S.early[c] != 0;
             }
-            for (int i = t0; i < n; i += T) {
+            bicg_rows<R>(t0, T, n, [&](int i, int u) {
 #pragma unroll
                 for (int c = 0; c < NR; ++c) {
                     if (!act[c]) continue;
                     size_t k = c * N + i;
-                    double di = MULTI ? dinv[k] : dinv[i];
+                    const double di = R > 0 ? dg[u] : MULTI ? dinv[k] : dinv[i];
+                    const double pi = R > 0 ? p.own[c][u] : a.p[k], xi = R > 0 ? x.own[c][u] : a.x[c][i];
+                    double xn;
                     if (early[c]) {
-                        a.x[c][i] = fma(alpha[c], di * a.p[k], a.x[c][i]);
+                        xn = fma(alpha[c], di * pi, xi);
                     } else {
-                        double si = a.s[k];
-                        a.x[c][i] = fma(di, fma(alpha[c], a.p[k], omg[c] * si), a.x[c][i]);
-                        double ri = fma(-omg[c], a.t[k], si);
-                        a.r[k] = ri;
+                        const double si = R > 0 ? sv.own[c][u] : a.s[k];
+                        xn = fma(di, fma(alpha[c], pi, omg[c] * si), xi);
+                        const double ri = fma(-omg[c], t.get(c, u, k), si);
+                        r.set(c, u, k, ri);
                         red[c] = fma(ri, ri, red[c]);
-                        red[NR + c] = fma(a.rt[k], ri, red[NR + c]);
+                        red[NR + c] = fma(rt.get(c, u, k), ri, red[NR + c]);
                     }
+                    if (R > 0) x.own[c][u] = xn;
+                    else a.x[c][i] = xn;
                 }
-            }
+            });
             if (!bicg_sum<2 * NR>(red, rc, a.gb, err)) return;
             if (tid < NR) {
                 const int c = tid;
@@ -777,6 +823,11 @@ __global__ void __launch_bounds__(RES ? BICG_RES_NT : KB, RES ? 1 : 4) k_bicgsta
             __syncwarp();
         }
     }
+    if (R > 0)
+        bicg_rows<R>(t0, T, n, [&](int i, int u) {
+#pragma unroll
+            for (int c = 0; c < NR; ++c) a.x[c][i] = x.own[c][u];
+        });
     if (blockIdx.x == 0 && tid < NR) {
         const int c = tid;
         int st = S.status[c];
@@ -1168,9 +1219,9 @@ static int bicg_blocks_for(int n, int maxb) {
 static int bicg_max_blocks(int nrhs, bool multi) {
     static int mb[4] = {0, 0, 0, 0};
     if (!mb[0]) {
-        mb[0] = coresident_blocks(k_bicgstab<1, false, false>);
-        mb[1] = coresident_blocks(k_bicgstab<3, false, false>);
-        mb[2] = coresident_blocks(k_bicgstab<3, true, false>);
+        mb[0] = coresident_blocks(k_bicgstab<1, false, false, 0>);
+        mb[1] = coresident_blocks(k_bicgstab<3, false, false, 0>);
+        mb[2] = coresident_blocks(k_bicgstab<3, true, false, 0>);
         mb[3] = std::max(std::max(mb[0], mb[1]), mb[2]);
     }
     if (nrhs < 0) return mb[3];
@@ -1224,9 +1275,15 @@ static void bicg_launch(const SellDev &A, const double *const *vals, bool multi,
     const size_t smem = (size_t)nt * R * A.wmax * 12;
     const bool res = !multi && nt <= BICG_RES_NT && R <= 4 && A.wmax <= 255 && smem <= BICG_SMEM;
     const void *k;
-    if (res) k = nrhs == 1 ? (const void *)k_bicgstab<1, false, true> : (const void *)k_bicgstab<3, false, true>;
-    else if (nrhs == 1) k = (const void *)k_bicgstab<1, false, false>;
-    else k = multi ? (const void *)k_bicgstab<3, true, false> : (const void *)k_bicgstab<3, false, false>;
+    if (res && nrhs == 1)
+        k = R == 1 ? (const void *)k_bicgstab<1, false, true, 1>
+                   : R == 2 ? (const void *)k_bicgstab<1, false, true, 2> : (const void *)k_bicgstab<1, false, true, 4>;
+    else if (res)
+        k = R == 1 ? (const void *)k_bicgstab<3, false, true, 1> : (const void *)k_bicgstab<3, false, true, 0>;
+    else if (nrhs == 1)
+        k = (const void *)k_bicgstab<1, false, false, 0>;
+    else
+        k = multi ? (const void *)k_bicgstab<3, true, false, 0> : (const void *)k_bicgstab<3, false, false, 0>;
     if (res) SYSU_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BICG_SMEM));
     SYSU_CUDA(cudaMemsetAsync(w.barrier.get(), 0, sizeof(GridBarrier), st));  // grid_sync starts from 0
     SYSU_CUDA(cudaLaunchCooperativeKernel(k, dim3(res ? C : a.G), dim3(res ? nt : KB), args, res ? smem : 0, st));
