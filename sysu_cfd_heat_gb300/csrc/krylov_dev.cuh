@@ -21,63 +21,11 @@ struct RedCtx {
     int parity;
 };
 
-__device__ __shared__ double g_red_smem[NVMAX * 32];  // up to 32 warps per block
-__device__ __shared__ double g_red_res[NVMAX];
-
-// Block-reduce NV values, publish per-block partials, barrier, and give every
-// thread the NV global sums.  Partials alternate between two buffers so that a
-// block that runs ahead to the next reduction cannot overwrite values another
-// block is still reading.
-template <int NV>
-__device__ __forceinline__ bool grid_reduce(double (&v)[NV], RedCtx &rc, GridBarrier *gb, int *err) {
-    block_sum<NV>(v, g_red_smem);
-    double *buf = rc.partials + (size_t)rc.parity * NVMAX * rc.G;
-    rc.parity ^= 1;
-    if (threadIdx.x == 0)
-#pragma unroll
-        for (int k = 0; k < NV; ++k) buf[(size_t)k * rc.G + blockIdx.x] = v[k];
-    if (!grid_sync(gb, err)) return false;
-    if (threadIdx.x < 32) {
-#pragma unroll
-        for (int k = 0; k < NV; ++k) {
-            double s = warp_sum_partials(buf + (size_t)k * rc.G, rc.G);
-            if (threadIdx.x == 0) g_red_res[k] = s;
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < NV; ++k) v[k] = g_red_res[k];
-    __syncthreads();
-    return true;
-}
-
-// As grid_reduce, but the global sums are valid in thread 0 only: the caller
-// derives its scalars there once per block and broadcasts them (divisions and
-// square roots are long FP64 sequences; doing them in every thread costs more
-// FP64 issue slots than a row of the vector updates).
-template <int NV>
-__device__ __forceinline__ bool grid_reduce_t0(double (&v)[NV], RedCtx &rc, GridBarrier *gb, int *err) {
-    block_sum_t0<NV>(v, g_red_smem);
-    double *buf = rc.partials + (size_t)rc.parity * NVMAX * rc.G;
-    rc.parity ^= 1;
-    if (threadIdx.x == 0)
-#pragma unroll
-        for (int k = 0; k < NV; ++k) buf[(size_t)k * rc.G + blockIdx.x] = v[k];
-    if (!grid_sync(gb, err)) return false;
-    if (threadIdx.x < 32) {
-#pragma unroll
-        for (int k = 0; k < NV; ++k) {
-            double s = warp_sum_partials(buf + (size_t)k * rc.G, rc.G);
-            if (threadIdx.x == 0) v[k] = s;
-        }
-    }
-    return true;
-}
-
 // Exact deterministic grid sums of NV <= XS_NVMAX values per thread
 // (exact_sum.cuh); the sums are valid in thread 0 only.  Per-block partials are
 // (exponent, 128-bit sum, nonfinite flag) in four 64-bit words, double
-// buffered like grid_reduce's; rc.partials must hold 2 * XS_NVMAX * G * 4 words.
+// buffered, so that a block that runs ahead to the next sum cannot overwrite
+// values another block is still reading; rc.partials must hold 2 * XS_NVMAX * G * 4 words.
 constexpr int XS_NVMAX = 3;
 __shared__ long long g_xs_smem[XS_NVMAX * 32 * 4];
 
