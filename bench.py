@@ -128,21 +128,22 @@ class ClockSampler:
 
 
 def cg_bytes_per_iter(n: int, nnz: int, fp32: bool = False) -> float:
-    """Algorithmic bytes of one CG iteration of the p' kernel (two phases):
-    S reads the matrix once (values + int32 columns), gathers z once (one value per
-    row), reads and writes p and q; X reads p, q, x (or the correction e), r,
-    D^-1 and writes x (e), r, z.  FP64: nnz*12 + 104*N; FP32 recurrences:
-    nnz*8 + 52*N."""
+    """Algorithmic bytes of one CG iteration of the p' kernel (two phases, on the
+    symmetrically scaled system: unit diagonal, r for z): S reads the off-diagonals once
+    (values + int32 columns), gathers r once (one value per row), reads and writes y (or
+    the correction e), p and q; X reads q and the FP32 diagonal weights and reads and
+    writes r.  FP64: (nnz-N)*12 + 84*N; FP32 recurrences: (nnz-N)*8 + 44*N."""
     if fp32:
-        return nnz * 8 + 52 * n
-    return nnz * 12 + 104 * n
+        return (nnz - n) * 8 + 44 * n
+    return (nnz - n) * 12 + 84 * n
 
 
 def cg_flops_per_iter(n: int, nnz_true: int) -> float:
-    """FP64 flops of one CG iteration: 2 per stored-true matrix entry, 6 per row in S
-    (p, q updates, p.q), 7 per row in X (x, r, z, r.z; r.r, which only serves the
-    stopping test, is estimated in FP32 and taken exactly only near the threshold)."""
-    return 2.0 * nnz_true + 13.0 * n
+    """FP64 flops of one CG iteration: 2 per true off-diagonal entry, 8 per row in S
+    (y, p, q updates, p.q), 4 per row in X (r, r.r; the true residual's norm, which only
+    serves the stopping test, is estimated in FP32 and taken exactly only near the
+    threshold)."""
+    return 2.0 * (nnz_true - n) + 12.0 * n
 
 
 def host_cpu() -> dict:
@@ -657,7 +658,7 @@ def matched_forms(s, args, n, nnz, hbm):
             b32 = cg_bytes_per_iter(n, nnz, fp32=True)
             init32 = nnz * 12 + 40 * n
             ach32 = statistics.mean([(it * b32 + init32) / (ms / 1000.0) / 1e9 for it, ms in zip(pit, pm) if ms > 0])
-            entry["roofline"] = {"bound": "hbm", "kernel": "k_cg_mixed_pipe", "achieved": ach32, "peak": hbm,
+            entry["roofline"] = {"bound": "hbm", "kernel": "k_cg_mixed_sym", "achieved": ach32, "peak": hbm,
                                  "unit": "GB/s", "frac": ach32 / hbm, "algorithmic_bytes_per_cg_iteration": b32}
         out[name] = entry
     for k, v in P_OPTION_DEFAULTS.items():
@@ -850,7 +851,9 @@ def run_ours(args, r, w, lr):
     hbm = hbm or 6800.0
     # dominant kernel: the persistent p' CG launch (one per outer iteration)
     b_iter = cg_bytes_per_iter(n, nnz)
-    init_b = nnz * 12 + 48 * n  # initial residual: matrix, x gathered, b, D^-1 read, r, z written
+    # initial residual: matrix, x gathered, b, S read, r written; the scaled copy: matrix read,
+    # off-diagonals written
+    init_b = nnz * 12 + 48 * n + nnz * 12 + (nnz - n) * 12
     bytes_launch = [it * b_iter + init_b for it in cg_it]
     ach = [b / (ms / 1000.0) / 1e9 for b, ms in zip(bytes_launch, p_ms) if ms > 0]
     achieved = statistics.mean(ach) if ach else None
@@ -901,11 +904,11 @@ def run_ours(args, r, w, lr):
         "e2e": {"value": w * args.steps / e2e_s, "unit": "iters/s", "h2d_bytes_per_step": h2d,
                 "d2h_bytes_per_step": d2h},
         "gpu_launches": int(launches),
-        "roofline": {"bound": "hbm", "kernel": "k_cg_pipe (persistent Jacobi-PCG for p')",
+        "roofline": {"bound": "hbm", "kernel": "k_cg_sym (persistent Jacobi-PCG for p')",
                      "achieved": achieved, "peak": hbm, "peak_source": peak_src, "unit": "GB/s",
                      "frac": (achieved / hbm) if achieved else None, "traffic": traffic,
                      "algorithmic_bytes_per_cg_iteration": b_iter},
-        "fp64_pipe": {"kernel": "k_cg_pipe", "achieved_tflops": dp_tflops, "peak_tflops": FP64_PEAK_TFLOPS,
+        "fp64_pipe": {"kernel": "k_cg_sym", "achieved_tflops": dp_tflops, "peak_tflops": FP64_PEAK_TFLOPS,
                       "peak_source": "nominal GB300 FP64 rate (2 FMA lanes per SM per clock)",
                       "frac": (dp_tflops / FP64_PEAK_TFLOPS) if dp_tflops else None,
                       "flops_per_cg_iteration": f_iter},
