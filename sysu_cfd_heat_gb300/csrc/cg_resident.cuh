@@ -13,9 +13,9 @@
 // and reported figures as k_cg_pipe / k_cg_mixed_pipe.
 //
 // Measured, us per iteration, streaming kernels before -> here: 13,824 rows of a hex mesh in
-// FP64 13.2 -> 6.6 (two sums of 2 us, the FP64 latencies of a row and of alpha),
-// 51,200 rows 13.8 -> 7.7, 256,000 rows 19.3 -> 13.2 (5.7 us of it FP64 pipe); 262,144 rows in
-// FP32 16.2 -> 8.2.  The line to the streaming kernels is the shared memory: there is no size
+// FP64 13.2 -> 6.1 (two sums of 2 us, the FP64 latencies of a row and of alpha; an idle thread
+// forms 1 / rho during the first sum), 256,000 rows 19.3 -> 12.8 (5.7 us of it FP64 pipe);
+// 262,144 rows in FP32 16.2 -> 7.7.  The line to the streaming kernels is the shared memory: there is no size
 // that fits and was faster streamed.
 #pragma once
 

@@ -125,11 +125,11 @@ __global__ void k_na_dinv(NaArgs a) {
 // other CTAs gather, is the only vector in memory.  Latency bounds it at every size up to the
 // limit: two sums (grid_all.cuh) and two FP64 divisions an iteration.  1,716 rows on 7 blocks
 // of 256 threads, with three barriers and FP64 shuffle trees, square roots and divisions in
-// every thread, took 13.7 us an iteration; on 54 CTAs here 6.9 (238,080 rows: 13.0).
+// every thread, took 13.7 us an iteration; on 54 CTAs here 6.6 (238,080 rows: 12.8).
 // CL: the grid is one cluster.  z lies in its CTAs' shared memory, the columns there are turned
 // into shared addresses of the cluster, and the sums meet at the cluster's barrier: 5.3 us with
 // the two sums, 4.6 with one (CgScalars) and a barrier.  Over the whole GPU that form is not
-// faster (6.9 either way at 32,768 rows, 7.5 against 7.2 at 60,680): three values at once and a
+// faster (6.9 against 6.8 at 32,768 rows, 7.5 against 7.2 at 60,680): three values at once and a
 // bare barrier take as long as the two sums.
 template <int R, bool CL>
 __global__ void __launch_bounds__(NA_NT, 1) k_na_cg(NaArgs a) {
