@@ -123,7 +123,7 @@ __global__ void k_na_dinv(NaArgs a) {
 // the caller's CSR in shared memory when it fits (17,066 entries a CTA, so always for the
 // 7-entry rows of a hex mesh; a CTA whose rows hold more reads the caller's arrays).  z, which
 // other CTAs gather, is the only vector in memory.  Latency bounds it at every size up to the
-// limit: two sums (grid_all.cuh) and two FP64 divisions an iteration.  1,716 rows on 7 blocks
+// limit: two sums (grid_all.cuh) and an FP64 division an iteration.  1,716 rows on 7 blocks
 // of 256 threads, with three barriers and FP64 shuffle trees, square roots and divisions in
 // every thread, took 13.7 us an iteration; on 54 CTAs here 6.6 (238,080 rows: 12.8).
 // CL: the grid is one cluster.  z lies in its CTAs' shared memory, the columns there are turned
