@@ -124,7 +124,7 @@ __device__ __forceinline__ bool sym_acquire(int slot, unsigned par, int *err) {
     return acquire_at(slot, par, err);
 }
 
-// S phase of a consumer warp over the CTA's tiles, one slice a tile: returns the thread's
+// S phase of a consumer warp over the CTA's tiles, at most one slice a tile: returns the thread's
 // partial p.q.  pend: the alpha of the last X phase, still owed to y.  Issue slots count here
 // (with the place of a row computed in every tile: 400 warp instructions a row and iteration
 // in FP32, S 22.3 us of the 2M-row solve, 17.3 here), so places and widths come from a table
@@ -138,9 +138,11 @@ __device__ __forceinline__ V sym_s_phase(const Part &P, Ring &R, const CgSymArgs
     V *pv = static_cast<V *>(a.p), *qv = static_cast<V *>(a.q), *yv = static_cast<V *>(a.y);
     const V *rv = static_cast<const V *>(a.r);
     V pq = 0;
-    int s = P.sb + (int)(threadIdx.x >> 5), i = 32 * s + lane;
+    const int warp = (int)(threadIdx.x >> 5);
+    int s = P.sb + warp, i = 32 * s + lane;
     for (int t = 0; t < nt; ++t, s += P.ts, i += 32 * P.ts) {
-        const bool act = i < a.A.n && s < P.se;
+        // wide rows: a tile holds fewer slices than there are consumer warps
+        const bool act = warp < P.ts && i < a.A.n && s < P.se;
         V r = 0, p = 0, q = 0, y = 0;
         int2 pl = make_int2(0, 0);
         if (act) {
