@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(CR_NT, 1) k_cg_res(CgResArgs a, int wmax) {
         if (!all_sum<1>(v1, CH_PQ, c, err, [&](int, double pq) {
                 g_bc[2] = pq == 0.0 ? 0.0 : s_rho / pq;
                 g_bc[3] = pq == 0.0 ? 1.0 : 0.0;
-            }, [&] { s_inv = 1.0 / s_rho; })) { ok = false; break; }
+            }, [&] { s_inv = recip(s_rho); })) { ok = false; break; }
         stamp(a.ts, it, 1);
         if (g_bc[3] != 0.0) { status = DEV_BREAKDOWN; break; }
         const double alpha = g_bc[2];
@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(CR_NT, 1) k_cg_res(CgResArgs a, int wmax) {
         if (bias) v2[0] = (double)rr32;
         if (!all_sum<2>(v2, CH_RZ, c, err, [&](int k, double sum) {
                 if (k == 1) {
-                    g_bc[1] = sum * s_inv;
+                    g_bc[1] = quotient(sum, s_rho, s_inv);
                     s_rho = sum;
                 } else if (bias) {
                     // the estimate decides only when it is clearly above the threshold
@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(CR_NT, 1) k_cg_mixed_res(CgResArgs a, int wmax
         if (!all_sum<1>(v1, CH_PQ, c, err, [&](int, double pq) {
                 g_bc[2] = pq == 0.0 ? 0.0 : s_rho / pq;
                 g_bc[3] = pq == 0.0 ? 1.0 : 0.0;
-            }, [&] { s_inv = 1.0 / s_rho; })) return;
+            }, [&] { s_inv = recip(s_rho); })) return;
         stamp(a.ts, total, 1);
         if (g_bc[3] != 0.0) { status = DEV_BREAKDOWN; break; }
         const float alpha = (float)g_bc[2];
@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(CR_NT, 1) k_cg_mixed_res(CgResArgs a, int wmax
         double w2[2] = {(double)h0, (double)h1};
         if (!all_sum<2>(w2, CH_RZ, c, err, [&](int k, double sum) {
                 if (k == 1) {
-                    g_bc[1] = sum * s_inv;  // the next beta, unless an update replaces r
+                    g_bc[1] = quotient(sum, s_rho, s_inv);  // the next beta, unless an update replaces r
                     s_rz = sum;
                 } else {
                     // reliable update: as k_cg_mixed_pipe (the FP32 sums are in sig^2 units)

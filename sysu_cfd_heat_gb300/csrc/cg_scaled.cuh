@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(SYM_NT, 1) k_cg_sym(CgSymArgs a) {
         v2[0] = (double)est;
         if (!all_sum<2>(v2, CH_RZ, gc, err, [&](int k, double sum) {
                 if (k == 1) {
-                    g_bc[1] = sum / s_rho;
+                    g_bc[1] = quotient(sum, s_rho, 0.0);
                     s_rho = sum;
                 } else {
                     // the estimate decides only when it is clearly above the threshold

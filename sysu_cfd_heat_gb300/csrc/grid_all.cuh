@@ -411,6 +411,18 @@ __device__ __forceinline__ bool all_sync(AllCtx &c, int *err) {
     return *reinterpret_cast<volatile int *>(&g_ax_bad) == 0;
 }
 
+// a / b by way of the reciprocal that an idle thread formed earlier, so that what stands in the
+// chain of an iteration is a multiplication (a division takes 840 clocks).  recip: 0 where 1 / b
+// is not a normal number (|b| below 2^-1021: it may be infinite where a / b is not); there the
+// quotient is divided, and 0 / b is 0 also where b has underflowed to 0: CG then starts a new
+// direction instead of losing x to 0 / 0.
+__device__ __forceinline__ double recip(double b) {
+    return fabs(b) >= 0x1p-1021 && fabs(b) <= 0x1p+1021 ? 1.0 / b : 0.0;
+}
+__device__ __forceinline__ double quotient(double a, double b, double inv_b) {
+    return inv_b != 0.0 ? a * inv_b : a == 0.0 ? 0.0 : a / b;
+}
+
 // ---- the same for a grid that is one thread-block cluster ----------------------
 // The blocks write their sums into each other's shared memory and meet at the cluster's
 // hardware barrier: 0.6 us a sum where the accumulators in L2 take 2 (16 blocks).  The totals
@@ -500,17 +512,22 @@ __device__ __forceinline__ void cl_sum(const double (&v)[NV], ClCtx &c, Fin &&fi
 // the next iteration needs are formed by an idle thread during the barrier.
 struct CgScalars {
     double gamma, delta, beta, alpha, den;
-    double inv_gamma, inv_alpha;  // of the iteration before; 0 in the first
+    double old_gamma, inv_gamma, inv_alpha;  // of the iteration before
 };
 
+__device__ __forceinline__ void cg_first(CgScalars &S) {  // beta = 0 and nothing taken off delta
+    S.old_gamma = __longlong_as_double(0x7FF0000000000000ll);
+    S.inv_gamma = S.inv_alpha = 0.0;
+}
 __device__ __forceinline__ void cg_scalars(CgScalars &S) {
-    S.beta = S.gamma * S.inv_gamma;
+    S.beta = quotient(S.gamma, S.old_gamma, S.inv_gamma);
     S.den = fma(-(S.beta * S.inv_alpha), S.gamma, S.delta);
     S.alpha = S.den == 0.0 ? 0.0 : S.gamma / S.den;
 }
 __device__ __forceinline__ void cg_next(CgScalars &S) {
-    S.inv_gamma = 1.0 / S.gamma;
-    S.inv_alpha = S.den * S.inv_gamma;
+    S.old_gamma = S.gamma;
+    S.inv_gamma = recip(S.gamma);
+    S.inv_alpha = S.gamma == 0.0 ? 0.0 : quotient(S.den, S.gamma, S.inv_gamma);
 }
 
 }  // namespace

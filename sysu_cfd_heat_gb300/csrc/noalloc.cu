@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(NA_NT, 1) k_na_cg(NaArgs a) {
             } else {
                 s_rho = s;
                 s_beta = 0.0;
-                S.inv_gamma = S.inv_alpha = 0.0;
+                sysu::cg_first(S);
             }
         })) return;
     auto product = [&](int u) {  // row u of A z
@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(NA_NT, 1) k_na_cg(NaArgs a) {
         if (!sysu::all_sum(v1, 3, c, &h->err, [&](int, double pq) {
                 s_brk = pq == 0.0;
                 s_alpha = pq == 0.0 ? 0.0 : s_rho / pq;
-            }, [&] { s_inv = 1.0 / s_rho; })) return;
+            }, [&] { s_inv = sysu::recip(s_rho); })) return;
         if (s_brk) { status = sysu::DEV_BREAKDOWN; break; }
         const double alpha = s_alpha;
         double v2[2] = {0.0, 0.0};
@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(NA_NT, 1) k_na_cg(NaArgs a) {
                 if (k == 0) {
                     s_rr = s;
                 } else {
-                    s_beta = s * s_inv;
+                    s_beta = sysu::quotient(s, s_rho, s_inv);
                     s_rho = s;
                 }
             })) return;
