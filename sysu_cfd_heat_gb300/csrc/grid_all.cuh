@@ -423,6 +423,17 @@ __device__ __forceinline__ double quotient(double a, double b, double inv_b) {
     return inv_b != 0.0 ? a * inv_b : a == 0.0 ? 0.0 : a / b;
 }
 
+// The stopping test ||r|| / ||b|| < eps, on the squares where thr = stop_threshold(eps, bb) > 0 (a
+// square root takes 2,600 clocks, a division 840).  0: eps is not positive, or eps^2 ||b||^2 leaves
+// the range of normal numbers, and the norms themselves are compared.
+__device__ __forceinline__ double stop_threshold(double eps, double bb) {
+    const double thr = eps * eps * bb;
+    return eps > 0.0 && thr >= 0x1p-1022 && isfinite(thr) ? thr : 0.0;
+}
+__device__ __forceinline__ bool stop_below(double rr, double thr, double eps, double bb) {
+    return thr > 0.0 ? rr < thr : sqrt(rr) / sqrt(bb) < eps;
+}
+
 // ---- the same for a grid that is one thread-block cluster ----------------------
 // The blocks write their sums into each other's shared memory and meet at the cluster's
 // hardware barrier: 0.6 us a sum where the accumulators in L2 take 2 (16 blocks).  The totals

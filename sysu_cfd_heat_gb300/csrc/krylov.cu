@@ -427,12 +427,14 @@ struct BicgArgs {
 // Scalar state of a BiCGSTAB solve, in shared memory.  One thread a component derives it
 // from the global sums (every block adds them in the same order, so all blocks hold the
 // same bits): the divisions run once per block, the components side by side, and the vector
-// loops keep only the scalars they use in registers.  Norms are compared squared: an FP64
-// square root takes 2,600 clocks here, a division 840.
+// loops keep only the scalars they use in registers.  Norms are compared squared (stop_below).
 struct BicgState {
     double bb[3], rr[3], thr[3], rho[3], rho_prev[3], alpha[3], omg[3], beta[3];
     int it[3], status[3], done[3], act[3], early[3];
 };
+__device__ __forceinline__ bool bicg_below(const BicgState &S, int c, double rr, double eps) {
+    return stop_below(rr, S.thr[c], eps, S.bb[c]);
+}
 constexpr int BICG_RES_NT = 2 * KB;  // threads of the resident form's CTA at most
 __shared__ double g_bicg_smem[9 * (BICG_RES_NT / 32)], g_bicg_sum[9];
 
@@ -645,7 +647,7 @@ __global__ void __launch_bounds__(RES ? BICG_RES_NT : KB, RES ? 1 : 4) k_bicgsta
         if (tid < NR) {
             const int c = tid;
             S.bb[c] = g_bicg_sum[c] == 0.0 ? 1.0 : g_bicg_sum[c];
-            S.thr[c] = a.eps * a.eps * S.bb[c];
+            S.thr[c] = stop_threshold(a.eps, S.bb[c]);
             S.rr[c] = S.rho[c] = g_bicg_sum[NR + c];
             S.rho_prev[c] = S.alpha[c] = S.omg[c] = 1.0;
             S.it[c] = 0;
@@ -658,7 +660,7 @@ __global__ void __launch_bounds__(RES ? BICG_RES_NT : KB, RES ? 1 : 4) k_bicgsta
     for (;;) {
         if (tid < NR) {
             const int c = tid;
-            bool ac = !S.done[c] && !(S.rr[c] < S.thr[c]) && S.it[c] < a.maxit;
+            bool ac = !S.done[c] && !bicg_below(S, c, S.rr[c], a.eps) && S.it[c] < a.maxit;
             if (ac && !isfinite(S.rr[c])) { S.done[c] = 1; S.status[c] = DEV_NONFINITE; ac = false; }
             if (ac && S.rho[c] == 0.0) { S.done[c] = 1; S.status[c] = DEV_BREAKDOWN; ac = false; }
             if (ac) {
@@ -767,7 +769,7 @@ __global__ void __launch_bounds__(RES ? BICG_RES_NT : KB, RES ? 1 : 4) k_bicgsta
             if (!bicg_sum<3 * NR>(red, rc, a.gb, err)) return;
             if (tid < NR) {
                 const int c = tid;
-                S.early[c] = S.act[c] && g_bicg_sum[2 * NR + c] < S.thr[c];
+                S.early[c] = S.act[c] && bicg_below(S, c, g_bicg_sum[2 * NR + c], a.eps);
                 if (S.early[c]) S.rr[c] = g_bicg_sum[2 * NR + c];
                 else if (S.act[c]) S.omg[c] = g_bicg_sum[NR + c] != 0.0 ? g_bicg_sum[c] / g_bicg_sum[NR + c] : 0.0;
             }
@@ -816,7 +818,7 @@ __global__ void __launch_bounds__(RES ? BICG_RES_NT : KB, RES ? 1 : 4) k_bicgsta
                         S.rr[c] = g_bicg_sum[c];
                         S.rho_prev[c] = S.rho[c];
                         S.rho[c] = g_bicg_sum[NR + c];
-                        if (S.omg[c] == 0.0 && !(S.rr[c] < S.thr[c])) { S.done[c] = 1; S.status[c] = DEV_BREAKDOWN; }
+                        if (S.omg[c] == 0.0 && !bicg_below(S, c, S.rr[c], a.eps)) { S.done[c] = 1; S.status[c] = DEV_BREAKDOWN; }
                     }
                 }
             }
@@ -831,7 +833,7 @@ __global__ void __launch_bounds__(RES ? BICG_RES_NT : KB, RES ? 1 : 4) k_bicgsta
     if (blockIdx.x == 0 && tid < NR) {
         const int c = tid;
         int st = S.status[c];
-        if (st == DEV_OK && !(S.rr[c] < S.thr[c])) st = isfinite(S.rr[c]) ? DEV_MAXITER : DEV_NONFINITE;
+        if (st == DEV_OK && !bicg_below(S, c, S.rr[c], a.eps)) st = isfinite(S.rr[c]) ? DEV_MAXITER : DEV_NONFINITE;
         a.info->status[c] = st;
         a.info->iters[c] = S.it[c] + (c == 0 ? it_before : 0);
         a.info->res[c] = sqrt(S.rr[c]) / sqrt(S.bb[c]);

@@ -180,7 +180,10 @@ __global__ void __launch_bounds__(NA_NT, 1) k_na_cg(NaArgs a) {
     };
     __shared__ double s_rr, s_rho, s_thr, s_bb, s_alpha, s_beta, s_inv;
     __shared__ sysu::CgScalars S;
-    __shared__ int s_brk;
+    __shared__ int s_brk, s_end;  // s_end: 1 converged, 2 the residual is not finite, 0 go on
+    auto end_code = [&](double rr) {
+        return sysu::stop_below(rr, s_thr, a.eps, s_bb) ? 1 : isfinite(rr) ? 0 : 2;
+    };
     double x[R], r[R], p[R], q[R], d[R];
     int e0[R], len[R];
     double v3[3] = {0.0, 0.0, 0.0};
@@ -209,7 +212,7 @@ __global__ void __launch_bounds__(NA_NT, 1) k_na_cg(NaArgs a) {
     if (!sum(v3, 0, [&](int k, double s) {
             if (k == 0) {
                 s_bb = s == 0.0 ? 1.0 : s;
-                s_thr = a.eps * a.eps * s_bb;
+                s_thr = sysu::stop_threshold(a.eps, s_bb);
             } else if (k == 1) {
                 s_rr = s;
             } else {
@@ -246,12 +249,17 @@ __global__ void __launch_bounds__(NA_NT, 1) k_na_cg(NaArgs a) {
             v[2] = fma(w[u], z, v[2]);
         }
         sysu::cl_sum(v, cl, [&](int k, double s) {
-            if (k == 0) s_rr = s;
-            else if (k == 1) S.gamma = s;
-            else S.delta = s;
+            if (k == 0) {
+                s_rr = s;
+                s_end = end_code(s);
+            } else if (k == 1) {
+                S.gamma = s;
+            } else {
+                S.delta = s;
+            }
         });
-        if (s_rr < s_thr || it >= a.maxit) break;
-        if (!isfinite(s_rr)) { status = sysu::DEV_NONFINITE; break; }
+        if (s_end == 1 || it >= a.maxit) break;
+        if (s_end == 2) { status = sysu::DEV_NONFINITE; break; }
         ++it;
         if (tid == 0) sysu::cg_scalars(S);
         __syncthreads();
@@ -269,8 +277,12 @@ __global__ void __launch_bounds__(NA_NT, 1) k_na_cg(NaArgs a) {
         }
         sysu::cl_sync([&] { sysu::cg_next(S); });
     }
-    while (!CL && !(s_rr < s_thr) && it < a.maxit) {
-        if (!isfinite(s_rr)) { status = sysu::DEV_NONFINITE; break; }
+    if (!CL) {  // (the first sums are taken by different warps)
+        if (tid == 0) s_end = end_code(s_rr);
+        __syncthreads();
+    }
+    while (!CL && s_end != 1 && it < a.maxit) {
+        if (s_end == 2) { status = sysu::DEV_NONFINITE; break; }
         ++it;
         const double beta = s_beta;
         double v1[1] = {0.0};
@@ -303,6 +315,7 @@ __global__ void __launch_bounds__(NA_NT, 1) k_na_cg(NaArgs a) {
         if (!sysu::all_sum(v2, 4, c, &h->err, [&](int k, double s) {
                 if (k == 0) {
                     s_rr = s;
+                    s_end = end_code(s);
                 } else {
                     s_beta = sysu::quotient(s, s_rho, s_inv);
                     s_rho = s;
@@ -315,7 +328,7 @@ __global__ void __launch_bounds__(NA_NT, 1) k_na_cg(NaArgs a) {
         if (i < R1) a.x[i] = x[u];
     }
     if (blockIdx.x == 0 && tid == 0) {
-        if (status == sysu::DEV_OK && !(s_rr < s_thr)) status = isfinite(s_rr) ? sysu::DEV_MAXITER : sysu::DEV_NONFINITE;
+        if (status == sysu::DEV_OK && s_end != 1) status = s_end == 0 ? sysu::DEV_MAXITER : sysu::DEV_NONFINITE;
         h->status = status;
         h->iters = it;
         h->res = sqrt(s_rr) / sqrt(s_bb);

@@ -18,12 +18,12 @@ from test_gpu_resident_cg import seven_point
 pytestmark = pytest.mark.gpu
 
 
-def noalloc(rp, c, v, b, maxit, eps, omega=1.3):
+def noalloc(rp, c, v, b, maxit, eps, x0=None, omega=1.3):
     torch = pytest.importorskip("torch")
     f = C.CDLL(LIB_PATH).sysu_csr_cg_noalloc
     f.argtypes = [C.c_int] + [C.c_void_p] * 5 + [C.c_int, C.c_double, C.c_double] + [C.c_void_p] * 4
     d = [torch.from_numpy(t).cuda() for t in (rp, c, v, b)]
-    x = torch.zeros(len(b), dtype=torch.float64, device="cuda")
+    x = torch.from_numpy(np.zeros(len(b)) if x0 is None else x0.copy()).cuda()
     torch.cuda.synchronize()
     it, res, st = C.c_int(), C.c_double(), C.c_int()
     assert f(len(b), *(t.data_ptr() for t in d), x.data_ptr(), maxit, eps, omega, None, C.addressof(it),
