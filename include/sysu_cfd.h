@@ -390,6 +390,10 @@ int sysu_gnn_set_multigrid(sysu_gnn *g, int on, double theta, double omega, doub
                            int max_levels);
 /* z = M(r): one application of the attached cycle (host vectors of n values) */
 int sysu_gnn_mg_apply(sysu_gnn *g, const double *r, double *z, int use_gnn);
+/* Self-test: marks the attached cycle as if a grid barrier of its coarse levels had
+ * given up (every wait is bounded).  The next call that runs the cycle (fcg, mg_apply,
+ * add_pair) returns SYSU_ERR_CUDA for it; the one after that is unaffected. */
+int sysu_gnn_mg_wait_selftest(sysu_gnn *g);
 /* hidden state h^layer (layer 1..4) of the network on r, FP32 [n][32] */
 int sysu_gnn_hidden(sysu_gnn *g, const double *r, int layer, float *h);
 /* device ms of one network application on r (mean of reps); fwd_per_sm > 0

@@ -730,4 +730,17 @@ int AggMultigrid::err_flag(cudaStream_t st) {
     return e;
 }
 
+void AggMultigrid::check_wait(cudaStream_t st) {
+    if (err_flag(st) != DEV_BARRIER_TIMEOUT) return;
+    err_.zero(st);
+    gb_.zero(st);
+    throw CaseError{"multigrid: a grid barrier of the coarse levels timed out"};
+}
+
+void AggMultigrid::mark_wait_failed(cudaStream_t st) {
+    const int e = DEV_BARRIER_TIMEOUT;
+    err_.upload(&e, 1, st);
+    SYSU_CUDA(cudaStreamSynchronize(st));
+}
+
 }  // namespace sysu

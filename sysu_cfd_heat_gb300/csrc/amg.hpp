@@ -131,6 +131,11 @@ class AggMultigrid {
     float sgn() const { return sgn_; }
     const float *w0() const { return lv_[0]->w.get(); }
     int err_flag(cudaStream_t st);  // nonzero if a bounded wait or the inverse failed
+    // Waits for st and throws if a grid barrier of a coarse levels' launch gave up since the
+    // last call (the cycles' results are then incomplete); the next cycle starts clean.  The
+    // flexible CG does not wait for the host, so its callers call this or read err_dev().
+    void check_wait(cudaStream_t st);
+    void mark_wait_failed(cudaStream_t st);  // as a barrier that gave up does (self-test)
     // the same flag in device memory (0 until set), for reading with other results
     const int *err_dev() const { return err_.get(); }
 

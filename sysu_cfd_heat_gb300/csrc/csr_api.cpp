@@ -105,6 +105,7 @@ int sysu_csr_solve(int method, int precond, int n, const int *rowptr, const int 
                 fcg.attach_multigrid(&mg);
                 o.inner_tol = 0.1;
                 fcg.fcg(db.get(), dx.get(), false, o, false, info.get(), st);
+                mg.check_wait(st);
                 if (mg.err_flag(st)) throw sysu::CaseError{"multigrid: the coarsest level is singular"};
                 sysu::SolveInfo h;
                 info.download(&h, 1, st);

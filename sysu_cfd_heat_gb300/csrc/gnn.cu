@@ -1803,7 +1803,8 @@ void GnnPrecond::fcg(const double *b, double *x, bool x0_zero, const KrylovOpts 
     }
     SYSU_CUDA(cudaGraphLaunch(sg->exec, st));
     g_launches += sg->launches;
-    // a network that timed out on a tensor-core wait (the plain cycle sets nothing)
+    // a network that timed out on a tensor-core wait (a grid barrier of the cycle that gave up is
+    // the caller's to report: AggMultigrid::check_wait)
     if (use_gnn || (mg_ && mg_->post_hook)) check_err(st);
 }
 

@@ -31,6 +31,10 @@ int guarded(F f) {
         return SYSU_ERR_CUDA;
     }
 }
+// a grid barrier of the attached cycle that gave up is an error of the call that ran it
+void check_cycle(sysu_gnn *g) {
+    if (g->net.multigrid()) g->mg.check_wait(g->st);
+}
 }  // namespace
 
 extern "C" {
@@ -128,6 +132,7 @@ int sysu_gnn_add_pair(sysu_gnn *g, const double *r, const double *e) {
         g->v1.upload(e, n, g->st);
         g->net.add_pair(g->v0.get(), g->v1.get(), g->st);
         SYSU_CUDA(cudaStreamSynchronize(g->st));
+        check_cycle(g);
     });
 }
 
@@ -180,6 +185,7 @@ int sysu_gnn_fcg(sysu_gnn *g, const double *b, double *x, int x0_zero, int maxit
         cudaEventElapsedTime(&ms, e0, e1);
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
+        check_cycle(g);
         sysu::FcgState f = g->net.last_state(g->st);
         if (iters) *iters = f.iters;
         if (res) *res = f.res;
@@ -242,7 +248,13 @@ int sysu_gnn_mg_apply(sysu_gnn *g, const double *r, double *z, int use_gnn) {
         g->net.apply_mg(g->v0.get(), g->v1.get(), use_gnn != 0, g->st);
         g->v1.download(z, n, g->st);
         SYSU_CUDA(cudaStreamSynchronize(g->st));
+        check_cycle(g);
     });
+}
+
+int sysu_gnn_mg_wait_selftest(sysu_gnn *g) {
+    if (!g || !g->net.multigrid()) return SYSU_ERR_INPUT;
+    return guarded([&] { g->mg.mark_wait_failed(g->st); });
 }
 
 const char *sysu_gnn_last_error(void) { return g_gnn_err.c_str(); }

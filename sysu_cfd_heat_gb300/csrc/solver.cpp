@@ -527,6 +527,7 @@ void SimpleSolver::solve_learned(const EqOpts &o, const double *val, const doubl
                 // the level's own hierarchy serves the training pairs' level solves only
                 mg_c.omega = o.mg_omega;
                 mg_c.gamma = o.mg_gamma;
+                mg_c.one_launch = mg.one_launch;
                 mg_c.refresh(mg.level_val64(lvl), mg.level_val32(lvl), st);
             }
             gnn_c.refresh(st);
@@ -598,6 +599,8 @@ void SimpleSolver::solve_learned(const EqOpts &o, const double *val, const doubl
             gnn_c.fcg(mg_rl64.get(), mg_el64.get(), true, kl, false, mg_info.get(), st);
             gnn_c.add_pair(mg_rl64.get(), mg_el64.get(), st);
         }
+        mg_c.check_wait(st);  // its cycles, and those of the plain solves above, made the pairs
+        mg.check_wait(st);
         for (int k = 0; k < o.learn_steps; ++k) gnn_c.train_step(k % gnn_c.pairs(), o.learn_lr, st);
         return;
     }
@@ -627,6 +630,7 @@ void SimpleSolver::p_cycle(const double *r, double *z, bool use_net) {
     }
     d.download(z, n, st);
     SYSU_CUDA(cudaStreamSynchronize(st));
+    mg.check_wait(st);
 }
 
 // CalculateVelocity + BuildVelocityMatrix, navier_velocity.cpp:12-357
