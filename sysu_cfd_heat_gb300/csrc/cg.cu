@@ -41,6 +41,7 @@
 // which no kernel thread writes, goes through the async proxy.  Every wait is
 // bounded; a CTA drains its copies before it leaves.
 #include <climits>
+#include <cmath>
 
 #include "bulk.cuh"
 #include "krylov_dev.cuh"
@@ -1031,7 +1032,8 @@ template <class V>
 static const int *sym_launch(const SellDev &A, const double *val, const double *b, double *x, const KrylovOpts &o,
                              KrylovWork &w, SolveInfo *info, const SolveInfo *gate, cudaStream_t st) {
     constexpr bool fp32 = sizeof(V) == 4;
-    if (!o.jacobi || w.sm_cap > 0) return nullptr;
+    // (a positive Jacobi weight cancels; with any other the form with M^-1 says what becomes of it)
+    if (!o.jacobi || !(o.omega > 0.0) || !std::isfinite(o.omega) || w.sm_cap > 0) return nullptr;
     const int n = A.n;
     if (w.wt.size() < (size_t)n) w.wt.alloc(n);
     if (w.scol.size() < (size_t)A.nnz) w.scol.alloc(A.nnz);
