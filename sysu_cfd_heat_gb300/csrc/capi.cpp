@@ -316,7 +316,11 @@ int sysu_solver_set_option(sysu_solver *s, const char *key, double value) {
                 e->mg_gamma = value;
                 return SYSU_OK;
             }
-            if (f == "mg_persistent") { e->mg_persistent = value != 0.0; return SYSU_OK; }
+            if (f == "mg_persistent") {
+                e->mg_persistent = value != 0.0;
+                e->mg_persistent_set = true;
+                return SYSU_OK;
+            }
             if (f == "learn_level") {
                 if (value < 0.0 || value > 15.0) return set_err(SYSU_ERR_INPUT, "learn_level: multigrid level 0..15");
                 e->learn_level = (int)value;

@@ -507,7 +507,7 @@ void SimpleSolver::solve_learned(const EqOpts &o, const double *val, const doubl
         // one cooperative launch for the coarse levels, except where other cases share the GPU
         // (a captured outer iteration, a capped solve): it needs a block on every SM at once,
         // and would hold up the graph's other branches.  Part of the captured iterations' key.
-        mg.one_launch = o.mg_persistent != 0 || (kw.sm_cap <= 0 && !stream_capturing(st));
+        mg.one_launch = o.mg_persistent_set ? o.mg_persistent != 0 : kw.sm_cap <= 0 && !stream_capturing(st);
         mg.refresh(val, f.Ap32.get(), st);
         if (o.learned) lvl = std::max(0, std::min(o.learn_level, mg.levels() - 2));
         if (lvl >= 1) {

@@ -58,7 +58,10 @@ struct EqOpts {
     double mg_theta = 0.25;
     double mg_omega = 0.8;
     double mg_gamma = 1.8;
-    int mg_persistent = 0;    // 1: the coarse levels as one cooperative launch in shared graphs too
+    // the coarse levels 1: as one cooperative launch, 0: one launch a step (same results); not
+    // set: one launch, but in shared graphs
+    int mg_persistent = 0;
+    bool mg_persistent_set = false;
     // learned form with precond PK_AMG: the multigrid level whose post-smoother
     // the network is (0 the finest; deeper than the last coarse level clamps)
     int learn_level = 2;
