@@ -881,21 +881,22 @@ __device__ __forceinline__ float bicg_row32(const BicgMixedArgs &a, const float 
                                             int j, const float *x) {
     const int s = i >> 5, w = __ldg(a.A.sl_w + s);
     const int e = RES ? 0 : __ldg(a.A.sl_ptr + s) + (i & 31);
+    constexpr int U = RES ? 8 : 4;
     float y = 0.f;
-    for (int k0 = 0; k0 < w; k0 += 8) {
-        int c[8];
-        float v[8], g[8];
+    for (int k0 = 0; k0 < w; k0 += U) {
+        int c[U];
+        float v[U], g[U];
 #pragma unroll
-        for (int u = 0; u < 8; ++u)
+        for (int u = 0; u < U; ++u)
             if (k0 + u < w) {
                 c[u] = RES ? mcol[(k0 + u) * ld + j] : __ldg(a.A.col + e + 32 * (k0 + u));
                 v[u] = RES ? mval[(k0 + u) * ld + j] : __ldg(a.sv32 + e + 32 * (k0 + u));
             }
 #pragma unroll
-        for (int u = 0; u < 8; ++u)
+        for (int u = 0; u < U; ++u)
             if (k0 + u < w) g[u] = x[c[u]];
 #pragma unroll
-        for (int u = 0; u < 8; ++u)
+        for (int u = 0; u < U; ++u)
             if (k0 + u < w) y = fmaf(v[u], g[u], y);
     }
     return y;
@@ -904,12 +905,19 @@ __device__ __forceinline__ float bicg_row32(const BicgMixedArgs &a, const float 
 // One CTA per SM owns a contiguous range of slices; three grid sums (grid_all.cuh) and two
 // bare barriers an iteration, the FP32 matrix in shared memory where it fits (RES).  s takes
 // r's storage.  Below 300k rows the grid-wide steps bound it: 256,000 rows of a hex mesh took
-// 48 us an iteration on 250 blocks of 256 with FP64 shuffle trees and four sums, here 30.
-constexpr int BICG_NT = 512;
+// 48 us an iteration on 250 blocks of 256 with FP64 shuffle trees and four sums, here 28.
+// A matrix beyond shared memory (from 520,000 rows of a hex mesh) is bound by what is in flight,
+// so by the threads: 1024 with four entries of a row at a time (64 registers, no spill); 512 with
+// eight, which is what fits best on chip, was slower there than 608 blocks of 256 with four sums.
+// us an iteration, those 608 blocks / 512 threads / 768 / 1024: 592,704 rows 54, 32.6, 29.7, 27.4;
+// 1,000,000 rows 65, 47, 42, 37.7; 1,996,800 rows 147, 159, 135, 117; 4,096,000 rows 270, 324, 265, 233.
+template <bool RES>
+constexpr int bicg_nt = RES ? 512 : 1024;
 extern __shared__ __align__(16) unsigned char g_bicg_rows[];
 
 template <bool RES>
-__global__ void __launch_bounds__(BICG_NT, 1) k_bicgstab_mixed(BicgMixedArgs a, int wmax, int ld) {
+__global__ void __launch_bounds__(bicg_nt<RES>, 1) k_bicgstab_mixed(BicgMixedArgs a, int wmax, int ld) {
+    constexpr int NT = bicg_nt<RES>;
     const int n = a.A.n, tid = threadIdx.x;
     const bool lead = tid == 0;
     int *err = &a.info->err;
@@ -923,7 +931,7 @@ __global__ void __launch_bounds__(BICG_NT, 1) k_bicgstab_mixed(BicgMixedArgs a, 
     float *mval = reinterpret_cast<float *>(g_bicg_rows);
     int *mcol = reinterpret_cast<int *>(mval + (size_t)wmax * ld);
     if (RES) {
-        for (int i = R0 + tid; i < R1; i += BICG_NT) {
+        for (int i = R0 + tid; i < R1; i += NT) {
             const int s = i >> 5, w = __ldg(a.A.sl_w + s), e = __ldg(a.A.sl_ptr + s) + (i & 31);
             for (int k = 0; k < w; ++k) {
                 const int c = __ldg(a.A.col + e + 32 * k);
@@ -938,7 +946,7 @@ __global__ void __launch_bounds__(BICG_NT, 1) k_bicgstab_mixed(BicgMixedArgs a, 
     // call) and ||b - A x||^2.  The lead thread then restarts the inner process.
     auto residual = [&](bool first) -> bool {
         double v2[2] = {0.0, 0.0};
-        for (int i = R0 + tid; i < R1; i += BICG_NT) {
+        for (int i = R0 + tid; i < R1; i += NT) {
             const double bi = a.b[i];
             const double ri = bi - row_dot(a.A, i, a.x);
             a.r64[i] = ri;
@@ -951,7 +959,7 @@ __global__ void __launch_bounds__(BICG_NT, 1) k_bicgstab_mixed(BicgMixedArgs a, 
             })) return false;
         const double sg = S.sig;
         float f2 = 0.f;
-        for (int i = R0 + tid; i < R1; i += BICG_NT) {
+        for (int i = R0 + tid; i < R1; i += NT) {
             const float rf = (float)(sg * a.r64[i]);
             r[i] = rf;
             rt[i] = rf;
@@ -992,7 +1000,7 @@ __global__ void __launch_bounds__(BICG_NT, 1) k_bicgstab_mixed(BicgMixedArgs a, 
     // x += M^-1 e / sig in FP64, then the FP64 residual
     auto update = [&]() -> bool {
         const double isg = 1.0 / S.sig;
-        for (int i = R0 + tid; i < R1; i += BICG_NT) a.x[i] = fma(a.dinv[i] * isg, (double)ev[i], a.x[i]);
+        for (int i = R0 + tid; i < R1; i += NT) a.x[i] = fma(a.dinv[i] * isg, (double)ev[i], a.x[i]);
         if (!all_sync(gc, err)) return false;
         return residual(false);
     };
@@ -1011,14 +1019,14 @@ __global__ void __launch_bounds__(BICG_NT, 1) k_bicgstab_mixed(BicgMixedArgs a, 
             const float beta = (float)S.beta, omg = (float)S.omg;
             const bool first = S.inner == 1;
 #pragma unroll RB
-            for (int i = R0 + tid; i < R1; i += BICG_NT)
+            for (int i = R0 + tid; i < R1; i += NT)
                 p[i] = first ? r[i] : fmaf(beta, fmaf(-omg, v[i], p[i]), r[i]);
         }
         if (!all_sync(gc, err)) return;
         // v = A M^-1 p ; rt . v
         {
             float f = 0.f;
-            for (int i = R0 + tid; i < R1; i += BICG_NT) {
+            for (int i = R0 + tid; i < R1; i += NT) {
                 const float y = bicg_row32<RES>(a, mval, mcol, ld, i, i - R0, p);
                 v[i] = y;
                 f = fmaf(rt[i], y, f);
@@ -1037,13 +1045,13 @@ __global__ void __launch_bounds__(BICG_NT, 1) k_bicgstab_mixed(BicgMixedArgs a, 
         {
             const float alpha = (float)S.alpha;
 #pragma unroll RB
-            for (int i = R0 + tid; i < R1; i += BICG_NT) r[i] = fmaf(-alpha, v[i], r[i]);
+            for (int i = R0 + tid; i < R1; i += NT) r[i] = fmaf(-alpha, v[i], r[i]);
         }
         if (!all_sync(gc, err)) return;
         // t = A M^-1 s ; t.s, t.t, s.s
         {
             float f0 = 0.f, f1 = 0.f, f2 = 0.f;
-            for (int i = R0 + tid; i < R1; i += BICG_NT) {
+            for (int i = R0 + tid; i < R1; i += NT) {
                 const float y = bicg_row32<RES>(a, mval, mcol, ld, i, i - R0, r);
                 const float si = r[i];
                 t[i] = y;
@@ -1061,7 +1069,7 @@ __global__ void __launch_bounds__(BICG_NT, 1) k_bicgstab_mixed(BicgMixedArgs a, 
         }
         const float alpha = (float)S.alpha, omg = (float)S.omg;
         if (S.early) {  // e += alpha p, then the FP64 update
-            for (int i = R0 + tid; i < R1; i += BICG_NT) ev[i] = fmaf(alpha, p[i], ev[i]);
+            for (int i = R0 + tid; i < R1; i += NT) ev[i] = fmaf(alpha, p[i], ev[i]);
             if (!update()) return;
             continue;
         }
@@ -1069,7 +1077,7 @@ __global__ void __launch_bounds__(BICG_NT, 1) k_bicgstab_mixed(BicgMixedArgs a, 
         {
             float f0 = 0.f, f1 = 0.f;
 #pragma unroll RB
-            for (int i = R0 + tid; i < R1; i += BICG_NT) {
+            for (int i = R0 + tid; i < R1; i += NT) {
                 const float si = r[i];
                 ev[i] = fmaf(alpha, p[i], fmaf(omg, si, ev[i]));
                 const float ri = fmaf(-omg, t[i], si);
@@ -1348,7 +1356,7 @@ void bicgstab_solve_mixed(const SellDev &A, const double *val, const double *b, 
     const void *kern = res ? (const void *)k_bicgstab_mixed<true> : (const void *)k_bicgstab_mixed<false>;
     if (res) SYSU_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget));
     void *args[] = {&a, &wmax, &ld};
-    SYSU_CUDA(cudaLaunchCooperativeKernel(kern, dim3(G), dim3(BICG_NT), args, res ? want : 0, st));
+    SYSU_CUDA(cudaLaunchCooperativeKernel(kern, dim3(G), dim3(res ? bicg_nt<true> : bicg_nt<false>), args, res ? want : 0, st));
     ++::sysu::g_launches;
     // FP64 takes over from the current x if the FP32 refinement stalled (the
     // launch returns at once otherwise)
