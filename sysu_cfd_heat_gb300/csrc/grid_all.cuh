@@ -417,10 +417,13 @@ __device__ __forceinline__ bool all_sync(AllCtx &c, int *err) {
 // quotient is divided, and 0 / b is 0 also where b has underflowed to 0: CG then starts a new
 // direction instead of losing x to 0 / 0.
 __device__ __forceinline__ double recip(double b) {
-    return fabs(b) >= 0x1p-1021 && fabs(b) <= 0x1p+1021 ? 1.0 / b : 0.0;
+    const int e = (__double2hiint(b) >> 20) & 0x7FF;  // |b| in [2^-1021, 2^1021), by integer tests
+    return e >= 2 && e < 2044 ? 1.0 / b : 0.0;
 }
 __device__ __forceinline__ double quotient(double a, double b, double inv_b) {
-    return inv_b != 0.0 ? a * inv_b : a == 0.0 ? 0.0 : a / b;
+    if (__double2hiint(inv_b) != 0) return a * inv_b;
+    asm volatile("");  // a branch: the division is not to be formed beside the product
+    return a == 0.0 ? 0.0 : a / b;
 }
 
 // The stopping test ||r|| / ||b|| < eps, on the squares where thr = stop_threshold(eps, bb) > 0 (a
@@ -430,9 +433,14 @@ __device__ __forceinline__ double stop_threshold(double eps, double bb) {
     const double thr = eps * eps * bb;
     return eps > 0.0 && thr >= 0x1p-1022 && isfinite(thr) ? thr : 0.0;
 }
+// (rr >= 0 or NaN and thr >= 0 compare as integers: an FP64 comparison waits 64 clocks)
 __device__ __forceinline__ bool stop_below(double rr, double thr, double eps, double bb) {
-    return thr > 0.0 ? rr < thr : sqrt(rr) / sqrt(bb) < eps;
+    const long long t = __double_as_longlong(thr);
+    if (t != 0) return __double_as_longlong(rr) < t;
+    asm volatile("");  // a branch: the roots are not to be formed beside the comparison
+    return eps > 0.0 && sqrt(rr) / sqrt(bb) < eps;
 }
+__device__ __forceinline__ bool finite_bits(double v) { return ((__double2hiint(v) >> 20) & 0x7FF) != 0x7FF; }
 
 // ---- the same for a grid that is one thread-block cluster ----------------------
 // The blocks write their sums into each other's shared memory and meet at the cluster's
