@@ -52,7 +52,8 @@ constexpr int NA_CL_ROWS = 16 * NA_NT;     // up to here one cluster of at most 
 enum NaBad : int { NA_BAD_NONE = 0, NA_BAD_ROWPTR = 1, NA_BAD_COL = 2, NA_BAD_DIAG = 3 };
 
 struct NaHeader {  // at the start of the array, cleared by every call
-    int unused[2];
+    int unused;
+    int wide;  // the rows of a CTA of the cluster do not fit its shared memory: it has not run
     int err;
     int status;
     int iters;
@@ -80,7 +81,13 @@ struct NaArgs {
     int maxit;
     double eps;
     double *base;  // device address of g_noalloc_scratch
+    int cluster;   // CTAs of the cluster that is to solve the system; 0: the whole GPU does
 };
+
+// First row of block o of G: whole groups of 32.
+__device__ __forceinline__ int na_first_row(int n, int o, int G) {
+    return min(n, 32 * (int)((long long)((n + 31) / 32) * o / G));
+}
 
 constexpr unsigned long long NA_GOOD = ~0ull;
 
@@ -90,11 +97,16 @@ __device__ __forceinline__ void na_report(NaHeader *h, int row, int kind) {
 
 // D^-1 scaled by omega, and the checks of the caller's CSR: rows whose pointer
 // decreases, columns outside 0..n-1 and rows without a nonzero diagonal are
-// recorded in the header (lowest row) instead of being used.
+// recorded in the header (lowest row) instead of being used.  Says also whether the cluster
+// can hold the matrix.
 __global__ void k_na_dinv(NaArgs a) {
     NaHeader *h = reinterpret_cast<NaHeader *>(a.base);
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= a.n) return;
+    if (i < a.cluster &&
+        (long long)a.rowptr[na_first_row(a.n, i + 1, a.cluster)] - a.rowptr[na_first_row(a.n, i, a.cluster)] >
+            NA_ENTRIES)
+        h->wide = 1;
     int k0 = a.rowptr[i], k1 = a.rowptr[i + 1];
     double d = 0.0;
     int kind = NA_BAD_NONE;
@@ -121,7 +133,7 @@ __global__ void k_na_dinv(NaArgs a) {
 //
 // One CTA per SM owns a contiguous range of rows: their vectors in registers, their part of
 // the caller's CSR in shared memory when it fits (17,066 entries a CTA, so always for the
-// 7-entry rows of a hex mesh; a CTA whose rows hold more reads the caller's arrays).  z, which
+// 7-entry rows of a hex mesh; without a cluster a CTA whose rows hold more reads the caller's arrays).  z, which
 // other CTAs gather, is the only vector in memory.  Latency bounds it at every size up to the
 // limit: two sums (grid_all.cuh) and an FP64 division an iteration.  1,716 rows on 7 blocks
 // of 256 threads, with three barriers and FP64 shuffle trees, square roots and divisions in
@@ -140,10 +152,9 @@ __global__ void __launch_bounds__(NA_NT, 1) k_na_cg(NaArgs a) {
     // k_na_dinv ran before this launch on the same stream: every block reads the
     // same check result, so on a malformed matrix all leave together, before any
     // row loop or barrier
-    if (__ldcg(&h->bad) != NA_GOOD) return;
+    if (__ldcg(&h->bad) != NA_GOOD || (CL && __ldcg(&h->wide))) return;
     const int groups = (n + 31) / 32;
-    const int R0 = 32 * (int)((long long)groups * blockIdx.x / gridDim.x);
-    const int R1 = min(n, 32 * (int)((long long)groups * (blockIdx.x + 1) / gridDim.x));
+    const int R0 = na_first_row(n, blockIdx.x, gridDim.x), R1 = na_first_row(n, blockIdx.x + 1, gridDim.x);
     sysu::AllCtx c = sysu::all_ctx(reinterpret_cast<unsigned long long *>(a.base + NA_SLOTS));
     sysu::ClCtx cl = sysu::cl_ctx();
     if (CL) sysu::cl_sync();  // every block has started before its shared memory is written to
@@ -163,7 +174,7 @@ __global__ void __launch_bounds__(NA_NT, 1) k_na_cg(NaArgs a) {
         return sysu::cl_addr(zs + (j - 32 * (int)((long long)groups * o / G)), o);
     };
     const int E0 = a.rowptr[R0], nent = a.rowptr[R1] - E0;
-    const bool res = nent <= NA_ENTRIES;
+    const bool res = CL || nent <= NA_ENTRIES;
     double *sval = reinterpret_cast<double *>(na_smem);
     int *scol = reinterpret_cast<int *>(sval + (res ? nent : 0));
     if (res) {
@@ -176,13 +187,13 @@ __global__ void __launch_bounds__(NA_NT, 1) k_na_cg(NaArgs a) {
     const int *mc = res ? scol : a.col + E0;
     auto zat = [&](int e) {
         if (!CL) return zg[mc[e]];
-        return sysu::cl_load(res ? (unsigned)mc[e] : at(mc[e]));
+        return sysu::cl_load((unsigned)mc[e]);
     };
     __shared__ double s_rr, s_rho, s_thr, s_bb, s_alpha, s_beta, s_inv;
     __shared__ sysu::CgScalars S;
     __shared__ int s_brk, s_end;  // s_end: 1 converged, 2 the residual is not finite, 0 go on
     auto end_code = [&](double rr) {
-        return sysu::stop_below(rr, s_thr, a.eps, s_bb) ? 1 : isfinite(rr) ? 0 : 2;
+        return sysu::stop_below(rr, s_thr, a.eps, s_bb) ? 1 : sysu::finite_bits(rr) ? 0 : 2;
     };
     double x[R], r[R], p[R], q[R], d[R];
     int e0[R], len[R];
@@ -423,7 +434,10 @@ int sysu_csr_cg_noalloc(int n, const int *d_rowptr, const int *d_col, const doub
     // One cluster where a thread a row suffices: CTAs of 128 rows, one warp a scheduler, up to 16
     // of them, then more rows each.  Cluster against whole GPU, us an iteration: 512 rows 4.6 and
     // 7.2, 1,716 rows 4.6 and 6.9, 4,096 rows 5.0 and 6.9, 8,000 rows 6.3 and 6.9; with two rows a
-    // thread and two sums (13,824 rows) 8.5 and 6.8.
+    // thread and two sums (13,824 rows) 8.5 and 6.8.  A matrix that the cluster's shared memory
+    // does not hold (16 x 17,066 entries at most; k_na_dinv says so, and the call launches again)
+    // goes to the whole GPU: 4,096 rows of 101 entries 11.6, 8,192 of 61 9.1, where the cluster
+    // reading the caller's arrays took 54 and 47 and the form before it 46 and 32.
     int cluster = 0;
     if (n <= NA_CL_ROWS && g_na_cluster[dev] > 0) {
         cluster = 1;
@@ -432,7 +446,7 @@ int sysu_csr_cg_noalloc(int n, const int *d_rowptr, const int *d_col, const doub
     const int rows = cluster ? 32 * ((groups + cluster - 1) / cluster) : 0;
     if (rows > NA_NT) cluster = 0;
     const int threads = rows < 128 ? 128 : rows;
-    NaArgs a{n, d_rowptr, d_col, d_val, d_b, d_x, omega, maxit, eps, base};
+    NaArgs a{n, d_rowptr, d_col, d_val, d_b, d_x, omega, maxit, eps, base, cluster};
     // what must start at zero: the exchange area of the grid sums and the status words;
     // the malformed-row key starts at all ones (no row found)
     e = cudaMemsetAsync(base, 0, offsetof(NaHeader, bad), st);
@@ -447,6 +461,12 @@ int sysu_csr_cg_noalloc(int n, const int *d_rowptr, const int *d_col, const doub
     void *args[] = {&a};
     const void *kern = need <= 1 ? (const void *)k_na_cg<1, false>
                                  : need <= 2 ? (const void *)k_na_cg<2, false> : (const void *)k_na_cg<NA_ROWS, false>;
+    NaHeader h;
+    auto whole_gpu = [&] { return cudaLaunchCooperativeKernel(kern, dim3(G), dim3(NA_NT), args, NA_SMEM, st); };
+    auto read_back = [&] {
+        cudaError_t r = cudaMemcpyAsync(&h, base, sizeof(NaHeader), cudaMemcpyDeviceToHost, st);
+        return r == cudaSuccess ? cudaStreamSynchronize(st) : r;
+    };
     if (cluster) {
         cudaLaunchAttribute at{};
         at.id = cudaLaunchAttributeClusterDimension;
@@ -461,12 +481,15 @@ int sysu_csr_cg_noalloc(int n, const int *d_rowptr, const int *d_col, const doub
         lc.numAttrs = 1;
         e = cudaLaunchKernelEx(&lc, k_na_cg<1, true>, a);
     } else {
-        e = cudaLaunchCooperativeKernel(kern, dim3(G), dim3(NA_NT), args, NA_SMEM, st);
+        e = whole_gpu();
     }
     if (e != cudaSuccess) return na_fail(SYSU_ERR_CUDA, std::string("cooperative launch: ") + cudaGetErrorString(e));
-    NaHeader h;
-    e = cudaMemcpyAsync(&h, base, sizeof(NaHeader), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    e = read_back();
+    if (e == cudaSuccess && cluster && h.wide && h.bad == NA_GOOD) {
+        e = whole_gpu();
+        if (e != cudaSuccess) return na_fail(SYSU_ERR_CUDA, std::string("cooperative launch: ") + cudaGetErrorString(e));
+        e = read_back();
+    }
     if (e != cudaSuccess) return na_fail(SYSU_ERR_CUDA, std::string("read-back: ") + cudaGetErrorString(e));
     if (h.bad != NA_GOOD) {
         static const char *what[] = {"", "a row pointer that decreases", "a column index outside 0..n-1",
