@@ -253,10 +253,12 @@ __global__ void __launch_bounds__(GT) k_gnn_fwd(NetArgs a) {
             for (int e = 0; e < 8; ++e) mv[e] = 0.f;
             int c[8];
             float v[8];
-            auto entries = [&](int k) {  // columns and values of the row's neighbours k .. k + 7
+            // columns and values of the row's neighbours k .. k + 7, past the last one the row itself
+            // with weight 0 (another row's features may be infinite)
+            auto entries = [&](int k) {
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
-                    c[i] = 0;
+                    c[i] = in ? row0 + l8 : 0;
                     v[i] = 0.f;
                     if (in && k + i < w) {
                         c[i] = a.g.col[base + (k + i) * 32 + l8];
