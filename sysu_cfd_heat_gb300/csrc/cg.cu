@@ -1064,28 +1064,26 @@ static const int *sym_launch(const SellDev &A, const double *val, const double *
     a.ts = w.phase_ts;
     a.gate = gate;
     check_aligned16({a.val, a.col});
-    const bool narrow = A.wmax <= 5;  // gathers a thread holds: 4 off-diagonals (tets) or 6 (hexes)
+    constexpr int threads = fp32 ? SYM_NT32 : SYM_NT;
+    a.plan = plan_cg(A.wmax - 1, (int)sizeof(V), threads / 32 - 1);
+    // gathers a thread holds: 4 off-diagonals (tets), 6 (hexes), or tiles of fewer slices than
+    // consumer warps
+    const int form = a.plan.ts < threads / 32 - 1 ? 2 : A.wmax <= 5 ? 0 : 1;
+    static int mb[3] = {0, 0, 0};
+    int &maxb = mb[form];
     const void *kern;
-    int threads, maxb;
     if constexpr (fp32) {
-        static int mb[2] = {0, 0};
-        int &m = mb[narrow ? 0 : 1];
-        kern = narrow ? (const void *)k_cg_mixed_sym<4> : (const void *)k_cg_mixed_sym<6>;
-        if (!m) m = narrow ? cg_max_blocks(k_cg_mixed_sym<4>, SYM_NT32) : cg_max_blocks(k_cg_mixed_sym<6>, SYM_NT32);
-        threads = SYM_NT32;
-        maxb = m;
+        const auto k = form == 2 ? k_cg_mixed_sym<SYM_WIDE> : form == 1 ? k_cg_mixed_sym<6> : k_cg_mixed_sym<4>;
+        if (!maxb) maxb = cg_max_blocks(k, threads);
+        kern = (const void *)k;
         a.r = w.r32.get(); a.p = w.p32.get(); a.q = w.q32.get(); a.y = w.e32.get();
         a.r64 = w.r.get();
     } else {
-        static int mb[2] = {0, 0};
-        int &m = mb[narrow ? 0 : 1];
-        kern = narrow ? (const void *)k_cg_sym<4> : (const void *)k_cg_sym<6>;
-        if (!m) m = narrow ? cg_max_blocks(k_cg_sym<4>, SYM_NT) : cg_max_blocks(k_cg_sym<6>, SYM_NT);
-        threads = SYM_NT;
-        maxb = m;
+        const auto k = form == 2 ? k_cg_sym<SYM_WIDE> : form == 1 ? k_cg_sym<6> : k_cg_sym<4>;
+        if (!maxb) maxb = cg_max_blocks(k, threads);
+        kern = (const void *)k;
         a.r = w.r.get(); a.p = w.p.get(); a.q = w.v.get(); a.y = w.t.get();
     }
-    a.plan = plan_cg(A.wmax - 1, (int)sizeof(V), threads / 32 - 1);
     void *args[] = {&a};
     const int G = std::min(cg_grid(A, a.plan, maxb, 0), AX_MAX_BLOCKS);
     // at least three slots, more up to 118 KB: beyond that the L1 left for the gathers of r

@@ -131,6 +131,10 @@ __device__ __forceinline__ bool sym_acquire(int slot, unsigned par, int *err) {
 // and rows advance by a constant.  No look-ahead: holding the next tile's gathers during this
 // one's FMAs, as k_cg_pipe does, measured no faster in FP64 (50.2 us an iteration both) and
 // slower in FP32 (27.6 against 25.9).
+// WR: gathers held at a time; SYM_WIDE for rows so wide that a tile holds fewer slices than there
+// are consumer warps, of which those beyond have none (the test, in every tile, costs the others
+// 0.3 % in FP64 and 0.9 % in FP32).
+constexpr int SYM_WIDE = 8;
 template <class V, int WR>
 __device__ __forceinline__ V sym_s_phase(const Part &P, Ring &R, const CgSymArgs &a, V beta, V pend, bool has_dir,
                                          int *err) {
@@ -138,11 +142,10 @@ __device__ __forceinline__ V sym_s_phase(const Part &P, Ring &R, const CgSymArgs
     V *pv = static_cast<V *>(a.p), *qv = static_cast<V *>(a.q), *yv = static_cast<V *>(a.y);
     const V *rv = static_cast<const V *>(a.r);
     V pq = 0;
-    const int warp = (int)(threadIdx.x >> 5);
-    int s = P.sb + warp, i = 32 * s + lane;
+    int s = P.sb + (int)(threadIdx.x >> 5), i = 32 * s + lane;
     for (int t = 0; t < nt; ++t, s += P.ts, i += 32 * P.ts) {
-        // wide rows: a tile holds fewer slices than there are consumer warps
-        const bool act = warp < P.ts && i < a.A.n && s < P.se;
+        bool act = i < a.A.n && s < P.se;
+        if (WR == SYM_WIDE) act = act && (int)(threadIdx.x >> 5) < P.ts;
         V r = 0, p = 0, q = 0, y = 0;
         int2 pl = make_int2(0, 0);
         if (act) {
