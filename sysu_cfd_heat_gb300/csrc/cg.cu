@@ -1035,6 +1035,14 @@ static const int *sym_launch(const SellDev &A, const double *val, const double *
     // (a positive Jacobi weight cancels; with any other the form with M^-1 says what becomes of it)
     if (!o.jacobi || !(o.omega > 0.0) || !std::isfinite(o.omega) || w.sm_cap > 0) return nullptr;
     const int n = A.n;
+    constexpr int threads = fp32 ? SYM_NT32 : SYM_NT;
+    const CgPlan plan = plan_cg(A.wmax - 1, (int)sizeof(V), threads / 32 - 1);
+    // Not where a row is too long for a slot of the ring, and the matrix would be read from global
+    // memory (us an iteration, form with M^-1 and this one: 700,013 rows of 7 entries and one of 900
+    // FP64 104 and 136, FP32 50 and 65), nor in FP64 where rows hold more than 30 entries on
+    // average, and 4 of 19 consumer warps have a slice (400,013 rows of 39: 72 and 94; of 21: 50 and
+    // 37; one row of 47 among 700,013 of 7: 92 and 48; FP32 with 39: 48 and 44).
+    if (plan.direct || (!fp32 && A.nnz > 30l * n)) return nullptr;
     if (w.wt.size() < (size_t)n) w.wt.alloc(n);
     if (w.scol.size() < (size_t)A.nnz) w.scol.alloc(A.nnz);
     if (!w.sym_bad.size()) w.sym_bad.alloc(1);
@@ -1064,8 +1072,7 @@ static const int *sym_launch(const SellDev &A, const double *val, const double *
     a.ts = w.phase_ts;
     a.gate = gate;
     check_aligned16({a.val, a.col});
-    constexpr int threads = fp32 ? SYM_NT32 : SYM_NT;
-    a.plan = plan_cg(A.wmax - 1, (int)sizeof(V), threads / 32 - 1);
+    a.plan = plan;
     // gathers a thread holds: 4 off-diagonals (tets), 6 (hexes), or tiles of fewer slices than
     // consumer warps
     const int form = a.plan.ts < threads / 32 - 1 ? 2 : A.wmax <= 5 ? 0 : 1;

@@ -14,14 +14,15 @@
 // ||r|| is estimated in FP32 from r' and sqrt(a_ii), and summed exactly in FP64 whenever the
 // estimate does not clearly exceed the threshold, as in k_cg_pipe.
 //
-// us an iteration, form with M^-1 -> here: 2M tets FP64 67.4 -> 45.8, FP32 33.9 -> 24.9; hex
+// us an iteration, form with M^-1 -> here: 2M tets FP64 67.4 -> 45.8, FP32 33.9 -> 24.2; hex
 // mesh of 990,000 rows FP64 43.0 -> 30.2, FP32 25.3 -> 18.7; 504,000 tets FP64 24.5 -> 17.7.
 // FP64 at 2M: the FP64 pipe takes 33 us of it, 264 MB through L2 and the two grid sums (4 us)
 // the rest.  Tried and dropped: the CTA's own r in shared memory (slower: 66 us, it takes the
 // L1 away), y updated in the X phase (61 us).
 //
-// Runs where all diagonal entries have one sign (k_sym_diag counts the others); otherwise,
-// and without a preconditioner, the form with M^-1 runs.
+// Runs where all diagonal entries have one sign (k_sym_diag counts the others) and the Jacobi
+// weight is positive; otherwise, without a preconditioner, and for the rows that sym_launch leaves
+// out (cg.cu), the form with M^-1 runs.
 #pragma once
 
 #include "grid_all.cuh"
@@ -105,10 +106,6 @@ __device__ __forceinline__ void sym_slices_init(const Part &P, const SellView &A
 template <class V>
 __device__ __forceinline__ void issue_sym_tile(const Part &P, const CgSymArgs &a, int t, unsigned char *dst,
                                                uint64_t *bar, uint64_t pol) {
-    if (a.plan.direct) {
-        mbar_arrive_expect_tx(bar, 0);
-        return;
-    }
     const long e0 = tile_entry_packed(P, a.A.sl_ptr, t), e1 = tile_entry_packed(P, a.A.sl_ptr, t + 1);
     const unsigned bv = (unsigned)((e1 - e0) * sizeof(V)), bc = (unsigned)((e1 - e0) * 4);
     mbar_arrive_expect_tx(bar, bv + bc);
@@ -163,10 +160,6 @@ __device__ __forceinline__ V sym_s_phase(const Part &P, Ring &R, const CgSymArgs
             const unsigned char *slot = cslot_ptr(R);
             const V *vs = reinterpret_cast<const V *>(slot) + pl.x + lane;
             const int *cs = reinterpret_cast<const int *>(slot + cnt * (int)sizeof(V)) + pl.x + lane;
-            if (a.plan.direct) {
-                vs = static_cast<const V *>(a.val) + e0 + pl.x + lane;
-                cs = a.col + e0 + pl.x + lane;
-            }
             int c[WR];
             V g[WR];
 #pragma unroll
