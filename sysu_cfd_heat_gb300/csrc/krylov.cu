@@ -525,8 +525,9 @@ __device__ __forceinline__ void row_dot_resident(const BicgRows &M, int wmax, in
 // y_c = A (dinv .* x_c) for NR right-hand sides, skipping inactive ones, from the
 // column-scaled values sv[e] = a_e dinv[col e]; MULTI: right-hand side c has its own values
 // svals[c] (same pattern).  Four entries' columns, values and gathers before their FMAs,
-// which take the entries in order.
-template <int NR, bool MULTI>
+// which take the entries in order.  WIDE: rows of many entries, whole groups with the next group's
+// columns and values on their way (every row has its diagonal entry: w >= 1).
+template <int NR, bool MULTI, bool WIDE>
 __device__ __forceinline__ void row_dot_scaled(const SellView &A, const double *const *svals, int i,
                                                const double *__restrict__ x, int n, const bool (&act)[3],
                                                double (&y)[NR]) {
@@ -536,7 +537,39 @@ __device__ __forceinline__ void row_dot_scaled(const SellView &A, const double *
     constexpr int U = NR == 1 ? 4 : (MULTI ? 1 : 2);
 #pragma unroll
     for (int c = 0; c < NR; ++c) y[c] = 0.0;
-    for (int k = 0; k < w; k += U, e += 32 * U) {
+    int k = 0;
+    if constexpr (WIDE && !MULTI) {
+        const int *__restrict__ col = A.col + e;
+        const double *__restrict__ val = svals[0] + e;
+        constexpr int L = NR == 1 ? 4 : 2;
+        int jn[L];
+        double an[L];
+#pragma unroll
+        for (int q = 0; q < L; ++q) { jn[q] = __ldg(col + 32 * min(q, w - 1)); an[q] = __ldg(val + 32 * min(q, w - 1)); }
+        for (; k + L <= w; k += L) {
+            double g[L][NR], av[L];
+#pragma unroll
+            for (int q = 0; q < L; ++q) {
+                av[q] = an[q];
+#pragma unroll
+                for (int c = 0; c < NR; ++c)
+                    if (act[c]) g[q][c] = x[(size_t)c * n + jn[q]];
+            }
+#pragma unroll
+            for (int q = 0; q < L; ++q) {
+                const int kk = 32 * min(k + L + q, w - 1);
+                jn[q] = __ldg(col + kk);
+                an[q] = __ldg(val + kk);
+            }
+#pragma unroll
+            for (int q = 0; q < L; ++q)
+#pragma unroll
+                for (int c = 0; c < NR; ++c)
+                    if (act[c]) y[c] = fma(av[q], g[q][c], y[c]);
+        }
+        e += 32 * k;
+    }
+    for (; k < w; k += U, e += 32 * U) {
         int j[U];
         double a[U][MULTI ? NR : 1], g[U][NR];
 #pragma unroll
@@ -599,8 +632,8 @@ __device__ __forceinline__ void bicg_rows(int t0, int T, int n, F &&f) {
 // vectors but for p and s, which other threads gather, in registers (R rows a thread).  Rows and
 // sums are dealt to the same (virtual) threads and blocks as without, so the bits are the same.
 // 60,680 rows, us an iteration: 23.6 without, 19.6 with the matrix, 17.6 with the vectors.
-template <int NR, bool MULTI, bool RES, int R>
-__global__ void __launch_bounds__(RES ? BICG_RES_NT : KB, RES ? 1 : 4) k_bicgstab(BicgArgs a) {
+template <int NR, bool MULTI, bool RES, int R, bool WIDE = false>
+__global__ void __launch_bounds__(RES ? BICG_RES_NT : KB, RES ? 1 : WIDE ? 2 : 4) k_bicgstab(BicgArgs a) {
     static_assert(!(MULTI && RES) && (RES || R == 0), "the resident form takes one matrix");
     if (a.gate && a.gate->status[0] != DEV_STALLED) return;  // the same word for every block
     const int it_before = a.gate ? a.gate->iters[0] : 0;
@@ -708,7 +741,7 @@ __global__ void __launch_bounds__(RES ? BICG_RES_NT : KB, RES ? 1 : 4) k_bicgsta
             bicg_rows<R>(t0, T, n, [&](int i, int u) {
                 double y[NR];
                 if constexpr (RES) row_dot_resident<NR>(M, a.wmax, u, a.p, n, act, y);
-                else row_dot_scaled<NR, MULTI>(a.A, a.svals, i, a.p, n, act, y);
+                else row_dot_scaled<NR, MULTI, WIDE>(a.A, a.svals, i, a.p, n, act, y);
 #pragma unroll
                 for (int c = 0; c < NR; ++c) {
                     if (!act[c]) continue;
@@ -754,7 +787,7 @@ __global__ void __launch_bounds__(RES ? BICG_RES_NT : KB, RES ? 1 : 4) k_bicgsta
             bicg_rows<R>(t0, T, n, [&](int i, int u) {
                 double y[NR];
                 if constexpr (RES) row_dot_resident<NR>(M, a.wmax, u, a.s, n, act, y);
-                else row_dot_scaled<NR, MULTI>(a.A, a.svals, i, a.s, n, act, y);
+                else row_dot_scaled<NR, MULTI, WIDE>(a.A, a.svals, i, a.s, n, act, y);
 #pragma unroll
                 for (int c = 0; c < NR; ++c) {
                     if (!act[c]) continue;
@@ -876,14 +909,36 @@ struct BicgMixedState {
 };
 
 // y = A_s x over FP32 column-scaled values, one row (FMAs in entry order); local row j
-template <bool RES>
+template <bool RES, bool WIDE>
 __device__ __forceinline__ float bicg_row32(const BicgMixedArgs &a, const float *mval, const int *mcol, int ld, int i,
                                             int j, const float *x) {
     const int s = i >> 5, w = __ldg(a.A.sl_w + s);
     const int e = RES ? 0 : __ldg(a.A.sl_ptr + s) + (i & 31);
-    constexpr int U = RES ? 8 : 4;
+    constexpr int U = RES || WIDE ? 8 : 4;
     float y = 0.f;
-    for (int k0 = 0; k0 < w; k0 += U) {
+    int k0 = 0;
+    if constexpr (WIDE && !RES) {
+        const int *__restrict__ col = a.A.col + e;
+        const float *__restrict__ val = a.sv32 + e;
+        int jn[U];
+        float an[U];
+#pragma unroll
+        for (int q = 0; q < U; ++q) { jn[q] = __ldg(col + 32 * min(q, w - 1)); an[q] = __ldg(val + 32 * min(q, w - 1)); }
+        for (; k0 + U <= w; k0 += U) {
+            float g[U], av[U];
+#pragma unroll
+            for (int q = 0; q < U; ++q) { av[q] = an[q]; g[q] = x[jn[q]]; }
+#pragma unroll
+            for (int q = 0; q < U; ++q) {
+                const int kk = 32 * min(k0 + U + q, w - 1);
+                jn[q] = __ldg(col + kk);
+                an[q] = __ldg(val + kk);
+            }
+#pragma unroll
+            for (int q = 0; q < U; ++q) y = fmaf(av[q], g[q], y);
+        }
+    }
+    for (; k0 < w; k0 += U) {
         int c[U];
         float v[U], g[U];
 #pragma unroll
@@ -910,14 +965,15 @@ __device__ __forceinline__ float bicg_row32(const BicgMixedArgs &a, const float 
 // so by the threads: 1024 with four entries of a row at a time (64 registers, no spill); 512 with
 // eight, which is what fits best on chip, was slower there than 608 blocks of 256 with four sums.
 // us an iteration, those 608 blocks / 512 threads / 768 / 1024: 592,704 rows 54, 32.6, 29.7, 27.4;
-// 1,000,000 rows 65, 47, 42, 37.7; 1,996,800 rows 147, 159, 135, 117; 4,096,000 rows 270, 324, 265, 233.
-template <bool RES>
-constexpr int bicg_nt = RES ? 512 : 1024;
+// 1,000,000 rows 65, 47, 42, 37.7; 1,996,800 rows 147, 159, 135, 117; 4,096,000 rows 270, 324, 265, 233.  WIDE: long rows (bicg_wide),
+// eight entries ahead on 512 threads.
+template <bool RES, bool WIDE = false>
+constexpr int bicg_nt = RES || WIDE ? 512 : 1024;
 extern __shared__ __align__(16) unsigned char g_bicg_rows[];
 
-template <bool RES>
-__global__ void __launch_bounds__(bicg_nt<RES>, 1) k_bicgstab_mixed(BicgMixedArgs a, int wmax, int ld) {
-    constexpr int NT = bicg_nt<RES>;
+template <bool RES, bool WIDE>
+__global__ void __launch_bounds__(bicg_nt<RES, WIDE>, 1) k_bicgstab_mixed(BicgMixedArgs a, int wmax, int ld) {
+    constexpr int NT = bicg_nt<RES, WIDE>;
     const int n = a.A.n, tid = threadIdx.x;
     const bool lead = tid == 0;
     int *err = &a.info->err;
@@ -1027,7 +1083,7 @@ __global__ void __launch_bounds__(bicg_nt<RES>, 1) k_bicgstab_mixed(BicgMixedArg
         {
             float f = 0.f;
             for (int i = R0 + tid; i < R1; i += NT) {
-                const float y = bicg_row32<RES>(a, mval, mcol, ld, i, i - R0, p);
+                const float y = bicg_row32<RES, WIDE>(a, mval, mcol, ld, i, i - R0, p);
                 v[i] = y;
                 f = fmaf(rt[i], y, f);
             }
@@ -1052,7 +1108,7 @@ __global__ void __launch_bounds__(bicg_nt<RES>, 1) k_bicgstab_mixed(BicgMixedArg
         {
             float f0 = 0.f, f1 = 0.f, f2 = 0.f;
             for (int i = R0 + tid; i < R1; i += NT) {
-                const float y = bicg_row32<RES>(a, mval, mcol, ld, i, i - R0, r);
+                const float y = bicg_row32<RES, WIDE>(a, mval, mcol, ld, i, i - R0, r);
                 const float si = r[i];
                 t[i] = y;
                 f0 = fmaf(y, si, f0);
@@ -1226,6 +1282,22 @@ static int bicg_blocks_for(int n, int maxb) {
     return (int)std::min<long>(maxb, std::max<long>(num_sms(), want));
 }
 
+// Rows of more than 64 entries on average take the kernels for wide rows: matrix from memory, a
+// row's next columns and values loaded ahead, 128 registers a thread.  us an iteration, the form
+// before with plain loops / groups of entries with a test each (what narrow rows take) / here:
+// FP64 3,000 rows of 201 entries 54 / 66 / 46, 90,000 of 201 225 / 350 / 203; mixed 35 / 42 / 28.6
+// and 150 / 140 / 103.  At 61 entries the resident kernels are level (20,000 rows 24.5 in FP64, 25
+// here).  FP64 beyond shared memory takes them from 24 entries (90,000 rows of 41 54 and 43, 150,000
+// of 61 127 / 176 / 109): the narrow rows' kernel spills at the 64 registers of its four blocks an
+// SM, which long rows pay for in every entry.
+static bool bicg_wide(const SellDev &A) { return A.nnz > 64l * A.n; }
+static int bicg_wide_blocks() {
+    static int mb = 0;
+    if (!mb)
+        mb = std::min(coresident_blocks(k_bicgstab<1, false, false, 0, true>),
+                      coresident_blocks(k_bicgstab<3, false, false, 0, true>));
+    return mb;
+}
 static int bicg_max_blocks(int nrhs, bool multi) {
     static int mb[4] = {0, 0, 0, 0};
     if (!mb[0]) {
@@ -1244,8 +1316,10 @@ static void bicg_launch(const SellDev &A, const double *const *vals, bool multi,
                         double *const *x, const KrylovOpts &o, KrylovWork &w, SolveInfo *info, cudaStream_t st,
                         const SolveInfo *gate = nullptr) {
     int n = A.n;
-    int maxb = bicg_max_blocks(nrhs, multi);
-    if (w.sm_cap > 0) maxb = std::min(maxb, w.sm_cap * std::max(1, maxb / num_sms()));
+    auto blocks = [&](int maxb) {
+        if (w.sm_cap > 0) maxb = std::min(maxb, w.sm_cap * std::max(1, maxb / num_sms()));
+        return grid_for(n, bicg_blocks_for(n, maxb));
+    };
     w.ensure(n, nrhs == 1 ? 1 : 3, bicg_max_blocks(-1, false), st);
     const int nmat = multi ? nrhs : 1;
     if (w.sval.size() < (size_t)A.nnz * nmat) w.sval.alloc((size_t)A.nnz * nmat);
@@ -1277,19 +1351,24 @@ static void bicg_launch(const SellDev &A, const double *const *vals, bool multi,
     a.maxit = o.maxit;
     a.eps = o.eps;
     void *args[] = {&a};
-    a.G = grid_for(n, bicg_blocks_for(n, maxb));
+    a.G = blocks(bicg_max_blocks(nrhs, multi));
     a.wmax = A.wmax;
     // the resident form wherever the CTAs' rows fit
     const int C = std::min(a.G, w.sm_cap > 0 ? std::min(w.sm_cap, num_sms()) : num_sms());
     const int nt = KB * ((a.G + C - 1) / C), R = (n + a.G * KB - 1) / (a.G * KB);
     const size_t smem = (size_t)nt * R * A.wmax * 12;
-    const bool res = !multi && nt <= BICG_RES_NT && R <= 4 && A.wmax <= 255 && smem <= BICG_SMEM;
+    const bool res = !multi && !bicg_wide(A) && nt <= BICG_RES_NT && R <= 4 && A.wmax <= 255 && smem <= BICG_SMEM;
+    const bool wide = !multi && !res && A.nnz > 24l * n;
+    if (wide) a.G = blocks(bicg_wide_blocks());
     const void *k;
     if (res && nrhs == 1)
         k = R == 1 ? (const void *)k_bicgstab<1, false, true, 1>
                    : R == 2 ? (const void *)k_bicgstab<1, false, true, 2> : (const void *)k_bicgstab<1, false, true, 4>;
     else if (res)
         k = R == 1 ? (const void *)k_bicgstab<3, false, true, 1> : (const void *)k_bicgstab<3, false, true, 0>;
+    else if (wide)
+        k = nrhs == 1 ? (const void *)k_bicgstab<1, false, false, 0, true>
+                      : (const void *)k_bicgstab<3, false, false, 0, true>;
     else if (nrhs == 1)
         k = (const void *)k_bicgstab<1, false, false, 0>;
     else
@@ -1324,7 +1403,7 @@ void bicgstab_solve_mixed(const SellDev &A, const double *val, const double *b, 
     const int G = std::max(1, std::min(A.nslices, cap));
     int wmax = A.wmax, ld = 32 * ((A.nslices + G - 1) / G);
     const size_t want = (size_t)ld * wmax * 8;
-    const bool res = want <= budget;
+    const bool wide = bicg_wide(A), res = want <= budget && !wide;
     w.ensure(n, 1, bicg_max_blocks(-1, false), st);
     w.ensure32(n, st);
     if (w.rt32.size() < (size_t)n) {
@@ -1353,10 +1432,12 @@ void bicgstab_solve_mixed(const SellDev &A, const double *val, const double *b, 
     a.maxit = o.maxit;
     a.eps = o.eps;
     a.inner_tol = o.inner_tol;
-    const void *kern = res ? (const void *)k_bicgstab_mixed<true> : (const void *)k_bicgstab_mixed<false>;
+    const void *kern = res ? (const void *)k_bicgstab_mixed<true, false>
+                           : wide ? (const void *)k_bicgstab_mixed<false, true>
+                                  : (const void *)k_bicgstab_mixed<false, false>;
     if (res) SYSU_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget));
     void *args[] = {&a, &wmax, &ld};
-    SYSU_CUDA(cudaLaunchCooperativeKernel(kern, dim3(G), dim3(res ? bicg_nt<true> : bicg_nt<false>), args, res ? want : 0, st));
+    SYSU_CUDA(cudaLaunchCooperativeKernel(kern, dim3(G), dim3(res || wide ? bicg_nt<true> : bicg_nt<false>), args, res ? want : 0, st));
     ++::sysu::g_launches;
     // FP64 takes over from the current x if the FP32 refinement stalled (the
     // launch returns at once otherwise)
