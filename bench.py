@@ -860,6 +860,8 @@ def run_ours(args, r, w, lr):
     f_iter = cg_flops_per_iter(n, nnz)
     dp = [it * f_iter / (ms / 1000.0) / 1e12 for it, ms in zip(cg_it, p_ms) if ms > 0]
     dp_tflops = statistics.mean(dp) if dp else None
+    # beyond 6 rows a thread of 152 CTAs of 512 threads the matrix never fits on chip
+    kernel = "k_cg_sym" if n > 152 * 512 * 6 else "k_cg_res (on chip) or k_cg_sym"
     traffic = None
     tp = os.path.join(ROOT, "profiles", "cg_pressure_traffic.json")
     if args.workload == "c3" and not args.p_mixed and os.path.exists(tp):
@@ -904,11 +906,11 @@ def run_ours(args, r, w, lr):
         "e2e": {"value": w * args.steps / e2e_s, "unit": "iters/s", "h2d_bytes_per_step": h2d,
                 "d2h_bytes_per_step": d2h},
         "gpu_launches": int(launches),
-        "roofline": {"bound": "hbm", "kernel": "k_cg_sym (persistent Jacobi-PCG for p')",
+        "roofline": {"bound": "hbm", "kernel": kernel + " (persistent Jacobi-PCG for p')",
                      "achieved": achieved, "peak": hbm, "peak_source": peak_src, "unit": "GB/s",
                      "frac": (achieved / hbm) if achieved else None, "traffic": traffic,
                      "algorithmic_bytes_per_cg_iteration": b_iter},
-        "fp64_pipe": {"kernel": "k_cg_sym", "achieved_tflops": dp_tflops, "peak_tflops": FP64_PEAK_TFLOPS,
+        "fp64_pipe": {"kernel": kernel, "achieved_tflops": dp_tflops, "peak_tflops": FP64_PEAK_TFLOPS,
                       "peak_source": "nominal GB300 FP64 rate (2 FMA lanes per SM per clock)",
                       "frac": (dp_tflops / FP64_PEAK_TFLOPS) if dp_tflops else None,
                       "flops_per_cg_iteration": f_iter},

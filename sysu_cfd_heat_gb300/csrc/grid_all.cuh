@@ -156,7 +156,10 @@ __device__ __forceinline__ void ax_warp_sum(AxNum &a) {
     for (int j = 0; j < 6; ++j) a.l[j] = __reduce_add_sync(FULL_MASK, a.l[j]);
 }
 
-// sum_j l[j] 2^(24 (ref - 3 + j) - 1075) as FP64, correctly rounded; |l[j]| < 2^40.
+// sum_j l[j] 2^(24 (ref - 3 + j) - 1075) as FP64, correctly rounded; |l[j]| < 2^38, so that two limbs
+// make a signed 64-bit group.  The largest come from ax_grid: limbs of carried block sums, at most
+// 2^24 in size, from up to AX_MAX_BLOCKS blocks.
+static_assert(AX_MAX_BLOCKS <= 1 << 13, "a limb's total over the blocks must stay below 2^38");
 __device__ __forceinline__ double ax_to_double(const long long (&l)[7], int ref) {
     constexpr unsigned long long M48 = 0xFFFFFFFFFFFFull;
     // 48-bit groups g0..g2 in [0, 2^48) and the signed rest g3

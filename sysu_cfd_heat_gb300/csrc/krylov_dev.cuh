@@ -184,13 +184,6 @@ __device__ __forceinline__ void stamp(unsigned long long *ts, int it, int k) {
     }
 }
 
-// CG kernels run 1024-thread blocks, one per SM: 152 arrivals per grid barrier
-// instead of 4x as many, and the vector phases walk 4 rows per thread with
-// 16-byte loads so each thread keeps several loads in flight.
-constexpr int KBC = 1024;
-
-__device__ __forceinline__ double2 ld2(const double *p, int j) { return reinterpret_cast<const double2 *>(p)[j]; }
-__device__ __forceinline__ void st2(double *p, int j, double2 v) { reinterpret_cast<double2 *>(p)[j] = v; }
 __device__ __forceinline__ float4 ld4(const float *p, int j) { return reinterpret_cast<const float4 *>(p)[j]; }
 __device__ __forceinline__ void st4(float *p, int j, float4 v) { reinterpret_cast<float4 *>(p)[j] = v; }
 

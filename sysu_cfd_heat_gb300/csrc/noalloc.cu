@@ -1,7 +1,7 @@
 // Jacobi-preconditioned CG on a caller-owned device CSR matrix that allocates
-// nothing: its scratch (residual, direction, product, inverse diagonal, the
-// per-block partial sums, the grid barrier and the status words) lives in one
-// file-scope device array, g_noalloc_scratch, of fixed size.
+// nothing: its scratch (z, the inverse diagonal, the exchange area of the grid
+// sums and the status words) lives in one file-scope device array,
+// g_noalloc_scratch, of fixed size.
 //
 // Who needs it: callers that cannot call cudaMalloc -- host applications that
 // own all device memory through their own pool and do not let libraries
@@ -14,7 +14,7 @@
 // * at most SYSU_NOALLOC_MAX_ROWS rows (262,144); larger systems are rejected;
 // * the array costs 4.2 MB on every GPU that loads the library, until exit;
 // * all calls share the array and it keeps the last call's contents: each call
-//   clears what must start at zero (barrier counter, status words) itself;
+//   clears what must start at zero (exchange area, status words) itself;
 //   calls that overlap on the GPU (two streams, two threads) race on it;
 // * every call looks up the array's device address (cudaGetSymbolAddress,
 //   which allocates nothing) with the calling thread's device current, so a
