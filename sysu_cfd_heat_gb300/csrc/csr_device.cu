@@ -1,11 +1,11 @@
 // CSR -> SELL-32 on the device, for the entry points that take a host CSR matrix and need no
 // host copy of the pattern.
 //
-// On the host this took 3.3 of the 10.5 ms of a 65,600-row BiCGSTAB call (row lists with the
+// On the host this took 3.3 of the 10.5 ms of a 60,680-row BiCGSTAB call (row lists with the
 // diagonal first 1.05 ms, SELL positions 0.55, the sweeps' level schedules and uploads 1.2,
 // values 0.5).  Here the CSR arrays go up as they are (20 to 30 us a megabyte) and two kernels
-// form the same arrays, the host only adding up the slices' widths: 9.75 -> 6.8 ms with the solver's
-// vectors in one allocation, of which the solve itself is 6.4.
+// form the same arrays, the host only adding up the slices' widths: 9.75 -> 6.8 ms a call with the
+// solver's vectors in one allocation (now 5.7, 4.4 of it the solve's kernel).
 #include "csr_device.hpp"
 
 namespace sysu {

@@ -959,8 +959,9 @@ __device__ __forceinline__ float bicg_row32(const BicgMixedArgs &a, const float 
 
 // One CTA per SM owns a contiguous range of slices; three grid sums (grid_all.cuh) and two
 // bare barriers an iteration, the FP32 matrix in shared memory where it fits (RES).  s takes
-// r's storage.  Below 300k rows the grid-wide steps bound it: 256,000 rows of a hex mesh took
-// 48 us an iteration on 250 blocks of 256 with FP64 shuffle trees and four sums, here 28.
+// r's storage.  Below 300k rows the grid-wide steps bound it: 200,000 rows of 7 entries took 42 us
+// an iteration on blocks of 256 with FP64 shuffle trees and four sums, 300,000 rows 46; here 20.7
+// and 23.4.
 // A matrix beyond shared memory (from 520,000 rows of a hex mesh) is bound by what is in flight,
 // so by the threads: 1024 with four entries of a row at a time (64 registers, no spill); 512 with
 // eight, which is what fits best on chip, was slower there than 608 blocks of 256 with four sums.

@@ -137,12 +137,12 @@ __global__ void k_na_dinv(NaArgs a) {
 // other CTAs gather, is the only vector in memory.  Latency bounds it at every size up to the
 // limit: two sums (grid_all.cuh) and an FP64 division an iteration.  1,716 rows on 7 blocks
 // of 256 threads, with three barriers and FP64 shuffle trees, square roots and divisions in
-// every thread, took 13.7 us an iteration; on 54 CTAs here 6.6 (238,080 rows: 12.8).
+// every thread, took 12.7 us an iteration; on 54 CTAs here 6.1 (238,080 rows: 12.4).
 // CL: the grid is one cluster.  z lies in its CTAs' shared memory, the columns there are turned
-// into shared addresses of the cluster, and the sums meet at the cluster's barrier: 5.3 us with
-// the two sums, 4.6 with one (CgScalars) and a barrier.  Over the whole GPU that form is not
-// faster (6.9 against 6.8 at 32,768 rows, 7.5 against 7.2 at 60,680): three values at once and a
-// bare barrier take as long as the two sums.
+// into shared addresses of the cluster, and the sums meet at the cluster's barrier: one sum
+// (CgScalars) and a barrier, 3.9 us; with the two sums 0.7 more.  Over the whole GPU the form with
+// one sum was not faster (6.9 against 6.8 at 32,768 rows, 7.5 against 7.2 at 60,680): three values
+// at once and a bare barrier take as long as the two sums.
 template <int R, bool CL>
 __global__ void __launch_bounds__(NA_NT, 1) k_na_cg(NaArgs a) {
     NaHeader *h = reinterpret_cast<NaHeader *>(a.base);
@@ -432,12 +432,12 @@ int sysu_csr_cg_noalloc(int n, const int *d_rowptr, const int *d_col, const doub
     const int G = groups < blocks ? groups : blocks;
     const int need = (32 * ((groups + G - 1) / G) + NA_NT - 1) / NA_NT;  // rows a thread
     // One cluster where a thread a row suffices: CTAs of 128 rows, one warp a scheduler, up to 16
-    // of them, then more rows each.  Cluster against whole GPU, us an iteration: 512 rows 4.6 and
-    // 7.2, 1,716 rows 4.6 and 6.9, 4,096 rows 5.0 and 6.9, 8,000 rows 6.3 and 6.9; with two rows a
-    // thread and two sums (13,824 rows) 8.5 and 6.8.  A matrix that the cluster's shared memory
-    // does not hold (16 x 17,066 entries at most; k_na_dinv says so, and the call launches again)
-    // goes to the whole GPU: 4,096 rows of 101 entries 11.6, 8,192 of 61 9.1, where the cluster
-    // reading the caller's arrays took 54 and 47 and the form before it 46 and 32.
+    // of them, then more rows each.  Cluster against whole GPU, us an iteration: 512 rows 3.7 and
+    // 5.9, 1,716 rows 3.9 and 6.1, 4,096 rows 4.4 and 6.0, 8,000 rows 5.8 and 6.0; with two rows a
+    // thread and two sums 13,824 rows took 8.5 when the whole GPU took 6.8.  A matrix that the
+    // cluster's shared memory does not hold (16 x 17,066 entries at most; k_na_dinv says so, and the
+    // call launches again) goes to the whole GPU: 4,096 rows of 101 entries 11.6, 8,192 of 61 9.1,
+    // where the cluster reading the caller's arrays took 54 and 47 and the form before it 46 and 32.
     int cluster = 0;
     if (n <= NA_CL_ROWS && g_na_cluster[dev] > 0) {
         cluster = 1;
